@@ -57,6 +57,8 @@ enum ErrorFlag : uint32_t {
 // FrameView::work_counter[kSkipWord] != 0: the binning and composite passes do nothing (their
 // inputs would not fit the arrays they write; set by frame_gate_kernel).
 constexpr int kSkipWord = 27;
+// work_counter[kMaskAlloc], [kMaskAlloc + 1]: work items and masks handed out, one 64-bit counter.
+constexpr int kMaskAlloc = 32;
 
 enum FetchKind : uint32_t {
   kFetchSolid = 0,
@@ -288,14 +290,10 @@ struct FrameView {
   uint32_t* cmd_xr;            // pixel columns x0 | x1 << 16 (inclusive; x0 > x1 = nothing)
   uint32_t* cmd_yr;            // pixel rows y0 | y1 << 16
   uint32_t* cmdrow_base;       // [num_cmds + 1]: first (cmd, strip row, tile column) slot
-  uint32_t* cmdrow_counts;     // [num_cmdrows + 1]
-  uint32_t* cmdrow_offsets;    // scratch for the scan of non-empty slots
-  uint32_t* slot_cmd;          // [num_cmdrows] command of each slot with segments
-  uint32_t* slot_mask;         // [num_cmdrows + 1] 1 + index of the slot's masks, 0 = no segments
-  uint32_t* mask_slot;         // [non-empty slots] slot of each compact mask index
+  uint32_t* slot_mask;         // [num_cmdrows + 1] the slot's segment count (binning), then 1 + index of its masks; 0 = no segments
+  uint32_t* mask_cursor;       // [non-empty slots] the mask's first work item; past its last one after the items are placed
   uint4* mask_info;            // [non-empty slots] {x of the slot's first column, its first row, flags << 16 | alpha, slot}
-  uint32_t* slot_first;        // [num_cmdrows + 1] first work item of each slot (exclusive scan of the counts)
-  uint2* entries;              // coverage work items {segment, mask index}, grouped by slot in slot order
+  uint2* entries;              // coverage work items {segment, mask index}, grouped by mask in mask order
   uint32_t mask_capacity;      // slots the masks array holds
   uint8_t* masks;              // [non-empty slots][kStripRows * kTileW]: analytic masks from the coverage pass
   uint32_t* backdrop;          // [num_cmdrows][kStripRows]: coverage carried into the slot's tile
@@ -317,7 +315,7 @@ struct FrameView {
                                //   [23] cubic pieces, [24] their queue, [25] quadratic pieces, [26] their queue,
                                //   [28] / [29] cubic pieces inside the clip box / clipped, [30] / [31] their queues
   uint32_t* totals;            // [8] segments, seglist bound, (cmd,strip) slots, row entries, gradient rows,
-                               //   slots with segments, conic row runs
+                               //   unused, conic row runs
   uint32_t* rs_count;          // [num_cmds + 1] gradient row states per command (radial/conic styles)
   uint32_t* rs_base;           // exclusive scan of rs_count
   float4* row_states;          // per (command, row): the fetcher's row values f0, f1, f2

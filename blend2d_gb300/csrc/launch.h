@@ -36,15 +36,14 @@ int launch_sum(const uint32_t* in, uint32_t n, uint32_t* total, cudaStream_t st)
 int launch_lut(const FrameView& f, cudaStream_t st);
 int launch_edges(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st);
 int launch_cmd_tiles(const FrameView& f, uint32_t* cmdrow_counts_per_cmd, cudaStream_t st);
-int launch_seg_bin(const FrameView& f, int scatter, cudaStream_t st);
+int launch_bin_count(const FrameView& f, cudaStream_t st);
 int launch_rows_and_tiles(const FrameView& f, uint32_t* row_canvas, cudaStream_t st);
 int launch_fine(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st);
 int launch_row_states(const FrameView& f, cudaStream_t st);
-int launch_backdrop_prefix(const FrameView& f, cudaStream_t st);
 int launch_frame_gate(const FrameView& f, cudaStream_t st);
 // Copies the `n` canvases of `xfers` (device memory) to their host images (to_host) or back.
 int launch_canvas_copy(const DevXfer* xfers, uint32_t n, int to_host, cudaStream_t st);
-int launch_coverage(const FrameView& f, const LaunchConfig& cfg, uint32_t* scan_tmp, cudaStream_t st);
+int launch_coverage(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st);
 int fine_grid_size(int blocks_per_sm);
 // Stroking: per-figure outline sizes and their exclusive scan (stroke_offsets), then the outlines.
 int launch_stroke_count(const FrameView& f, cudaStream_t st);

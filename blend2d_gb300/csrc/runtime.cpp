@@ -705,15 +705,14 @@ int Runtime::enqueue_count_half(cudaStream_t st) {
 int Runtime::enqueue_render_half(cudaStream_t st, bool timed) {
   const FrameView& f = view;
   int k = launch_frame_gate(f, st);
-  cudaMemsetAsync(f.cmdrow_counts, 0, sizeof(uint32_t) * (f.num_cmdrows + 1), st);
+  cudaMemsetAsync(f.slot_mask, 0, sizeof(uint32_t) * (f.num_cmdrows + 1), st);
   cudaMemsetAsync(f.backdrop, 0, sizeof(uint32_t) * kStripRows * (size_t(f.num_cmdrows) + 1), st);
-  k += launch_seg_bin(f, 0, st);
-  k += launch_backdrop_prefix(f, st);
+  k += launch_bin_count(f, st);
   k += launch_rows_and_tiles(f, row_canvas, st);
   k += launch_row_states(f, st);
   // the fine stage: coverage (masks of analytic fills) + composite, timed together
   if (timed) cudaEventRecord(ev[1], st);
-  k += launch_coverage(f, cfg, f.cmdrow_offsets + f.num_cmdrows + 1, st);
+  k += launch_coverage(f, cfg, st);
   if (timed) cudaEventRecord(ev[4], st);
   if (f.num_lut_jobs) cudaStreamWaitEvent(st, join_ev, 0);     // the composite reads the LUTs
   k += launch_fine(f, cfg, st);
@@ -725,14 +724,10 @@ int Runtime::enqueue_render_half(cudaStream_t st, bool timed) {
 // work items), and each has one block of masks.
 static void plan_dynamic(Layout& L, FrameView& v, const FrameTotals& t) {
   const uint32_t slots = std::min(t.cmdrows, t.seglist);
-  v.cmdrow_counts = L.take<uint32_t>(t.cmdrows + 1);
-  v.cmdrow_offsets = L.take<uint32_t>(t.cmdrows + 1 + scan_temp_words(t.cmdrows + 1));
-  v.slot_cmd = L.take<uint32_t>(t.cmdrows + 1);
-  v.slot_mask = L.take<uint32_t>(t.cmdrows + 1);
-  v.slot_first = L.take<uint32_t>(t.cmdrows + 2);
+  v.slot_mask = L.take<uint32_t>(size_t(t.cmdrows) + 1);
   v.backdrop = L.take<uint32_t>((size_t(t.cmdrows) + 1) * kStripRows);
   v.entries = L.take<uint2>(size_t(t.seglist) + 1);
-  v.mask_slot = L.take<uint32_t>(size_t(slots) + 1);
+  v.mask_cursor = L.take<uint32_t>(size_t(slots) + 1);
   v.mask_info = L.take<uint4>(size_t(slots) + 1);
   v.masks = L.take<uint8_t>((size_t(slots) + 1) * kStripRows * kTileW);
   v.row_box = L.take<uint2>(size_t(t.row_entries) + 1);
