@@ -230,8 +230,10 @@ struct alignas(16) DevPiece {
   double2 p[4];
   uint32_t cmd;
   uint32_t any;
-  uint32_t pad[2];
+  uint32_t node;           // kPieceNode | sign << 8 | level: a subtree (eb::TreeNode) of a clipped piece; else 0
+  uint32_t pad;
 };
+constexpr uint32_t kPieceNode = 0x80000000u;
 
 // One figure of a stroked path: commands [first, end) of the frame's stroke input (the extent the
 // reference's stroker walks), the stroke command whose outline it adds to, and its options.
@@ -277,7 +279,8 @@ struct FrameView {
   DevItem* items;              // lines and curves of every analytic command (any order)
   DevItem* curve_items;        // cubic curves from the front, quadratic / conic curves from the back
   DevPiece* pieces;            // their monotonic pieces, cubic from the front, quadratic from the back
-  uint32_t* piece_list;        // cubic piece indices: inside the clip box from the front, clipped from the back
+  uint32_t* piece_list;        // [2 * piece_capacity] cubic, then quadratic piece indices: those the safe loop
+                               //   flattens from the front of their half, clipped ones from its back
   uint32_t piece_capacity;
   int4* cmd_bbox;              // [num_cmds] 24.8 bbox of the emitted segments: xmin, ymin, xmax, ymax
   DevSeg* segs;                // emitted segments (any order)
@@ -311,9 +314,9 @@ struct FrameView {
   uint32_t* strip_start;       // [num_tiles * strips per tile] first list entry the composite needs (occlusion)
   uint32_t* tile_order;        // tile processing order for the persistent fine kernel
   uint32_t* tile_canvas;       // canvas index per global tile
-  uint32_t* work_counter;      // [0] fine work queue, [1] items, [2] cubics, [3] their queue, [21] quads, [22] their queue,
-                               //   [23] cubic pieces, [24] their queue, [25] quadratic pieces, [26] their queue,
-                               //   [28] / [29] cubic pieces inside the clip box / clipped, [30] / [31] their queues
+  uint32_t* work_counter;      // [0] fine work queue, [1] items, [2] cubics, [21] quads, [23] / [25] cubic / quadratic
+                               //   pieces, [28..31] and [34..37] cubic / quadratic pieces the safe loop flattens, clipped
+                               //   ones, their queues, [38] / [39] cubic / quadratic subtrees handed over
   uint32_t* totals;            // [8] segments, seglist bound, (cmd,strip) slots, row entries, gradient rows,
                                //   unused, conic row runs
   uint32_t* rs_count;          // [num_cmds + 1] gradient row states per command (radial/conic styles)

@@ -730,6 +730,35 @@ __device__ __forceinline__ bool piece_flattens_safe(const Pt* pts, int deg, uint
   return f.x < l.x ? (f.x >= eb.cx0 && l.x <= eb.cx1) : (f.x <= eb.cx1 && l.x >= eb.cx0);
 }
 
+// What a monotonic piece of a clipped curve adds when no part of it lies in the clip box: nothing
+// (above or below it), or the vertical run y0..y1 at its left or right side, in the piece's
+// direction (`sign`). These are the cases in which flatten_unsafe leaves its loops without a line:
+// left or right of the box its leaves only ever reach the "outside" exits, which accumulate the
+// clipped y extent, and a piece that starts above the box gets there only with its end strictly
+// outside (on the side itself, the clipper emits a line).
+enum PieceOutside : int { kCrosses = 0, kNothing, kLeftRun, kRightRun };
+
+__device__ __forceinline__ PieceOutside piece_outside(const Pt* pts, int deg, const Builder& eb, double& y0, double& y1,
+                                                      uint32_t& sign) {
+  sign = pts[0].y > pts[deg].y;
+  const Pt f = sign ? pts[deg] : pts[0], l = sign ? pts[0] : pts[deg];
+  y0 = f.y;
+  y1 = dmin(l.y, eb.cy1);
+  if ((y0 >= y1) | (y1 <= eb.cy0)) return kNothing;
+  const bool above = y0 < eb.cy0;
+  y0 = dmax(y0, eb.cy0);
+  if (fabs(f.x - l.x) <= 0.00390625) {
+    if (dmax(f.x, l.x) <= eb.cx0) return kLeftRun;
+    return dmin(f.x, l.x) >= eb.cx1 ? kRightRun : kCrosses;
+  }
+  if (f.x < l.x) {
+    if (f.x >= eb.cx1) return kRightRun;
+    return (above ? l.x < eb.cx0 : f.x < eb.cx0 && l.x <= eb.cx0) ? kLeftRun : kCrosses;
+  }
+  if (f.x <= eb.cx0) return kLeftRun;
+  return (above ? l.x > eb.cx1 : f.x > eb.cx1 && l.x >= eb.cx1) ? kRightRun : kCrosses;
+}
+
 // One node: true for a leaf, else its two halves (Mono::is_flat / split / push / pop).
 template<int DEG>
 __device__ __forceinline__ bool tree_step(const TreeNode<DEG>& n, double tol_sq, TreeNode<DEG>& left, TreeNode<DEG>& right) {
@@ -1217,26 +1246,52 @@ struct LaneCurve {
     }
   }
 
-  // One pass of the current loop's body.
-  __device__ __forceinline__ void step(Builder& eb) {
+  // One pass of the current loop's body. With kHandOver it returns true, having done nothing, at a
+  // node whose subtree no clip can reach (in an inside loop, ending within the box: its subdivision
+  // points lie between its ends) and that is far from flat: the caller may have the subtree's
+  // segments emitted elsewhere (a TreeNode of points mc.p, level mc.sp) and call skip_node, or call
+  // split_node to go on here. Squared distances fall to 1/16 with each split, so a node beyond 256
+  // times the limit has at least four leaves or so: fewer are not worth the hand-over.
+  template<bool kHandOver = false>
+  __device__ __forceinline__ bool step(Builder& eb) {
     switch (state) {
-      case kLsLTop: out = mc.first().x >= eb.cx1; if (out) { exit_loop(eb, true); return; } break;
-      case kLsLLeft: out = mc.first().y >= eb.cy1; if (out) { exit_loop(eb, false); return; } break;
-      case kLsRTop: out = mc.first().x <= eb.cx0; if (out) { exit_loop(eb, false); return; } break;
-      case kLsRRight: out = mc.first().y >= eb.cy1; if (out) { exit_loop(eb, true); return; } break;
+      case kLsLTop: out = mc.first().x >= eb.cx1; if (out) { exit_loop(eb, true); return false; } break;
+      case kLsLLeft: out = mc.first().y >= eb.cy1; if (out) { exit_loop(eb, false); return false; } break;
+      case kLsRTop: out = mc.first().x <= eb.cx0; if (out) { exit_loop(eb, false); return false; } break;
+      case kLsRRight: out = mc.first().y >= eb.cy1; if (out) { exit_loop(eb, true); return false; } break;
       default: break;
     }
     Step st;
     if (!mc.is_flat(st)) {
+      if (kHandOver && st.value > 256.0 * st.limit && mc.last().y < eb.cy1 &&
+          ((state == kLsLIn && mc.last().x <= eb.cx1) || (state == kLsRIn && mc.last().x >= eb.cx0)))
+        return true;
       mc.split(st);
       const Pt m = mc.step_mid(st);
       const bool discard = ((state == kLsLTop) | (state == kLsRTop)) ? (m.y <= eb.cy0)
                          : state == kLsLLeft ? (m.x <= eb.cx0)
                          : state == kLsRRight ? (m.x >= eb.cx1) : false;
-      if (discard) { mc.discard_and_advance(st); return; }
-      if (mc.can_push()) { mc.push(st); return; }
+      if (discard) { mc.discard_and_advance(st); return false; }
+      if (mc.can_push()) { mc.push(st); return false; }
     }
     leaf(eb);
+    return false;
+  }
+
+  // The current node's subtree has been handed over: go on behind its last leaf.
+  __device__ __forceinline__ void skip_node(Builder& eb) {
+    eb.px = trunc_i(mc.last().x);
+    eb.py = trunc_i(mc.last().y);
+    out = 0;
+    if (!mc.can_pop()) { finish(eb); return; }
+    mc.pop();
+  }
+
+  // The current node (not flat, in an inside loop) flattened here after all.
+  __device__ __forceinline__ void split_node(Builder& eb) {
+    Step st;
+    mc.split(st);
+    if (mc.can_push()) mc.push(st); else leaf(eb);
   }
 
   __device__ __forceinline__ void leaf(Builder& eb) {

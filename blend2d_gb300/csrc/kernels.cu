@@ -457,125 +457,279 @@ __device__ __forceinline__ void finish_curve(FrameView& f, eb::Builder& b, uint3
 // the batched workload (piece kernel 10.8 -> 14.2 ms): the shared-memory carve-out shrinks the L1
 // that the stacks' and the segment sinks' local memory hits in.
 constexpr int kCurveThreads = 128;
-// work_counter words: cubic pieces inside the clip box, clipped cubic pieces, and their queues
-constexpr uint32_t kSafePieces = 28, kClipPieces = 29;
+constexpr uint32_t kSplitBlocksPerSM = 8;      // of each kind of curve
+// work_counter words of the cubic and of the quadratic / conic curves
+template<int DEG>
+struct CurveWords {
+  static constexpr uint32_t kCurves = DEG == 3 ? 2 : 21;     // curves of the curve list
+  static constexpr uint32_t kPieces = DEG == 3 ? 23 : 25;    // their monotonic pieces
+  static constexpr uint32_t kSafe = DEG == 3 ? 28 : 34;      // pieces the safe loop flattens
+  static constexpr uint32_t kClip = kSafe + 1;               // the other ones
+  static constexpr uint32_t kTreeQueue = kSafe + 2, kClipQueue = kSafe + 3;
+  static constexpr uint32_t kHanded = DEG == 3 ? 38 : 39;    // subtrees of clipped pieces handed to the tree flattener
+};
 // Idle lanes a warp waits for before it takes new pieces: each refill's set-up costs the warp its
 // FP64 instructions whatever the number of lanes refilled. On the batched workload 24 and 28
 // measured 246-248 ms per step, 16 and 20 250 ms, 32 251 ms, 8 257 ms and 4 259 ms.
-constexpr int kPieceRefillLanes = 24;
+constexpr uint32_t kPieceRefillLanes = 24;
 
-// Curves in two kernels. curve_split_kernel<DEG>: one thread per curve of the curve list does
+// Curves in three kernels, each with the cubic curves in the first half of its blocks and the
+// quadratic and conic ones in the second, so that neither kind's tail waits for the other's and a
+// frame without one kind loses blocks that leave at once, not launches. (Not alternating blocks: the
+// even ones go to one half of the SMs, and a frame of cubics alone took twice as long.)
+// curve_split_kernel: one thread per curve does
 // curve_to's set-up (transform, clip flags, a curve entirely on one side of the clip box, the split
 // into monotonic pieces: the divergent, FP64-heavy part) with every lane converged on it, and
-// writes the pieces. edge_pieces_kernel<DEG> flattens the pieces lane-scheduled, so taking a new
-// piece is cheap and the lanes' subdivision steps stay together. A piece is built by its own
+// writes the pieces. edge_pieces_kernel flattens the clipped pieces lane-scheduled, so taking a new
+// piece is cheap and the lanes' subdivision steps stay together; edge_tree_kernel then flattens what
+// no clip touches. A piece is built by its own
 // builder: the border runs a curve accumulates are vertical lines at the clip box's x0/x1 whose
 // cells add up the same whether the runs of consecutive pieces are merged or not.
 template<int DEG>
-__global__ void __launch_bounds__(128) curve_split_kernel(FrameView f) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ void split_curves(FrameView& f, uint32_t block, uint32_t blocks) {
+  using W = CurveWords<DEG>;
   const int lane = threadIdx.x & 31;
-  const uint32_t n_cubic = min(f.work_counter[2], f.item_capacity);
-  const uint32_t n_items = DEG == 3 ? n_cubic : min(f.work_counter[21], f.item_capacity - n_cubic);
-  uint32_t rows = 0, npieces = 0, cmd_i = 0;
-  eb::Pt spline[DEG == 3 ? 25 : 7];
-  uint32_t any = 0;
-  if (t < n_items) {
-    const DevItem it = f.curve_items[DEG == 3 ? t : f.item_capacity - 1u - t];
-    const DevCmd& cmd = f.cmds[it.cmd];
-    const DevXform& xf = f.xforms[cmd.xform];
-    eb::Builder b;
-    init_builder(b, f.canvases[cmd.canvas]);
-    b.sink.init(f.segs, f.seg_meta, f.totals + 0, f.seg_capacity, it.cmd);
-    eb::Src src;
-    src.xy = f.verts + 2ull * cmd.geom_first;
-    src.affine = xf.affine != 0;
-    src.m00 = xf.m[0]; src.m01 = xf.m[1]; src.m10 = xf.m[2]; src.m11 = xf.m[3]; src.m20 = xf.m[4]; src.m21 = xf.m[5];
-    const eb::Pt p0 = src.tf(int(it.a));
-    spline[1] = src.tf(int(it.b));
-    if (DEG == 3) { spline[2] = src.tf(int(it.b) + 1); spline[DEG] = src.tf(int(it.b) + 2); }
-    else spline[DEG] = src.tf(int(it.b) + (it.kind == kItemConic ? 2 : 1));
-    cmd_i = it.cmd;
-    // curve_to's set-up (LaneCurve::prepare, restated on this thread's own spline)
-    const uint32_t p0_flags = b.fxy(p0);
-    uint32_t common = p0_flags;
-    any = p0_flags;
+  const uint32_t n_cubic = min(f.work_counter[CurveWords<3>::kCurves], f.item_capacity);
+  const uint32_t n_items = DEG == 3 ? n_cubic : min(f.work_counter[CurveWords<2>::kCurves], f.item_capacity - n_cubic);
+  uint32_t* const list = f.piece_list + (DEG == 3 ? 0u : f.piece_capacity);
+  uint32_t rows = 0;
+  for (uint32_t t = block * blockDim.x + threadIdx.x; t - uint32_t(lane) < n_items; t += blocks * blockDim.x) {
+    uint32_t keep = 0, safe = 0, cmd_i = 0;       // bit k: piece k goes on; flattens as by the safe loop
+    eb::Pt spline[DEG == 3 ? 25 : 7];
+    uint32_t any = 0;
+    if (t < n_items) {
+      const DevItem it = f.curve_items[DEG == 3 ? t : f.item_capacity - 1u - t];
+      const DevCmd& cmd = f.cmds[it.cmd];
+      const DevXform& xf = f.xforms[cmd.xform];
+      eb::Builder b;
+      init_builder(b, f.canvases[cmd.canvas]);
+      b.sink.init(f.segs, f.seg_meta, f.totals + 0, f.seg_capacity, it.cmd);
+      eb::Src src;
+      src.xy = f.verts + 2ull * cmd.geom_first;
+      src.affine = xf.affine != 0;
+      src.m00 = xf.m[0]; src.m01 = xf.m[1]; src.m10 = xf.m[2]; src.m11 = xf.m[3]; src.m20 = xf.m[4]; src.m21 = xf.m[5];
+      const eb::Pt p0 = src.tf(int(it.a));
+      spline[1] = src.tf(int(it.b));
+      if (DEG == 3) { spline[2] = src.tf(int(it.b) + 1); spline[DEG] = src.tf(int(it.b) + 2); }
+      else spline[DEG] = src.tf(int(it.b) + (it.kind == kItemConic ? 2 : 1));
+      cmd_i = it.cmd;
+      // curve_to's set-up (LaneCurve::prepare, restated on this thread's own spline)
+      const uint32_t p0_flags = b.fxy(p0);
+      uint32_t common = p0_flags;
+      any = p0_flags;
 #pragma unroll
-    for (int i = 1; i <= DEG; i++) { const uint32_t fl = b.fxy(spline[i]); common &= fl; any |= fl; }
-    if (common) {
-      if (!(common & (eb::CF_Y0 | eb::CF_Y1))) {
-        const double y0 = eb::dclamp(p0.y, b.cy0, b.cy1), y1 = eb::dclamp(spline[DEG].y, b.cy0, b.cy1);
-        if (common & eb::CF_X0) b.acc_left(y0, y1); else b.acc_right(y0, y1);
+      for (int i = 1; i <= DEG; i++) { const uint32_t fl = b.fxy(spline[i]); common &= fl; any |= fl; }
+      if (common) {
+        if (!(common & (eb::CF_Y0 | eb::CF_Y1))) {
+          const double y0 = eb::dclamp(p0.y, b.cy0, b.cy1), y1 = eb::dclamp(spline[DEG].y, b.cy0, b.cy1);
+          if (common & eb::CF_X0) b.acc_left(y0, y1); else b.acc_right(y0, y1);
+        }
+        finish_curve(f, b, it.cmd, rows);
       }
-      finish_curve(f, b, it.cmd, rows);
+      else {
+        spline[0] = p0;
+        int nout = DEG == 3 ? eb::split_cubic(spline) : eb::split_quad(spline);
+        if (nout == 0) nout = DEG;
+        bool runs = false;
+        for (int k = 0; k < nout / DEG; k++) {
+          if (any) {
+            // pieces outside the clip box end here, with at most a run at its side
+            double y0, y1;
+            uint32_t sign;
+            const eb::PieceOutside where = eb::piece_outside(spline + k * DEG, DEG, b, y0, y1, sign);
+            if (where == eb::kLeftRun) b.acc_left_s(y0, y1, sign);
+            else if (where == eb::kRightRun) b.acc_right_s(y0, y1, sign);
+            runs |= where >= eb::kLeftRun;
+            if (where != eb::kCrosses) continue;
+          }
+          keep |= 1u << k;
+          if (eb::piece_flattens_safe(spline + k * DEG, DEG, any, b)) safe |= 1u << k;
+        }
+        if (runs) finish_curve(f, b, it.cmd, rows);
+      }
     }
-    else {
-      spline[0] = p0;
-      int nout = DEG == 3 ? eb::split_cubic(spline) : eb::split_quad(spline);
-      if (nout == 0) nout = DEG;
-      npieces = uint32_t(nout / DEG);
-    }
-  }
-  // one atomic per warp for the pieces of its curves
-  uint32_t incl = npieces;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-  uint32_t base = 0;
-  if (lane == 31 && total) base = atomicAdd(f.work_counter + (DEG == 3 ? 23 : 25), total);
-  base = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - npieces;
-  for (uint32_t k = 0; k < npieces; k++) {
-    const uint32_t idx = base + k;
-    if (idx >= f.piece_capacity) { atomicOr(f.error_flags, kErrPieces); break; }
-    DevPiece pc;
-#pragma unroll
-    for (int i = 0; i <= DEG; i++) pc.p[i] = make_double2(spline[k * DEG + i].x, spline[k * DEG + i].y);
-    pc.cmd = cmd_i;
-    pc.any = any;
-    f.pieces[DEG == 3 ? idx : f.piece_capacity - 1u - idx] = pc;
-  }
-  if (DEG == 3) {
-    // cubic pieces the safe loop flattens listed from the front of piece_list, the others from its
-    // back (one atomic per warp for each), in the pieces' order
-    uint32_t safe_mask = 0;                    // bit k: piece k flattens as by the safe loop
-    if (npieces) {
-      eb::Builder cb;
-      init_builder(cb, f.canvases[f.cmds[cmd_i].canvas]);
-      for (uint32_t k = 0; k < npieces; k++)
-        if (eb::piece_flattens_safe(spline + k * DEG, DEG, any, cb)) safe_mask |= 1u << k;
-    }
-    const uint32_t n_safe = uint32_t(__popc(safe_mask)), n_clip = npieces - n_safe;
-    uint32_t is = n_safe, ic = n_clip;
+    const uint32_t npieces = uint32_t(__popc(keep));
+    // one atomic per warp for the pieces of its curves
+    uint32_t incl = npieces;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t vs = __shfl_up_sync(0xFFFFFFFFu, is, o), vc = __shfl_up_sync(0xFFFFFFFFu, ic, o);
-      if (lane >= o) { is += vs; ic += vc; }
+      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += v;
     }
-    const uint32_t ts = __shfl_sync(0xFFFFFFFFu, is, 31), tc = __shfl_sync(0xFFFFFFFFu, ic, 31);
-    uint32_t bs = 0, bc = 0;
-    if (lane == 31) {
-      if (ts) bs = atomicAdd(f.work_counter + kSafePieces, ts);
-      if (tc) bc = atomicAdd(f.work_counter + kClipPieces, tc);
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    uint32_t base = 0;
+    if (lane == 31 && total) base = atomicAdd(f.work_counter + W::kPieces, total);
+    base = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - npieces;
+    uint32_t idx = base;
+    for (uint32_t todo = keep; todo; todo &= todo - 1u, idx++) {
+      const int k = __ffs(todo) - 1;
+      if (idx >= f.piece_capacity) { atomicOr(f.error_flags, kErrPieces); break; }
+      DevPiece pc;
+#pragma unroll
+      for (int i = 0; i <= DEG; i++) pc.p[i] = make_double2(spline[k * DEG + i].x, spline[k * DEG + i].y);
+      pc.cmd = cmd_i;
+      pc.any = any;
+      pc.node = 0u;
+      f.pieces[DEG == 3 ? idx : f.piece_capacity - 1u - idx] = pc;
     }
-    bs = __shfl_sync(0xFFFFFFFFu, bs, 31) + is - n_safe;
-    bc = __shfl_sync(0xFFFFFFFFu, bc, 31) + ic - n_clip;
-    uint32_t ks = 0, kc = 0;
-    for (uint32_t k = 0; k < npieces; k++) {
-      const uint32_t idx = base + k;
-      if (idx >= f.piece_capacity) break;
-      if ((safe_mask >> k) & 1u) f.piece_list[bs + ks++] = idx;
-      else f.piece_list[f.piece_capacity - 1u - (bc + kc++)] = idx;
+    {
+      // pieces the safe loop flattens listed from the front of the kind's list, the others from its
+      // back (one atomic per warp for each), in the pieces' order
+      const uint32_t n_safe = uint32_t(__popc(safe)), n_clip = npieces - n_safe;
+      uint32_t is = n_safe, ic = n_clip;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t vs = __shfl_up_sync(0xFFFFFFFFu, is, o), vc = __shfl_up_sync(0xFFFFFFFFu, ic, o);
+        if (lane >= o) { is += vs; ic += vc; }
+      }
+      const uint32_t ts = __shfl_sync(0xFFFFFFFFu, is, 31), tc = __shfl_sync(0xFFFFFFFFu, ic, 31);
+      uint32_t bs = 0, bc = 0;
+      if (lane == 31) {
+        if (ts) bs = atomicAdd(f.work_counter + W::kSafe, ts);
+        if (tc) bc = atomicAdd(f.work_counter + W::kClip, tc);
+      }
+      bs = __shfl_sync(0xFFFFFFFFu, bs, 31) + is - n_safe;
+      bc = __shfl_sync(0xFFFFFFFFu, bc, 31) + ic - n_clip;
+      uint32_t ks = 0, kc = 0;
+      idx = base;
+      for (uint32_t todo = keep; todo; todo &= todo - 1u, idx++) {
+        if (idx >= f.piece_capacity) break;
+        const uint32_t at = DEG == 3 ? idx : f.piece_capacity - 1u - idx;
+        if ((safe >> (__ffs(todo) - 1)) & 1u) list[bs + ks++] = at;
+        else list[f.piece_capacity - 1u - (bc + kc++)] = at;
+      }
     }
   }
   rows = __reduce_add_sync(0xFFFFFFFFu, rows);
   if (lane == 0 && rows) atomicAdd(f.totals + 1, rows);
 }
 
-// The cubic pieces the safe loop flattens (those of curves inside the clip box, and the inside
-// pieces of clipped curves: eb::piece_flattens_safe), flattened as subdivision trees (eb::TreeNode)
+__global__ void __launch_bounds__(128) curve_split_kernel(FrameView f) {
+  const uint32_t half = gridDim.x / 2u;
+  if (blockIdx.x >= half) split_curves<2>(f, blockIdx.x - half, half);
+  else split_curves<3>(f, blockIdx.x, half);
+}
+
+// The clipped pieces: the clipping state machine, one step of a lane's piece per iteration of a
+// warp-wide loop. Only the nodes on the way to a clip are walked here: a subtree inside the clip box
+// is handed to the tree flattener, as a piece in the gap between the cubic pieces (from the front of
+// the piece array) and the others (from its back), while there is room (half of the gap each). A
+// clipped piece then costs its lane some seven steps on average, not one per leaf. Bound: latency, with
+// 5 of 32 lanes active. Against flattening every leaf here, one kernel per kind of curve, all
+// quadratic pieces included: large shapes on 1023x767 0.65 -> 0.06 ms (the tree flattener 0.07 ->
+// 0.04), 10,000 stroked paths (quadratic outlines) 0.94 -> 0.06 (tree 0.03 -> 0.30), a 64x64 icon
+// 0.10 -> 0.04, 20,000 curve paths on 1920x1080 0.17 -> 0.13, 512 canvases of the batch 3.04 -> 2.12
+// (there mostly because pieces outside the box end in curve_split_kernel, 1.92 -> 2.16).
+
+// The gap's entries for handed-over subtrees of one kind.
+__device__ __forceinline__ uint32_t handed_room(const FrameView& f, uint32_t n_cubic, uint32_t n_quad) {
+  return n_cubic + n_quad < f.piece_capacity ? (f.piece_capacity - n_cubic - n_quad) / 2u : 0u;
+}
+
+// Pieces a warp takes at a time: all its idle lanes can hold, or, in frames whose pieces are fewer
+// than the launch's lanes, an even share of them once all its lanes are idle, so that every warp has
+// some.
+__device__ __forceinline__ uint32_t piece_share(uint32_t n_items, uint32_t blocks) {
+  const uint32_t warps = blocks * (kCurveThreads / 32);
+  return min(32u, (n_items + warps - 1u) / warps);
+}
+
+template<int DEG>
+__device__ void flatten_clipped(FrameView& f, uint32_t blocks) {
+  using W = CurveWords<DEG>;
+  const int lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t n_cubic = min(f.work_counter[CurveWords<3>::kPieces], f.piece_capacity);
+  const uint32_t n_quad = min(f.work_counter[CurveWords<2>::kPieces], f.piece_capacity - n_cubic);
+  const uint32_t n_mine = DEG == 3 ? n_cubic : n_quad;
+  const uint32_t n_items = min(f.work_counter[W::kClip], n_mine);
+  const uint32_t room = handed_room(f, n_cubic, n_quad), share = piece_share(n_items, blocks);
+  const uint32_t* const list = f.piece_list + (DEG == 3 ? 0u : f.piece_capacity);
+  uint32_t* queue = f.work_counter + W::kClipQueue;
+  eb::Builder b;
+  eb::LaneCurve<DEG, eb::CachedStack<DEG>> lc;
+  bool busy = false, exhausted = false;
+  uint32_t cur = 0, rows = 0;
+
+  for (;;) {
+    // hand the next pieces of the list to the idle lanes (one atomic per warp), once enough lanes
+    // are idle that the set-up's FP64 instructions serve several pieces at once
+    const uint32_t want = __ballot_sync(0xFFFFFFFFu, !busy && !exhausted);
+    const bool none = !__any_sync(0xFFFFFFFFu, busy);
+    if (want && ((share == 32u && uint32_t(__popc(want)) >= kPieceRefillLanes) || none)) {
+      const int leader = __ffs(want) - 1;
+      const uint32_t take = none ? min(uint32_t(__popc(want)), share) : uint32_t(__popc(want));
+      uint32_t base = 0;
+      if (lane == leader) base = atomicAdd(queue, take);
+      base = __shfl_sync(0xFFFFFFFFu, base, leader);
+      if (base >= n_items) exhausted = true;
+      const uint32_t rank = uint32_t(__popc(want & lt));
+      if (!busy && !exhausted && rank < take) {
+        const uint32_t t = base + rank;
+        if (t >= n_items) {
+          exhausted = true;
+        }
+        else {
+          const uint32_t pi = list[f.piece_capacity - 1u - t];
+          // a list entry is written only for a piece that fit in the piece array; with a frame
+          // that overflowed it (reported by curve_split), an entry may be stale: the lane then
+          // stays idle and takes another piece
+          if (DEG == 3 ? pi < n_cubic : (pi < f.piece_capacity && pi >= f.piece_capacity - n_quad)) {
+            const DevPiece pc = f.pieces[pi];
+            cur = pc.cmd;
+            init_builder(b, f.canvases[f.cmds[cur].canvas]);
+            b.sink.init(f.segs, f.seg_meta, f.totals + 0, f.seg_capacity, cur);
+            eb::Pt pts[DEG + 1];
+#pragma unroll
+            for (int i = 0; i <= DEG; i++) pts[i] = eb::Pt{pc.p[i].x, pc.p[i].y};
+            busy = lc.begin_piece(b, pts, pc.any);
+            if (!busy) finish_curve(f, b, cur, rows);
+          }
+        }
+      }
+    }
+    if (__all_sync(0xFFFFFFFFu, !busy && exhausted)) break;   // the list is exhausted
+    const bool hand = busy && lc.template step<true>(b);
+    const uint32_t hands = __ballot_sync(0xFFFFFFFFu, hand);
+    if (hands) {
+      const int leader = __ffs(hands) - 1;
+      uint32_t at = 0;
+      if (lane == leader) at = atomicAdd(f.work_counter + W::kHanded, uint32_t(__popc(hands)));
+      at = __shfl_sync(0xFFFFFFFFu, at, leader) + uint32_t(__popc(hands & lt));
+      if (hand) {
+        if (at < room) {
+          DevPiece pc;
+#pragma unroll
+          for (int i = 0; i <= DEG; i++) pc.p[i] = make_double2(lc.mc.p[i].x, lc.mc.p[i].y);
+          pc.cmd = cur;
+          pc.any = 0;
+          pc.node = kPieceNode | (lc.sign << 8) | uint32_t(lc.mc.sp);
+          f.pieces[DEG == 3 ? n_cubic + at : f.piece_capacity - 1u - n_quad - at] = pc;
+          // the subtree's segments count towards this command's bounds where they are emitted
+          lc.skip_node(b);
+        }
+        else {
+          lc.split_node(b);
+        }
+      }
+    }
+    if (busy && lc.state == eb::kLsDone && !lc.next_piece(b, true)) {
+      finish_curve(f, b, cur, rows);
+      busy = false;
+    }
+  }
+  rows = __reduce_add_sync(0xFFFFFFFFu, rows);
+  if (lane == 0 && rows) atomicAdd(f.totals + 1, rows);
+}
+
+__global__ void __launch_bounds__(kCurveThreads) edge_pieces_kernel(FrameView f) {
+  const uint32_t half = gridDim.x / 2u;
+  if (blockIdx.x >= half) flatten_clipped<2>(f, half);
+  else flatten_clipped<3>(f, half);
+}
+
+// The pieces the safe loop flattens (those of curves inside the clip box, and the inside pieces of
+// clipped curves: eb::piece_flattens_safe) and the subtrees edge_pieces_kernel handed over, flattened as subdivision trees (eb::TreeNode)
 // whose nodes the lanes of a warp share. A lane splits its node, goes on with the left half and keeps the
 // right half on its own stack, unless a lane of the warp is out of work: then the right half goes
 // to that lane through shared memory. So lanes do not sit idle while other lanes' trees still have
@@ -590,23 +744,28 @@ __global__ void __launch_bounds__(128) curve_split_kernel(FrameView f) {
 constexpr int kTreeRefillLanes = 16;
 constexpr int kTreeBlocksPerSM = 3;
 
+template<int DEG>
 struct alignas(16) TreeXchg {
-  double x[4], y[4];
+  double x[DEG + 1], y[DEG + 1];
   uint32_t cmd, level, sign, pad;
 };
 
-__global__ void __launch_bounds__(kCurveThreads) edge_tree_kernel(FrameView f) {
-  constexpr int kWarps = kCurveThreads / 32;
-  __shared__ TreeXchg xchg[kWarps][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+template<int DEG>
+__device__ void flatten_trees(FrameView& f, TreeXchg<DEG>* xchg, uint32_t blocks) {
+  using W = CurveWords<DEG>;
+  const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t n_cubic = min(f.work_counter[23], f.piece_capacity);
-  const uint32_t n_items = min(f.work_counter[kSafePieces], n_cubic);
-  uint32_t* queue = f.work_counter + kSafePieces + 2;
+  const uint32_t n_cubic = min(f.work_counter[CurveWords<3>::kPieces], f.piece_capacity);
+  const uint32_t n_quad = min(f.work_counter[CurveWords<2>::kPieces], f.piece_capacity - n_cubic);
+  const uint32_t n_safe = min(f.work_counter[W::kSafe], DEG == 3 ? n_cubic : n_quad);
+  const uint32_t n_items = n_safe + min(f.work_counter[W::kHanded], handed_room(f, n_cubic, n_quad));
+  const uint32_t share = piece_share(n_items, blocks);
+  const uint32_t* const list = f.piece_list + (DEG == 3 ? 0u : f.piece_capacity);
+  uint32_t* queue = f.work_counter + W::kTreeQueue;
   const double tol = 0.20 * 256.0;
   const double tol_sq = tol * tol;                    // init_builder's
-  eb::TreeNode<3> cur;
-  eb::TreeNode<3> stack[eb::kStackLevels];
+  eb::TreeNode<DEG> cur;
+  eb::TreeNode<DEG> stack[eb::kStackLevels];
   int nst = 0;
   uint32_t cmd = 0, sign = 0;
   bool busy = false, exhausted = false;
@@ -631,25 +790,38 @@ __global__ void __launch_bounds__(kCurveThreads) edge_tree_kernel(FrameView f) {
   for (;;) {
     // new pieces for the idle lanes, as edge_pieces_kernel takes them
     const uint32_t want = __ballot_sync(0xFFFFFFFFu, !busy && !exhausted);
-    if (want && (__popc(want) >= kTreeRefillLanes || !__any_sync(0xFFFFFFFFu, busy))) {
+    const bool none = !__any_sync(0xFFFFFFFFu, busy);
+    if (want && ((share == 32u && __popc(want) >= kTreeRefillLanes) || none)) {
       const int leader = __ffs(want) - 1;
+      const uint32_t take = none ? min(uint32_t(__popc(want)), share) : uint32_t(__popc(want));
       uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(queue, uint32_t(__popc(want)));
+      if (lane == leader) base = atomicAdd(queue, take);
       base = __shfl_sync(0xFFFFFFFFu, base, leader);
-      if (!busy && !exhausted) {
-        const uint32_t t = base + uint32_t(__popc(want & lt));
+      if (base >= n_items) exhausted = true;
+      const uint32_t rank = uint32_t(__popc(want & lt));
+      if (!busy && !exhausted && rank < take) {
+        const uint32_t t = base + rank;
         if (t >= n_items) {
           exhausted = true;
         }
         else {
-          const uint32_t pi = f.piece_list[t];
+          const uint32_t e = t - n_safe;         // a handed-over subtree when t >= n_safe
+          const uint32_t pi = t < n_safe ? list[t] : DEG == 3 ? n_cubic + e : f.piece_capacity - 1u - n_quad - e;
           // an entry of a piece that did not fit in the piece array (the frame fails) is skipped
-          if (pi < n_cubic) {
+          if (t >= n_safe || (DEG == 3 ? pi < n_cubic : pi < f.piece_capacity && pi >= f.piece_capacity - n_quad)) {
             const DevPiece pc = f.pieces[pi];
-            eb::Pt pts[4];
+            eb::Pt pts[DEG + 1];
 #pragma unroll
-            for (int i = 0; i < 4; i++) pts[i] = eb::Pt{pc.p[i].x, pc.p[i].y};
-            cur = eb::tree_root<3>(pts, sign);
+            for (int i = 0; i <= DEG; i++) pts[i] = eb::Pt{pc.p[i].x, pc.p[i].y};
+            if (pc.node & kPieceNode) {          // oriented and bounded already
+#pragma unroll
+              for (int i = 0; i <= DEG; i++) cur.p[i] = pts[i];
+              cur.level = int(pc.node & 0xFFu);
+              sign = (pc.node >> 8) & 1u;
+            }
+            else {
+              cur = eb::tree_root<DEG>(pts, sign);
+            }
             cmd = pc.cmd;
             nst = 0;
             busy = true;
@@ -659,15 +831,15 @@ __global__ void __launch_bounds__(kCurveThreads) edge_tree_kernel(FrameView f) {
     }
     if (__all_sync(0xFFFFFFFFu, !busy && exhausted)) break;
 
-    eb::TreeNode<3> left, right;
-    const bool leaf = busy && eb::tree_step<3>(cur, tol_sq, left, right);
+    eb::TreeNode<DEG> left, right;
+    const bool leaf = busy && eb::tree_step<DEG>(cur, tol_sq, left, right);
     const bool split = busy && !leaf;
 
     // a leaf's segment (Builder::add after desc_open, Sink::emit), one atomic for the warp
     int x0 = 0, y0 = 0, x1 = 0, y1 = 0;
     if (leaf) {
       x0 = eb::trunc_i(cur.p[0].x); y0 = eb::trunc_i(cur.p[0].y);
-      x1 = eb::trunc_i(cur.p[3].x); y1 = eb::trunc_i(cur.p[3].y);
+      x1 = eb::trunc_i(cur.p[DEG].x); y1 = eb::trunc_i(cur.p[DEG].y);
     }
     const bool emit = leaf && y0 != y1;
     const uint32_t em = __ballot_sync(0xFFFFFFFFu, emit);
@@ -706,9 +878,9 @@ __global__ void __launch_bounds__(kCurveThreads) edge_tree_kernel(FrameView f) {
     if (split) {
       const int r = __popc(donors & lt);
       if (r < k) {
-        TreeXchg& x = xchg[w][r];
+        TreeXchg<DEG>& x = xchg[r];
 #pragma unroll
-        for (int i = 0; i < 4; i++) { x.x[i] = right.p[i].x; x.y[i] = right.p[i].y; }
+        for (int i = 0; i <= DEG; i++) { x.x[i] = right.p[i].x; x.y[i] = right.p[i].y; }
         x.cmd = cmd;
         x.level = uint32_t(right.level);
         x.sign = sign;
@@ -722,9 +894,9 @@ __global__ void __launch_bounds__(kCurveThreads) edge_tree_kernel(FrameView f) {
     if (!busy) {
       const int q = __popc(idle & lt);
       if (q < k) {
-        const TreeXchg& x = xchg[w][q];
+        const TreeXchg<DEG>& x = xchg[q];
 #pragma unroll
-        for (int i = 0; i < 4; i++) cur.p[i] = eb::Pt{x.x[i], x.y[i]};
+        for (int i = 0; i <= DEG; i++) cur.p[i] = eb::Pt{x.x[i], x.y[i]};
         cur.level = int(x.level);
         cmd = x.cmd;
         sign = x.sign;
@@ -739,68 +911,12 @@ __global__ void __launch_bounds__(kCurveThreads) edge_tree_kernel(FrameView f) {
   if (lane == 0 && rows) atomicAdd(f.totals + 1, rows);
 }
 
-// Cubic pieces in two kernels: those inside the clip box (most of them) are flattened by
-// edge_tree_kernel, whose lanes share the nodes of their subdivision trees; the clipped ones run the
-// clipping state machine here. Quadratic and conic pieces all take this kernel.
-enum PieceSet : int { kPiecesAll = 0, kPiecesClipped = 2 };
-
-template<int DEG, int SET>
-__global__ void __launch_bounds__(kCurveThreads) edge_pieces_kernel(FrameView f) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t n_cubic = min(f.work_counter[23], f.piece_capacity);
-  const uint32_t n_items = SET == kPiecesClipped ? min(f.work_counter[kClipPieces], n_cubic)
-                         : DEG == 3 ? n_cubic : min(f.work_counter[25], f.piece_capacity - n_cubic);
-  uint32_t* queue = f.work_counter + (SET == kPiecesClipped ? kClipPieces + 2 : DEG == 3 ? 24 : 26);
-  eb::Builder b;
-  eb::LaneCurve<DEG, eb::CachedStack<DEG>> lc;
-  bool busy = false, exhausted = false;
-  uint32_t cur = 0, rows = 0;
-
-  for (;;) {
-    // hand the next pieces of the list to the idle lanes (one atomic per warp), once enough lanes
-    // are idle that the set-up's FP64 instructions serve several pieces at once
-    const uint32_t want = __ballot_sync(0xFFFFFFFFu, !busy && !exhausted);
-    if (want && (__popc(want) >= kPieceRefillLanes || !__any_sync(0xFFFFFFFFu, busy))) {
-      const int leader = __ffs(want) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(queue, uint32_t(__popc(want)));
-      base = __shfl_sync(0xFFFFFFFFu, base, leader);
-      if (!busy && !exhausted) {
-        const uint32_t t = base + uint32_t(__popc(want & ((1u << lane) - 1u)));
-        if (t >= n_items) {
-          exhausted = true;
-        }
-        else {
-          const uint32_t pi = SET == kPiecesClipped ? f.piece_list[f.piece_capacity - 1u - t]
-                            : DEG == 3 ? t : f.piece_capacity - 1u - t;
-          // a list entry is written only for a piece that fit in the piece array; with a frame
-          // that overflowed it (reported by curve_split), an entry may be stale: the lane then
-          // stays idle and takes another piece
-          if (SET == kPiecesAll || pi < n_cubic) {
-            const DevPiece pc = f.pieces[pi];
-            cur = pc.cmd;
-            init_builder(b, f.canvases[f.cmds[cur].canvas]);
-            b.sink.init(f.segs, f.seg_meta, f.totals + 0, f.seg_capacity, cur);
-            eb::Pt pts[DEG + 1];
-#pragma unroll
-            for (int i = 0; i <= DEG; i++) pts[i] = eb::Pt{pc.p[i].x, pc.p[i].y};
-            busy = lc.begin_piece(b, pts, pc.any);
-            if (!busy) finish_curve(f, b, cur, rows);
-          }
-        }
-      }
-    }
-    if (__all_sync(0xFFFFFFFFu, !busy && exhausted)) break;   // the list is exhausted
-    if (busy) {
-      lc.step(b);
-      if (lc.state == eb::kLsDone && !lc.next_piece(b, true)) {
-        finish_curve(f, b, cur, rows);
-        busy = false;
-      }
-    }
-  }
-  rows = __reduce_add_sync(0xFFFFFFFFu, rows);
-  if (lane == 0 && rows) atomicAdd(f.totals + 1, rows);
+__global__ void __launch_bounds__(kCurveThreads) edge_tree_kernel(FrameView f) {
+  __shared__ TreeXchg<3> xchg[kCurveThreads / 32][32];
+  const int w = threadIdx.x >> 5;
+  const uint32_t half = gridDim.x / 2u;
+  if (blockIdx.x >= half) flatten_trees<2>(f, reinterpret_cast<TreeXchg<2>*>(xchg[w]), half);
+  else flatten_trees<3>(f, xchg[w], half);
 }
 
 __global__ void __launch_bounds__(256) edge_items_kernel(FrameView f) {
@@ -1965,22 +2081,19 @@ static int max_blocks_per_sm(K kernel, int threads, size_t dyn_smem = 0) {
 int launch_edges(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st) {
   if (!f.num_cmds) return 0;
   const int sms = device_sms();
-  static const int max_per_sm = max_blocks_per_sm(edge_pieces_kernel<3, kPiecesClipped>, kCurveThreads);
+  static const int max_per_sm = max_blocks_per_sm(edge_pieces_kernel, kCurveThreads);
   const int per_sm = cfg.cubic_blocks_per_sm > 0 && cfg.cubic_blocks_per_sm < max_per_sm ? cfg.cubic_blocks_per_sm : max_per_sm;
   const uint32_t eb = cfg.edge_block == 64 || cfg.edge_block == 256 ? uint32_t(cfg.edge_block) : 128u;
   classify_kernel<<<cdiv(f.num_cmds, 128), 128, 0, st>>>(f);
   edge_items_kernel<<<cdiv(f.item_capacity ? f.item_capacity : 1, eb), eb, 0, st>>>(f);
-  const uint32_t cubic_grid = uint32_t(sms * per_sm);
-  const uint32_t split_grid = cdiv(f.item_capacity ? f.item_capacity : 1, 128);
-  curve_split_kernel<3><<<split_grid, 128, 0, st>>>(f);
-  curve_split_kernel<2><<<split_grid, 128, 0, st>>>(f);
-  const uint32_t pgrid = cdiv(f.piece_capacity ? f.piece_capacity : 1, kCurveThreads);
-  const uint32_t pieces_grid = pgrid < cubic_grid ? pgrid : cubic_grid;
-  const uint32_t tree_grid = min(pgrid, uint32_t(sms * kTreeBlocksPerSM));
-  edge_tree_kernel<<<tree_grid, kCurveThreads, 0, st>>>(f);
-  edge_pieces_kernel<3, kPiecesClipped><<<pieces_grid, kCurveThreads, 0, st>>>(f);
-  edge_pieces_kernel<2, kPiecesAll><<<pieces_grid, kCurveThreads, 0, st>>>(f);
-  return 7;
+  // every curve kernel has twice the blocks of one kind of curve (the first half cubic, the second quadratic)
+  const uint32_t split_grid = min(cdiv(f.item_capacity ? f.item_capacity : 1, 128), uint32_t(sms) * kSplitBlocksPerSM);
+  curve_split_kernel<<<2 * split_grid, 128, 0, st>>>(f);
+  // as many warps as there may be pieces, up to the grids' limits
+  const uint32_t pgrid = cdiv(f.piece_capacity ? f.piece_capacity : 1, kCurveThreads / 32);
+  edge_pieces_kernel<<<2 * min(pgrid, uint32_t(sms * per_sm)), kCurveThreads, 0, st>>>(f);
+  edge_tree_kernel<<<2 * min(pgrid, uint32_t(sms * kTreeBlocksPerSM)), kCurveThreads, 0, st>>>(f);
+  return 5;
 }
 
 int launch_cmd_tiles(const FrameView& f, uint32_t* cmdrow_counts_per_cmd, cudaStream_t st) {
