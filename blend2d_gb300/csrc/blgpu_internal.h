@@ -244,6 +244,22 @@ struct DevStrokeFig {
   uint32_t param;          // stroke parameter index
 };
 
+// Stroked curves (stroke.cu): their offset quads in chunks from a pool, and where a curve's quads go in
+// the outline: side A forward from vertex `a`, side B backward from vertex `b`.
+constexpr uint32_t kStrokeChunk = 4;                  // quads per chunk
+constexpr uint32_t kStrokeQuadBytes = 64, kStrokeRecBytes = 136;   // sk::OffsetQuad, sk::CurveRec
+enum StrokeCounter : uint32_t { kStrokeCurves = 0, kStrokeChunks = 1, kStrokeCounters = 2 };
+enum CurveDestFlag : uint32_t {
+  kDestSideB = 1u,         // the outline has a side B
+  kDestClosed = 2u,        // of a closed figure
+  kDestLast = 4u           // the curve's last vertex is side B's last one
+};
+struct DevCurveDest {
+  uint32_t a, b;
+  uint32_t count;          // quads; 0: the figure's thread wrote the curve itself
+  uint32_t flags;          // CurveDestFlag
+};
+
 // Width, miter limit, join and caps of a stroke (BLStrokeOptions without the dash array).
 struct DevStrokeParams {
   double width, miter_limit;
@@ -331,8 +347,8 @@ struct FrameView {
   uint32_t num_tiles;
   uint32_t num_rows;
   uint32_t num_lut_jobs;
-  // Stroking: the stroke input paths, one thread per figure counts (stroke_counts: total, A, B,
-  // C | closed << 30 | B taken << 31) and then writes the figure's outline at
+  // Stroking (stroke.cu): the stroke input paths; one thread per figure counts (stroke_counts: total,
+  // A, B, C | closed << 30 | B taken << 31) and then writes the figure's outline at
   // verts / path_cmds[stroke_vert_base + stroke_offsets[fig]].
   const DevStrokeFig* stroke_figs;
   const uint32_t* stroke_order;   // thread -> figure: figures with alike work side by side
@@ -343,6 +359,14 @@ struct FrameView {
   uint32_t* stroke_totals;
   uint32_t* stroke_offsets;   // num_stroke_figs + 1 (the last one: the outline's size)
   uint32_t* stroke_scan_tmp;
+  uint32_t* stroke_counters;  // StrokeCounter
+  uint32_t* stroke_curve_at;  // per stroke vertex: the index of the curve whose command starts there
+  uint2* stroke_curves;       // curve -> its first control vertex, its stroke parameters
+  void* stroke_recs;          // sk::CurveRec per curve
+  void* stroke_pool;          // chunks of sk::OffsetQuad
+  uint32_t* stroke_chunk_next;
+  DevCurveDest* stroke_dests;
+  uint32_t stroke_curve_cap, stroke_chunk_cap;
   uint32_t num_stroke_figs;
   uint32_t stroke_vert_base;
   uint32_t num_segs;

@@ -383,6 +383,10 @@ BLGpuResult Runtime::prepare_strokes(const Frame& fr, FrameView& v, uint32_t& ou
     for (uint32_t k = 0; k < kBuckets; k++) start[k + 1] += start[k];
     for (uint32_t i = 0; i < nf; i++) stroke_order[start[keys[i]]++] = i;
   }
+  // a curve takes two vertices or more; chunks: what a vertex took at most in the frames so far
+  const uint32_t nv = uint32_t(fr.stroke_cmds.size());
+  v.stroke_curve_cap = nv / 2u;
+  v.stroke_chunk_cap = uint32_t(std::min<double>(double(nv) * stroke_chunks_per_vertex, 4e9));
   auto plan = [&](Layout& L) {
     v.stroke_figs = L.take<DevStrokeFig>(nf);
     v.stroke_order = L.take<uint32_t>(nf);
@@ -391,8 +395,15 @@ BLGpuResult Runtime::prepare_strokes(const Frame& fr, FrameView& v, uint32_t& ou
     v.stroke_cmds = L.take<uint8_t>(fr.stroke_cmds.size());
     v.stroke_counts = L.take<uint4>(nf);
     v.stroke_totals = L.take<uint32_t>(nf + 1);
-    v.stroke_offsets = L.take<uint32_t>(nf + 1);
+    v.stroke_offsets = L.take<uint32_t>(nf + 1 + kStrokeCounters);
+    v.stroke_counters = v.stroke_offsets + nf + 1;               // read back with the outline's size
     v.stroke_scan_tmp = L.take<uint32_t>(scan_temp_words(nf + 1));
+    v.stroke_curve_at = L.take<uint32_t>(nv);
+    v.stroke_curves = L.take<uint2>(v.stroke_curve_cap);
+    v.stroke_recs = L.take<char>(size_t(v.stroke_curve_cap) * kStrokeRecBytes);
+    v.stroke_dests = L.take<DevCurveDest>(v.stroke_curve_cap);
+    v.stroke_pool = L.take<char>(size_t(v.stroke_chunk_cap) * kStrokeChunk * kStrokeQuadBytes);
+    v.stroke_chunk_next = L.take<uint32_t>(v.stroke_chunk_cap);
   };
   Layout measure;
   plan(measure);
@@ -417,9 +428,13 @@ BLGpuResult Runtime::prepare_strokes(const Frame& fr, FrameView& v, uint32_t& ou
   BLGPU_CHECK(put(v.stroke_cmds, fr.stroke_cmds.data(), fr.stroke_cmds.size()));
   launch_stroke_count(v, stream);
   BLGPU_CHECK(cudaGetLastError());
-  BLGPU_CHECK(cudaMemcpyAsync(host_totals + 16, v.stroke_offsets + nf, 4, cudaMemcpyDeviceToHost, stream));
-  d2h_bytes += 4;
+  constexpr size_t kBack = sizeof(uint32_t) * (1 + kStrokeCounters);
+  BLGPU_CHECK(cudaMemcpyAsync(host_totals + 16, v.stroke_offsets + nf, kBack, cudaMemcpyDeviceToHost, stream));
+  d2h_bytes += kBack;
   BLGPU_CHECK(cudaStreamSynchronize(stream));
+  // a pool that ran out costs time, not the outline: the next frame's is larger
+  const uint32_t chunks = host_totals[16 + 1 + kStrokeChunks];
+  if (chunks > v.stroke_chunk_cap) stroke_chunks_per_vertex = 1.25 * double(chunks) / double(nv);
   if (host_totals[16] > 0x3FFFFFFFu) return BLGPU_ERROR_DATA_TOO_LARGE;
   outline_verts = host_totals[16];
   strokes_counted = true;

@@ -187,6 +187,7 @@ struct Runtime {
   DeviceBuffer seg_buf;     // segments + their metadata, appended by the edge builders
   DeviceBuffer stroke_buf;  // stroke inputs, per-figure outline counts and offsets
   bool strokes_counted = false;   // the upload's sizing pass left this frame's counts in place
+  double stroke_chunks_per_vertex = 2.0;   // size of the offset quads' pool (prepare_strokes)
   std::vector<uint32_t> stroke_order;   // thread -> figure order of the frame being uploaded
   uint32_t seg_capacity = 0;
   void* host_staging = nullptr;

@@ -1,5 +1,5 @@
-// The path stroker, shared by the device (stroke_count_kernel / stroke_emit_kernel, one thread
-// per figure) and the host (blgpu_stroke_outline_d). Restates bl::PathInternal::PathStroker
+// The path stroker, shared by the device (stroke.cu: the curves' offsets one thread per curve, the
+// figures around them one thread per figure) and the host (blgpu_stroke_outline_d). Restates bl::PathInternal::PathStroker
 // (blend2d/core/pathstroke.cpp:126-971) and the Bezier helpers it uses
 // (blend2d/geometry/bezier_p.h, blend2d/geometry/commons_p.h) operation by operation in double
 // precision without FMA contraction (device code is built with -fmad=false, host code with
@@ -298,6 +298,16 @@ struct Side {
   SK_HD void flush() {
     for (; done < n; done++) sink.put(done, rc[done % kWin], rp[done % kWin]);
   }
+  // `count` quads already stored elsewhere: everything up to and with them is final (a join never
+  // looks back past a curve's end), the last one's vertices stay readable.
+  SK_HD void skip_quads(uint32_t count, V first_control, V control, V end) {
+    flush();
+    if (n < 2) { first_c[1] = kQuad; first_p[1] = first_control; }   // n >= 1: after the figure's move
+    n += 2 * count;
+    done = n;
+    rc[(n - 2) % kWin] = kQuad; rp[(n - 2) % kWin] = control;
+    rc[(n - 1) % kWin] = kOn; rp[(n - 1) % kWin] = end;
+  }
   SK_HD void quarter_arc_to(V p1, V p2) {     // PathAppender::arc_quadrant_to (path_p.h:374-390)
     V p0 = last();
     cubic_to(p0 + (p1 - p0) * kKappa, p2 + (p1 - p2) * kKappa, p2);
@@ -338,11 +348,143 @@ struct FigureCounts {
   SK_HD uint32_t total() const { return a + b_out() + c_out(); }
 };
 
+// One quad of a curve's offset: its control and end points on side A and on side B ...
+struct OffsetQuad {
+  V a1, a2, b1, b2;
+};
+// ... with the curve point it ends at and the unit normal there.
+struct OffsetPiece {
+  OffsetQuad q;
+  V p, n;
+};
+
+// Offsets a quad or cubic to both sides, one offset quad per step (offset_quad, pathstroke.cpp:
+// 860-905, and approximate_cubic_with_quads, bezier_p.h:943-982, unrolled into a state), so the
+// lanes of a warp, each on its own curve, issue the piece arithmetic together however many t-steps,
+// quads and pieces their curves need. The pieces depend only on the curve and the offset.
+struct Offsetter {
+  double d = 0.0, d2 = 0.0;                    // the offset, and twice it
+  bool cubic_ = false, pieces_ = false;
+  uint32_t qn_ = 0, qe_ = 0;                   // quads of the current step start at q_[qn_], end at qe_
+  double t_ = 0.0;                             // the cubic's next t-step
+  V w_[7];                                     // the cubic's remainder in w_[3..6]
+  V q_[5];
+  double ts_[3];
+  QuadPieces it_;
+
+  SK_HD bool active() const { return pieces_ || qn_ < qe_ || cubic_; }
+
+  SK_HD void begin_quad(const V* q) {
+    q_[0] = q[0]; q_[1] = q[1]; q_[2] = q[2];
+    qn_ = 0; qe_ = 2;
+    cubic_ = false; pieces_ = false;
+  }
+
+  SK_HD void begin_cubic(const V* c) {
+    double tol = 54.0 * kSimplifyTolerance;
+    t_ = sk_pow(tol * tol / mag_sq(cubic_identity(c)), 1.0 / 6.0);
+    w_[3] = c[0]; w_[4] = c[1]; w_[5] = c[2]; w_[6] = c[3];
+    qn_ = qe_ = 0;
+    cubic_ = true; pieces_ = false;
+  }
+
+  // One piece; `put(OffsetPiece)` unless it is degenerate.
+  template <class F>
+  SK_HD void step(F&& put) {
+    if (!pieces_) {
+      if (qn_ >= qe_) {                          // the cubic's next t-step: two quads
+        t_ = t_ < 1.0 ? t_ : 1.0;
+        if (t_ >= 0.999) t_ = 1.0;
+        cubic_split(w_ + 3, w_, w_ + 3, t_);
+        cubic_two_quads(w_, q_);
+        qn_ = 0; qe_ = 4;
+        if (t_ >= 1.0) cubic_ = false;
+        else {
+          double prev = t_;
+          t_ = t_ / (1.0 - t_);
+          if (prev - t_ < 1e-3) t_ += 0.01;
+        }
+      }
+      // the next quad, cut at its offset's cusps
+      const V* q = q_ + qn_;
+      qn_ += 2;
+      uint32_t tn = quad_offset_cusps(q, d, ts_);
+      ts_[tn++] = 1.0;
+      it_ = QuadPieces(q, ts_, tn);
+      pieces_ = true;
+    }
+    double t = quad_angle_step(it_.piece, kOffsetParameter);
+    if (!(t > kOffsetQuadEpsilonT && t < 1.0 - kOffsetQuadEpsilonT)) t = 1.0;
+    V head[3];
+    quad_split(it_.piece, head, it_.piece, t);
+    if (head[0] != head[2]) {                    // offset_quad_simple (:885-905)
+      V v0 = head[1] - head[0], v1 = head[2] - head[1];
+      V m0 = unit_normal(head[0] != head[1] ? v0 : v1);
+      V m2 = unit_normal(head[1] != head[2] ? v1 : v0);
+      V m = m0 + m2;
+      V k1 = m * d2 / mag_sq(m);
+      V k2 = m2 * d;
+      put(OffsetPiece{{head[1] + k1, head[2] + k2, head[1] - k1, head[2] - k2}, head[2], m2});
+    }
+    if (t == 1.0 && !it_.next()) pieces_ = false;
+  }
+};
+
+// A curve command offset on its own: valid for a stroker whose current point is `from` (bit for
+// bit), where the command takes none of the stroker's degenerate paths (flat, collinear, cusp).
+struct CurveRec {
+  V from, n_first;                             // the curve's start and its unit normal there
+  OffsetPiece last;
+  uint32_t count;                              // offset quads; 0: not usable
+  uint32_t chunk;                              // the first chunk of its stored quads
+};
+
+SK_HD bool same_bits(V a, V b) {
+#if defined(__CUDA_ARCH__)
+  return __double_as_longlong(a.x) == __double_as_longlong(b.x) && __double_as_longlong(a.y) == __double_as_longlong(b.y);
+#else
+  return a == b && !(a.x == 0.0 && (1.0 / a.x != 1.0 / b.x)) && !(a.y == 0.0 && (1.0 / a.y != 1.0 / b.y));
+#endif
+}
+
+// Sets up `off` for the curve command at cmd[i] (vtx[i]: its first control point, vtx[i - 1]: the
+// vertex before it) as the stroker does when its current point is vtx[i - 1], with the normal the
+// join or the figure's start takes; false where the stroker would not offset it as it is.
+SK_HD bool begin_curve_alone(const uint8_t* cmd, const V* vtx, uint32_t i, Offsetter& off, V& n_first) {
+  const V p0 = vtx[i - 1], p1 = vtx[i];
+  if (cmd[i] == kQuad) {
+    const V v1 = p1 - p0, v2 = vtx[i + 1] - p1;
+    n_first = unit_normal(v1);
+    if (sk_fabs(cross(v2, v1)) <= kCollinearityEpsilon) return false;
+    if (mag_sq(v1) < kLengthEpsilonSq || mag_sq(v2) < kLengthEpsilonSq) return false;
+    off.begin_quad(vtx + i - 1);
+    return true;
+  }
+  const V p[4] = {p0, p1, vtx[i + 1], vtx[i + 2]};
+  if (cubic_is_flat(p, kDegenerateFlatness)) return false;
+  double tc, tl;
+  cubic_inflections(p, tc, tl);
+  if (tl == 0.0 && tc > 0.0 && tc < 1.0) return false;
+  V v1 = p[1] - p0;
+  if (is_zero(v1)) v1 = p[2] - p0;
+  n_first = unit_normal(v1);
+  off.begin_cubic(p);
+  return true;
+}
+
+// No stored curves: every curve is offset by the figure's own stroker.
+struct NoCurves {
+  SK_HD const CurveRec* find(uint32_t, V) const { return nullptr; }
+  SK_HD void place(const CurveRec&, uint32_t, uint32_t) {}
+  SK_HD const OffsetQuad& first_quad(const CurveRec& r) const { return r.last.q; }
+};
+
 // Strokes the figure whose commands are cmd[first, end) (end: where the reference's stroker
 // leaves the figure; the commands were validated). Sinks receive A's and B's vertices.
-template <class SinkA, class SinkB>
+template <class SinkA, class SinkB, class Curves = NoCurves>
 class FigureStroker {
  public:
+  Curves curves_;
   Side<SinkA> a;
   Side<SinkB> b;
   Side<NullSink> c;                            // start cap: at most 9 vertices, never handed out
@@ -350,6 +492,7 @@ class FigureStroker {
   SK_HD FigureStroker(const Params& p) : opt_(p), join_(p.join) {
     d_[0] = p.width * 0.5; d2_[0] = p.width;
     d_[1] = -d_[0]; d2_[1] = -d2_[0];
+    off_.d = d_[0]; off_.d2 = d2_[0];
     if (join_ <= kJoinMiterRound) {             // the miter joins and their fallbacks
       if (join_ == kJoinMiterBevel) join_ = kJoinBevel;
       else if (join_ == kJoinMiterRound) join_ = kJoinRound;
@@ -596,77 +739,25 @@ class FigureStroker {
     });
   }
 
-  SK_HD void offset_quad_piece(V q0, V q1, V q2) {   // offset_quad_simple (:885-905)
-    if (q0 == q2) return;
-    V v0 = q1 - q0, v1 = q2 - q1;
-    V m0 = unit_normal(q0 != q1 ? v0 : v1);
-    V m2 = unit_normal(q1 != q2 ? v1 : v0);
-    p0_ = q2; n0_ = m2;
-    V m = m0 + m2;
-    V k1 = m * d2_[0] / mag_sq(m);
-    V k2 = m2 * d_[0];
-    a.quad_to(q1 + k1, q2 + k2);
-    b.quad_to(q1 - k1, q2 - k2);
-  }
-
-  // --- offsetting, one piece per step ------------------------------------------------------
-  // offset_quad (:860-883) and approximate_cubic_with_quads (bezier_p.h:943-982) unrolled into a
-  // state the figure loop advances by one offset quad piece per iteration, so the lanes of a warp,
-  // each on its own figure, issue the piece arithmetic together however many t-steps, quads and
-  // pieces their curves need.
-  bool cubic_ = false, pieces_ = false;
-  uint32_t qn_ = 0, qe_ = 0;                   // quads of the current step start at q_[qn_], end at qe_
-  double t_ = 0.0;                             // the cubic's next t-step
-  V w_[7];                                     // the cubic's remainder in w_[3..6]
-  V q_[5];
-  double ts_[3];
-  QuadPieces it_;
-
-  SK_HD bool offsetting() const { return pieces_ || qn_ < qe_ || cubic_; }
-
-  SK_HD void begin_quad(const V* q) {
-    q_[0] = q[0]; q_[1] = q[1]; q_[2] = q[2];
-    qn_ = 0; qe_ = 2;
-    cubic_ = false; pieces_ = false;
-  }
-
-  SK_HD void begin_cubic(const V* c) {
-    double tol = 54.0 * kSimplifyTolerance;
-    t_ = sk_pow(tol * tol / mag_sq(cubic_identity(c)), 1.0 / 6.0);
-    w_[3] = c[0]; w_[4] = c[1]; w_[5] = c[2]; w_[6] = c[3];
-    qn_ = qe_ = 0;
-    cubic_ = true; pieces_ = false;
-  }
+  Offsetter off_;
 
   SK_HD void offset_step() {
-    if (!pieces_) {
-      if (qn_ >= qe_) {                          // the cubic's next t-step: two quads
-        t_ = t_ < 1.0 ? t_ : 1.0;
-        if (t_ >= 0.999) t_ = 1.0;
-        cubic_split(w_ + 3, w_, w_ + 3, t_);
-        cubic_two_quads(w_, q_);
-        qn_ = 0; qe_ = 4;
-        if (t_ >= 1.0) cubic_ = false;
-        else {
-          double prev = t_;
-          t_ = t_ / (1.0 - t_);
-          if (prev - t_ < 1e-3) t_ += 0.01;
-        }
-      }
-      // the next quad, cut at its offset's cusps
-      const V* q = q_ + qn_;
-      qn_ += 2;
-      uint32_t tn = quad_offset_cusps(q, d_[0], ts_);
-      ts_[tn++] = 1.0;
-      it_ = QuadPieces(q, ts_, tn);
-      pieces_ = true;
-    }
-    double t = quad_angle_step(it_.piece, kOffsetParameter);
-    if (!(t > kOffsetQuadEpsilonT && t < 1.0 - kOffsetQuadEpsilonT)) t = 1.0;
-    V head[3];
-    quad_split(it_.piece, head, it_.piece, t);
-    offset_quad_piece(head[0], head[1], head[2]);
-    if (t == 1.0 && !it_.next()) pieces_ = false;
+    off_.step([&](const OffsetPiece& o) {
+      p0_ = o.p; n0_ = o.n;
+      a.quad_to(o.q.a1, o.q.a2);
+      b.quad_to(o.q.b1, o.q.b2);
+    });
+  }
+
+  // A curve whose offset quads another thread has computed and stored (CurveRec).
+  SK_HD void stored_curve(const CurveRec& r) {
+    if (!open_) start_with_curve(r.n_first);
+    else curve_join(r.n_first);
+    curves_.place(r, a.n, b.n);
+    const OffsetQuad& f = curves_.first_quad(r);
+    a.skip_quads(r.count, f.a1, r.last.q.a1, r.last.q.a2);
+    b.skip_quads(r.count, f.b1, r.last.q.b1, r.last.q.b2);
+    p0_ = r.last.p; n0_ = r.last.n;
   }
 
   // --- input commands, one per step ----------------------------------------------------------
@@ -689,7 +780,7 @@ class FigureStroker {
     if (!open_) start_with_curve(n1);
     else if (!after_cusp) curve_join(n1);
     else cusp_curve_join(n1);
-    begin_cubic(p);
+    off_.begin_cubic(p);
   }
 
   // One command of the figure (PathStroker::stroke's loop body, pathstroke.cpp:266-456); false
@@ -702,6 +793,13 @@ class FigureStroker {
       i++;
       line_step(p1);
       return true;
+    }
+    if (c == kQuad || c == kCubic) {
+      if (const CurveRec* r = curves_.find(i, p0_)) {
+        i += c == kQuad ? 2 : 3;
+        stored_curve(*r);
+        return true;
+      }
     }
     if (c == kQuad) {
       i += 2;
@@ -727,7 +825,7 @@ class FigureStroker {
       if (mag_sq(v1) < kLengthEpsilonSq || mag_sq(v2) < kLengthEpsilonSq) { line_step(p2); return true; }
       if (!open_) start_with_curve(n1);
       else curve_join(n1);
-      begin_quad(q);
+      off_.begin_quad(q);
       return true;
     }
     if (c == kCubic) {
@@ -790,15 +888,15 @@ class FigureStroker {
 };
 
 // The figure loop of PathStroker::stroke (pathstroke.cpp:256-478), one unit of work per iteration.
-template <class SinkA, class SinkB>
-SK_HD FigureCounts FigureStroker<SinkA, SinkB>::run(const uint8_t* cmd, const V* vtx, uint32_t first, uint32_t end) {
+template <class SinkA, class SinkB, class Curves>
+SK_HD FigureCounts FigureStroker<SinkA, SinkB, Curves>::run(const uint8_t* cmd, const V* vtx, uint32_t first, uint32_t end) {
   FigureCounts out;
   uint32_t i = first;
   p0_ = vtx[i];
   p_start_ = p0_;
   i++;
   for (;;) {
-    if (offsetting()) offset_step();
+    if (off_.active()) offset_step();
     else if (cusp_pending_) { cusp_pending_ = false; cubic_step(cusp_half_, true); }
     else if (!command_step(cmd, vtx, i, end)) break;
   }
@@ -864,10 +962,13 @@ struct ReverseSink {
   SK_HD void fix0(V p) { put(0, kMove, p); }
 };
 
-// Second pass: writes the figure's outline (counts from the first pass) at cmd/xy.
+// Second pass: writes the figure's outline (counts from the first pass) at cmd/xy, but for the quads
+// of stored curves (`curves.place` says where they go).
+template <class Curves = NoCurves>
 SK_HD void emit_figure(const uint8_t* in_cmd, const V* in_vtx, uint32_t first, uint32_t end, const Params& p,
-                       const FigureCounts& fc, uint8_t* out_cmd, double* out_xy) {
-  FigureStroker<ForwardSink, ReverseSink> s(p);
+                       const FigureCounts& fc, uint8_t* out_cmd, double* out_xy, const Curves& curves = Curves()) {
+  FigureStroker<ForwardSink, ReverseSink, Curves> s(p);
+  s.curves_ = curves;
   s.a.sink = ForwardSink{out_cmd, out_xy};
   const uint32_t rb = fc.a;
   s.b.sink = ReverseSink{out_cmd + rb, out_xy + 2 * rb, fc.b, fc.closed, fc.b_ok};
@@ -887,8 +988,11 @@ SK_HD void emit_figure(const uint8_t* in_cmd, const V* in_vtx, uint32_t first, u
 }
 
 // First pass: the figure's outline sizes.
-SK_HD FigureCounts count_figure(const uint8_t* in_cmd, const V* in_vtx, uint32_t first, uint32_t end, const Params& p) {
-  FigureStroker<NullSink, NullSink> s(p);
+template <class Curves = NoCurves>
+SK_HD FigureCounts count_figure(const uint8_t* in_cmd, const V* in_vtx, uint32_t first, uint32_t end, const Params& p,
+                                const Curves& curves = Curves()) {
+  FigureStroker<NullSink, NullSink, Curves> s(p);
+  s.curves_ = curves;
   return s.run(in_cmd, in_vtx, first, end);
 }
 
