@@ -356,84 +356,192 @@ __device__ __forceinline__ void init_builder(eb::Builder& b, const DevCanvas& cv
   b.px = b.py = 0; b.psign = 0; b.pasc = false;
 }
 
-// Walks the figures of a command the way add_from_source does (edgebuilder_p.h:1032-1070) and
-// calls fn(kind, a, b) for every line, curve and closing line.
+// work_counter words of the cubic and of the quadratic / conic curves
+template<int DEG>
+struct CurveWords {
+  static constexpr uint32_t kCurves = DEG == 3 ? 2 : 21;     // curves of the curve list
+  static constexpr uint32_t kPieces = DEG == 3 ? 23 : 25;    // their monotonic pieces
+  static constexpr uint32_t kSafe = DEG == 3 ? 28 : 34;      // pieces the safe loop flattens
+  static constexpr uint32_t kClip = kSafe + 1;               // the other ones
+  static constexpr uint32_t kTreeQueue = kSafe + 2, kClipQueue = kSafe + 3;
+  static constexpr uint32_t kHanded = DEG == 3 ? 38 : 39;    // subtrees of clipped pieces handed to the tree flattener
+};
+// Walks the figures of a command the way add_from_source does (edgebuilder_p.h:1032-1070), by a warp,
+// 32 vertices at a time, and calls fn(kind, a, b, has) for every vertex's line, curve or closing line
+// (at most one; all lanes call it, `has` says whether the lane's vertex has an item).
+// What a vertex is depends on what came before it only through a state of four values - seeking a
+// figure's move, expecting a command, one or two vertices of a curve still to pass - so each vertex is
+// a function on the states (2 bits per state), and a scan of the functions' compositions gives every
+// lane the state it starts from.
 template<typename Fn>
-__device__ void for_each_item(const uint8_t* cmd, int n, Fn&& fn) {
-  int i = 0;
-  for (;;) {
-    if (cmd) { while (i < n && cmd[i] != 0) i++; }
-    if (i >= n) return;
-    int start = i++, prev = start;
-    for (;;) {
-      if (cmd ? (i != n && cmd[i] == 1) : (i != n)) { fn(kItemLine, prev, i); prev = i; i += 1; }
-      else if (cmd && i <= n - 2 && cmd[i] == 2) { fn(kItemQuad, prev, i); prev = i + 1; i += 2; }
-      else if (cmd && i < n - 2 && cmd[i] == 4) { fn(kItemCubic, prev, i); prev = i + 2; i += 3; }
-      else if (cmd && i < n - 2 && cmd[i] == 3) { fn(kItemConic, prev, i); prev = i + 2; i += 2; }
-      else { fn(kItemLine, prev, start); break; }
+__device__ __forceinline__ void for_each_item(const uint8_t* cmd, int n, int lane, Fn&& fn) {
+  if (!cmd) {                                       // a polygon: one figure of lines
+    for (int base = 0; base < n; base += 32) {
+      const int i = base + lane;
+      // vertex i's line ends at i; vertex 0 stands for the closing line
+      fn(uint32_t(kItemLine), i ? i - 1 : n - 1, i, i < n);
     }
-    if (!cmd) return;
+    return;
   }
+  enum : uint32_t { kSeek = 0, kNext = 1, kPass1 = 2, kPass2 = 3 };
+  uint32_t state = kSeek, conics_before = 0;        // conic commands among the 32 vertices before
+  int start = 0;
+  for (int base = 0; base < n; base += 32) {
+    const int i = base + lane;
+    const uint32_t c = i < n ? cmd[i] : 255u;
+    const bool quad = c == 2u && i <= n - 2, cubic = c == 4u && i < n - 2, conic = c == 3u && i < n - 2;
+    const uint32_t figure = c == 0u ? kNext : kSeek;     // a vertex that ends a figure may begin another
+    const uint32_t next = c == 1u ? kNext : cubic ? kPass2 : (quad || conic) ? kPass1 : figure;
+    uint32_t acc = i < n ? figure | (next << 2) | (kNext << 4) | (kPass1 << 6) : 0xE4u;   // past the end: unchanged
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t f = __shfl_up_sync(0xFFFFFFFFu, acc, o);      // first f, then acc
+      const uint32_t both = ((acc >> (2u * (f & 3u))) & 3u) | (((acc >> (2u * ((f >> 2) & 3u))) & 3u) << 2) |
+                            (((acc >> (2u * ((f >> 4) & 3u))) & 3u) << 4) | (((acc >> (2u * (f >> 6))) & 3u) << 6);
+      if (lane >= o) acc = both;
+    }
+    const uint32_t before = __shfl_up_sync(0xFFFFFFFFu, acc, 1);
+    const uint32_t st = lane ? (before >> (2u * state)) & 3u : state;
+    const bool expects = st == kNext && i < n;
+    const bool other = c != 1u && !quad && !cubic && !conic;       // ends the figure: its closing line
+    const uint32_t starts = __ballot_sync(0xFFFFFFFFu, c == 0u && st <= kNext);
+    const uint32_t conics = __ballot_sync(0xFFFFFFFFu, conic && st == kNext);
+    const uint32_t starts_before = starts & ((1u << lane) - 1u);
+    const int figure_start = starts_before ? base + 31 - __clz(starts_before) : start;
+    // the point before a vertex is the vertex before it, but a conic ends on the vertex after its own
+    const bool after_conic = lane >= 2 ? (conics >> (lane - 2)) & 1u : (conics_before >> (30 + lane)) & 1u;
+    const int prev = after_conic ? i : i - 1;
+    fn(cubic ? uint32_t(kItemCubic) : quad ? uint32_t(kItemQuad) : conic ? uint32_t(kItemConic) : uint32_t(kItemLine),
+       prev, other ? figure_start : i, expects);
+    if (starts) start = base + 31 - __clz(starts);
+    conics_before = conics;
+    state = (__shfl_sync(0xFFFFFFFFu, acc, 31) >> (2u * state)) & 3u;
+  }
+  // the last figure's closing line
+  fn(uint32_t(kItemLine), n - 1, start, state == kNext && lane == 0);
 }
 
-__global__ void classify_kernel(FrameView f) {
-  uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= f.counts[kCntCmds]) return;
-  const DevCmd cmd = f.cmds[c];
-  if (cmd.kind != kFillAnalytic) return;
-  f.cmd_bbox[c] = make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN);
-  f.cmds_rw[c].status = 0u;
-  const uint8_t* pc = cmd.geom == kGeomPath ? f.path_cmds + cmd.geom_first : nullptr;
-  const int n = int(cmd.geom_count);
-  // A command with a non-finite transformed point is built whole, by one thread, exactly as the
-  // reference builds it (its clip flags then depend on the order points are visited in).
-  {
-    const DevXform xf = f.xforms[cmd.xform];
-    const double* xy = f.verts + 2ull * cmd.geom_first;
-    bool finite = true;
-    for (int k = 0; k < n; k++) {
-      double x = xy[2 * k], y = xy[2 * k + 1], tx, ty;
-      if (xf.affine) { tx = x * xf.m[0] + y * xf.m[2] + xf.m[4]; ty = x * xf.m[1] + y * xf.m[3] + xf.m[5]; }
-      else { tx = x * xf.m[0] + xf.m[4]; ty = y * xf.m[3] + xf.m[5]; }
-      finite &= isfinite(tx) & isfinite(ty);
+// One warp per command (four in turn in frames of many commands): the finite check, then one item per
+// line and curve. Lines go to the item list (edge_items_kernel); cubic curves to the front of the
+// curve list and quadratic / conic curves to its back. A block counts its commands' items, takes
+// room for all of them with one atomic per list and walks them again to write them. One thread per
+// command, walking its vertices in turn, and three atomics a command: 20,000 curve paths 43 -> 28 us,
+// 10,000 stroke outlines of 230 vertices 515 -> 99 us, the 395,000 commands of 512
+// batch canvases 311 -> 260 us.
+constexpr int kClassifyWarps = 8;
+constexpr uint32_t kClassifyMax = 4;           // commands per warp
+
+__global__ void __launch_bounds__(32 * kClassifyWarps) classify_kernel(FrameView f, uint32_t per_warp) {
+  __shared__ uint3 room[kClassifyWarps * kClassifyMax];       // counts, then first places
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u, num_cmds = f.counts[kCntCmds];
+  const uint32_t block_first = blockIdx.x * kClassifyWarps * per_warp;
+  if (block_first >= num_cmds) return;                        // whole blocks leave together
+  uint32_t whole = 0;                                         // bit k: the warp's command k is built whole
+  for (uint32_t k = 0; k < per_warp; k++) {
+    const uint32_t c = block_first + uint32_t(w) * per_warp + k;
+    uint32_t lines = 0, cubics = 0, quads = 0;
+    if (c < num_cmds && f.cmds[c].kind == kFillAnalytic) {
+      const DevCmd& cmd = f.cmds[c];
+      const int n = int(cmd.geom_count);
+      const uint32_t geom = cmd.geom_first;
+      if (lane == 0) {
+        f.cmd_bbox[c] = make_int4(INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN);
+        f.cmds_rw[c].status = 0u;
+      }
+      // A command with a non-finite transformed point is built whole, by one thread, exactly as the
+      // reference builds it (its clip flags then depend on the order points are visited in). With
+      // coordinates and matrix below 2^500 no transformed point overflows: only larger ones (or
+      // infinities and NaNs) are transformed to see.
+      const DevXform& xf = f.xforms[cmd.xform];
+      const double2* xy = reinterpret_cast<const double2*>(f.verts) + geom;
+      auto large = [](double v) { return ((uint32_t(__double2hiint(v)) >> 20) & 0x7FFu) >= 1023u + 500u; };
+      bool finite = true;
+      const bool large_m = large(xf.m[0]) | large(xf.m[1]) | large(xf.m[2]) | large(xf.m[3]) | large(xf.m[4]) | large(xf.m[5]);
+      for (int i = lane; i < n; i += 32) {
+        const double2 p = xy[i];
+        if (large_m | large(p.x) | large(p.y)) {
+          double tx, ty;
+          if (xf.affine) { tx = p.x * xf.m[0] + p.y * xf.m[2] + xf.m[4]; ty = p.x * xf.m[1] + p.y * xf.m[3] + xf.m[5]; }
+          else { tx = p.x * xf.m[0] + xf.m[4]; ty = p.y * xf.m[3] + xf.m[5]; }
+          finite &= isfinite(tx) & isfinite(ty);
+        }
+      }
+      if (!__all_sync(0xFFFFFFFFu, finite)) {
+        whole |= 1u << k;
+        lines = 1;
+      }
+      else {
+        for_each_item(cmd.geom == kGeomPath ? f.path_cmds + geom : nullptr, n, lane, [&](uint32_t kind, int, int, bool has) {
+          lines += uint32_t(__popc(__ballot_sync(0xFFFFFFFFu, has && kind == kItemLine)));
+          cubics += uint32_t(__popc(__ballot_sync(0xFFFFFFFFu, has && kind == kItemCubic)));
+          quads += uint32_t(__popc(__ballot_sync(0xFFFFFFFFu, has && (kind == kItemQuad || kind == kItemConic))));
+        });
+      }
     }
-    if (!finite) {
-      uint32_t base = atomicAdd(f.work_counter + 1, 1u);
-      if (base < f.item_capacity) f.items[base] = DevItem{c, kItemWhole, 0u, 0u};
-      else atomicOr(f.error_flags, kErrItems);
-      return;
-    }
+    if (lane == 0) room[uint32_t(w) * per_warp + k] = make_uint3(lines, cubics, quads);
   }
-  // Lines go to the item list (edge_items_kernel); cubic curves to the front of the curve list
-  // and quadratic / conic curves to its back (edge_curves_kernel<3> / <2>).
-  uint32_t lines = 0, cubics = 0, quads = 0;
-  for_each_item(pc, n, [&](uint32_t kind, int, int) {
-    lines += kind == kItemLine ? 1u : 0u;
-    cubics += kind == kItemCubic ? 1u : 0u;
-    quads += (kind == kItemQuad) | (kind == kItemConic) ? 1u : 0u;
-  });
-  uint32_t base = lines ? atomicAdd(f.work_counter + 1, lines) : 0u;
-  uint32_t cbase = cubics ? atomicAdd(f.work_counter + 2, cubics) : 0u;
-  uint32_t qbase = quads ? atomicAdd(f.work_counter + 21, quads) : 0u;
-  // cubics fill the curve list from the front and quadratics from the back: together, and each
-  // list on its own, they must fit (the bound is one item per vertex)
-  if (base + lines > f.item_capacity || cbase + cubics > f.item_capacity || qbase + quads > f.item_capacity)
-    atomicOr(f.error_flags, kErrItems);
-  for_each_item(pc, n, [&](uint32_t kind, int a, int b) {
-    const DevItem it{c, kind, uint32_t(a), uint32_t(b)};
-    if (kind == kItemLine) {
-      if (base < f.item_capacity) f.items[base] = it;
-      base++;
+  __syncthreads();
+  if (w == 0) {
+    const bool on = uint32_t(lane) < kClassifyWarps * per_warp;
+    const uint3 mine = on ? room[lane] : make_uint3(0u, 0u, 0u);
+    uint3 sum = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, sum.x, o), y = __shfl_up_sync(0xFFFFFFFFu, sum.y, o),
+                     z = __shfl_up_sync(0xFFFFFFFFu, sum.z, o);
+      if (lane >= o) { sum.x += x; sum.y += y; sum.z += z; }
     }
-    else if (kind == kItemCubic) {
-      if (cbase < f.item_capacity) f.curve_items[cbase] = it;
-      cbase++;
+    uint32_t bx = 0, by = 0, bz = 0;
+    if (lane == 31) {
+      if (sum.x) bx = atomicAdd(f.work_counter + 1, sum.x);
+      if (sum.y) by = atomicAdd(f.work_counter + CurveWords<3>::kCurves, sum.y);
+      if (sum.z) bz = atomicAdd(f.work_counter + CurveWords<2>::kCurves, sum.z);
+      // cubics fill the curve list from the front and quadratics from the back: together, and each
+      // list on its own, they must fit (the bound is one item per vertex)
+      if (bx + sum.x > f.item_capacity || by + sum.y > f.item_capacity || bz + sum.z > f.item_capacity)
+        atomicOr(f.error_flags, kErrItems);
     }
-    else {
-      if (qbase < f.item_capacity) f.curve_items[f.item_capacity - 1u - qbase] = it;
-      qbase++;
+    bx = __shfl_sync(0xFFFFFFFFu, bx, 31);
+    by = __shfl_sync(0xFFFFFFFFu, by, 31);
+    bz = __shfl_sync(0xFFFFFFFFu, bz, 31);
+    if (on) room[lane] = make_uint3(bx + sum.x - mine.x, by + sum.y - mine.y, bz + sum.z - mine.z);
+  }
+  __syncthreads();
+  for (uint32_t k = 0; k < per_warp; k++) {
+    const uint32_t c = block_first + uint32_t(w) * per_warp + k;
+    if (c >= num_cmds || f.cmds[c].kind != kFillAnalytic) continue;
+    uint3 at = room[uint32_t(w) * per_warp + k];
+    if ((whole >> k) & 1u) {
+      if (lane == 0 && at.x < f.item_capacity) f.items[at.x] = DevItem{c, kItemWhole, 0u, 0u};
+      continue;
     }
-  });
+    const DevCmd& cmd = f.cmds[c];
+    for_each_item(cmd.geom == kGeomPath ? f.path_cmds + cmd.geom_first : nullptr, int(cmd.geom_count), lane,
+                  [&](uint32_t kind, int a, int b, bool has) {
+      const uint32_t l = __ballot_sync(0xFFFFFFFFu, has && kind == kItemLine);
+      const uint32_t cu = __ballot_sync(0xFFFFFFFFu, has && kind == kItemCubic);
+      const uint32_t q = __ballot_sync(0xFFFFFFFFu, has && (kind == kItemQuad || kind == kItemConic));
+      if (has) {
+        const DevItem it{c, kind, uint32_t(a), uint32_t(b)};
+        if (kind == kItemLine) {
+          const uint32_t at_l = at.x + uint32_t(__popc(l & lt));
+          if (at_l < f.item_capacity) f.items[at_l] = it;
+        }
+        else if (kind == kItemCubic) {
+          const uint32_t at_c = at.y + uint32_t(__popc(cu & lt));
+          if (at_c < f.item_capacity) f.curve_items[at_c] = it;
+        }
+        else {
+          const uint32_t at_q = at.z + uint32_t(__popc(q & lt));
+          if (at_q < f.item_capacity) f.curve_items[f.item_capacity - 1u - at_q] = it;
+        }
+      }
+      at.x += uint32_t(__popc(l));
+      at.y += uint32_t(__popc(cu));
+      at.z += uint32_t(__popc(q));
+    });
+  }
 }
 
 // The end of a curve's or piece's builder: border runs emitted, segments flushed, the command's
@@ -458,16 +566,6 @@ __device__ __forceinline__ void finish_curve(FrameView& f, eb::Builder& b, uint3
 // that the stacks' and the segment sinks' local memory hits in.
 constexpr int kCurveThreads = 128;
 constexpr uint32_t kSplitBlocksPerSM = 8;      // of each kind of curve
-// work_counter words of the cubic and of the quadratic / conic curves
-template<int DEG>
-struct CurveWords {
-  static constexpr uint32_t kCurves = DEG == 3 ? 2 : 21;     // curves of the curve list
-  static constexpr uint32_t kPieces = DEG == 3 ? 23 : 25;    // their monotonic pieces
-  static constexpr uint32_t kSafe = DEG == 3 ? 28 : 34;      // pieces the safe loop flattens
-  static constexpr uint32_t kClip = kSafe + 1;               // the other ones
-  static constexpr uint32_t kTreeQueue = kSafe + 2, kClipQueue = kSafe + 3;
-  static constexpr uint32_t kHanded = DEG == 3 ? 38 : 39;    // subtrees of clipped pieces handed to the tree flattener
-};
 // Idle lanes a warp waits for before it takes new pieces: each refill's set-up costs the warp its
 // FP64 instructions whatever the number of lanes refilled. On the batched workload 24 and 28
 // measured 246-248 ms per step, 16 and 20 250 ms, 32 251 ms, 8 257 ms and 4 259 ms.
@@ -2084,7 +2182,9 @@ int launch_edges(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st) {
   static const int max_per_sm = max_blocks_per_sm(edge_pieces_kernel, kCurveThreads);
   const int per_sm = cfg.cubic_blocks_per_sm > 0 && cfg.cubic_blocks_per_sm < max_per_sm ? cfg.cubic_blocks_per_sm : max_per_sm;
   const uint32_t eb = cfg.edge_block == 64 || cfg.edge_block == 256 ? uint32_t(cfg.edge_block) : 128u;
-  classify_kernel<<<cdiv(f.num_cmds, 128), 128, 0, st>>>(f);
+  // four commands a warp once one each would be more than a wave of blocks
+  const uint32_t per_warp = f.num_cmds > uint32_t(sms) * 8u * kClassifyWarps ? kClassifyMax : 1u;
+  classify_kernel<<<cdiv(f.num_cmds, kClassifyWarps * per_warp), 32 * kClassifyWarps, 0, st>>>(f, per_warp);
   edge_items_kernel<<<cdiv(f.item_capacity ? f.item_capacity : 1, eb), eb, 0, st>>>(f);
   // every curve kernel has twice the blocks of one kind of curve (the first half cubic, the second quadratic)
   const uint32_t split_grid = min(cdiv(f.item_capacity ? f.item_capacity : 1, 128), uint32_t(sms) * kSplitBlocksPerSM);
