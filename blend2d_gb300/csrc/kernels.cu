@@ -1525,7 +1525,10 @@ int launch_frame_gate(const FrameView& f, cudaStream_t st) {
   return 1;
 }
 
-constexpr uint32_t kRecSolid = 0x80000000u;   // command-list record: the style is solid, its colour in the record
+// Command-list records: word 0.w is the command's kind (bits 0-1), flags (2-3), alpha (4-11), its style's
+// fetch kind and dither flag; word 1.z the style with bit 31 set when it is solid, its colour in 1.w.
+constexpr uint32_t kRecSolid = 0x80000000u;
+constexpr uint32_t kRecFetchShift = 16, kRecDither = 1u << 20;
 
 // Per tile row: commands overlapping the row in painter's order (one block per row).
 __global__ void row_fill_kernel(FrameView f, const uint32_t* row_canvas) {
@@ -1555,8 +1558,10 @@ __global__ void row_fill_kernel(FrameView f, const uint32_t* row_canvas) {
       // nor the style.
       const DevCmd& cmd = f.cmds[c];
       const uint32_t ctx = f.cmd_tile_x[c];
-      const uint32_t meta = cmd.kind | (cmd.flags << 2) | (cmd.alpha << 4);
-      const bool solid = f.styles[cmd.style].fetch == kFetchSolid;
+      const DevStyle& style = f.styles[cmd.style];
+      const bool solid = style.fetch == kFetchSolid;
+      const uint32_t meta = cmd.kind | (cmd.flags << 2) | (cmd.alpha << 4) | (style.fetch << kRecFetchShift) |
+                            (style.dither ? kRecDither : 0u);
       uint4* rec = f.row_recs + 2u * (out + pos);
       f.row_box[out + pos] = make_uint2(f.cmd_xr[c], f.cmd_yr[c]);
       rec[0] = make_uint4(c, f.cmd_xr[c], f.cmd_yr[c], meta);
@@ -1585,6 +1590,7 @@ __global__ void row_fill_kernel(FrameView f, const uint32_t* row_canvas) {
 
 constexpr int kStripsPerTile = kTileH / kStripRows;
 constexpr int kFineWarps = kFineThreads / 32;
+constexpr int kFineBlocksPerSM = 4;
 constexpr int kSlotPixels = kStripRows * kTileW;
 constexpr int kCoverWarps = 4;
 
@@ -1662,51 +1668,45 @@ __global__ void __launch_bounds__(32 * kCoverWarps) coverage_kernel(FrameView f)
 // lane from the coverage pass, box fills compute theirs, then fetch + SrcOver/SrcCopy.
 // ---------------------------------------------------------------------------------------------
 
-// The lane's 4 masks of command `ci` in its strip: analytic commands from the slot's masks (or the
-// backdrop alone when no segment reaches the slot: `mw` is then the row's backdrop), boxes from
+// Masks of the lane's four pixels as bytes of a word, for a command without stored masks: boxes from
 // their rectangles.
-__device__ __forceinline__ void strip_masks(const FrameView& f, uint32_t ckind, uint32_t ci, uint32_t cmeta,
-                                            uint32_t cnseg, uint32_t mw, int xp, int y, uint32_t m[4]) {
-  const uint32_t alpha = cmeta & 0xFFFFu;
-  if (ckind == kFillAnalytic) {
-    if (cnseg) {
-      m[0] = mw & 0xFFu; m[1] = (mw >> 8) & 0xFFu; m[2] = (mw >> 16) & 0xFFu; m[3] = mw >> 24;
+__device__ __forceinline__ uint32_t box_masks(const FrameView& f, uint32_t kind, uint32_t ci, uint32_t alpha, uint32_t xr,
+                                              uint32_t yr, int xp, int y) {
+  uint32_t w = 0;
+  if (kind == kFillBoxA) {           // the pixel box is the command's own columns and rows
+    const int x0 = int(xr & 0xFFFFu), x1 = int(xr >> 16);
+    if (y >= int(yr & 0xFFFFu) && y <= int(yr >> 16)) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) w |= (xp + k >= x0 && xp + k <= x1) ? alpha << (8 * k) : 0u;
     }
-    else {
-      // no segment reaches this slot: every pixel of a row has the row's carried-in coverage
-      const uint32_t rule = ((cmeta >> 16) & 2u) ? 0x1FFu : 0xFFFFFFFFu;
-      m[0] = px::calc_mask((256u << 9) + mw, rule, alpha);
-      m[1] = m[2] = m[3] = m[0];
-    }
+    return w;
   }
-  else {
-    const DevCmd& cmd = f.cmds[ci];
-    if (ckind == kFillBoxA) {
-      bool in_y = y >= cmd.box[1] && y < cmd.box[3];
+  const DevCmd& cmd = f.cmds[ci];
+  if (kind == kFillMaskA) {
+    // FillMask_Base's vmask spans (fillgeneric_p.h:67-162, compopgeneric_p.h:165-183): the mask
+    // byte, times the fill alpha below 255 (udiv255)
+    const bool in_y = y >= cmd.box[1] && y < cmd.box[3];
+    const uint8_t* row = reinterpret_cast<const uint8_t*>(f.images) +
+                         ((uint64_t(cmd.xform) << 32) | cmd.geom_first) + int64_t(y - cmd.box[1]) * cmd.geom_count;
 #pragma unroll
-      for (int k = 0; k < 4; k++) m[k] = (in_y && xp + k >= cmd.box[0] && xp + k < cmd.box[2]) ? alpha : 0u;
-    }
-    else if (ckind == kFillMaskA) {
-      // FillMask_Base's vmask spans (fillgeneric_p.h:67-162, compopgeneric_p.h:165-183): the mask
-      // byte, times the fill alpha below 255 (udiv255)
-      const bool in_y = y >= cmd.box[1] && y < cmd.box[3];
-      const uint8_t* row = reinterpret_cast<const uint8_t*>(f.images) +
-                           ((uint64_t(cmd.xform) << 32) | cmd.geom_first) + int64_t(y - cmd.box[1]) * cmd.geom_count;
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        uint32_t v = 0u;
-        if (in_y && xp + k >= cmd.box[0] && xp + k < cmd.box[2]) {
-          v = __ldg(row + (xp + k - cmd.box[0]));
-          if (alpha < 255u) v = ((v * alpha + 0x80u) * 0x101u) >> 16;
-        }
-        m[k] = v;
+    for (int k = 0; k < 4; k++) {
+      if (in_y && xp + k >= cmd.box[0] && xp + k < cmd.box[2]) {
+        uint32_t v = __ldg(row + (xp + k - cmd.box[0]));
+        if (alpha < 255u) v = ((v * alpha + 0x80u) * 0x101u) >> 16;
+        w |= v << (8 * k);
       }
     }
-    else {
-#pragma unroll
-      for (int k = 0; k < 4; k++) m[k] = px::box_u_mask(cmd.box, alpha, xp + k, y);
-    }
+    return w;
   }
+#pragma unroll
+  for (int k = 0; k < 4; k++) w |= px::box_u_mask(cmd.box, alpha, xp + k, y) << (8 * k);
+  return w;
+}
+
+// A word of four equal mask bytes for a slot no segment reaches: every pixel of a row has the row's
+// carried-in coverage `bd`.
+__device__ __forceinline__ uint32_t uniform_mask(uint32_t bd, uint32_t flags, uint32_t alpha) {
+  return px::calc_mask((256u << 9) + bd, (flags & 2u) ? 0x1FFu : 0xFFFFFFFFu, alpha);
 }
 
 // Slot of an analytic command in strip row `strip_row`, tile column tx, from its list records
@@ -1717,6 +1717,12 @@ __device__ __forceinline__ uint32_t strip_slot(const FrameView& f, uint32_t slot
   const uint32_t slot = slot0 + (strip_row - ((yr & 0xFFFFu) >> kStripShift)) * (tcols >> 16) + (uint32_t(tx) - (tcols & 0xFFFFu));
   nseg = f.slot_mask[slot];
   return slot;
+}
+
+// The bytes of a lane's mask word whose pixels lie on the canvas.
+__device__ __forceinline__ uint32_t pixels_on_canvas(int xp, int y, const DevCanvas& cv) {
+  const int n = y < cv.h ? min(max(cv.w - xp, 0), 4) : 0;
+  return n == 4 ? 0xFFFFFFFFu : (1u << (8 * n)) - 1u;
 }
 
 // Occlusion, per strip: a SrcCopy command whose mask is 255 on every pixel of the strip writes its
@@ -1746,7 +1752,7 @@ __global__ void __launch_bounds__(kFineThreads) cull_kernel(FrameView f) {
     const uint32_t strip_row = uint32_t(row0) >> kStripShift;
     const int row1 = min(row0 + kStripRows, cv.h) - 1;
     const int y = row0 + prow, xp = x_base + pcol;
-    const bool row_ok = y < cv.h;
+    const uint32_t on_canvas = pixels_on_canvas(xp, y, cv);
     const uint32_t list_first = f.row_offsets[row_id];
     const uint32_t list_count = f.row_counts[row_id];
     const uint32_t strip_y = uint32_t(row0) | (uint32_t(row1) << 16);
@@ -1764,7 +1770,7 @@ __global__ void __launch_bounds__(kFineThreads) cull_kernel(FrameView f) {
           const uint4* rec = f.row_recs + 2u * (list_first + uint32_t(cb + lane));
           ra = rec[0];
           rb = rec[1];
-          cand = ((ra.w >> 2) & 1u) && (ra.w >> 4) == 255u;
+          cand = ((ra.w >> 2) & 1u) && ((ra.w >> 4) & 0xFFu) == 255u;
         }
       }
       uint32_t todo = __ballot_sync(0xFFFFFFFFu, cand);
@@ -1774,20 +1780,20 @@ __global__ void __launch_bounds__(kFineThreads) cull_kernel(FrameView f) {
         todo &= ~(1u << bit);
         const uint32_t ci = __shfl_sync(0xFFFFFFFFu, ra.x, bit);
         const uint32_t rmeta = __shfl_sync(0xFFFFFFFFu, ra.w, bit);
-        const uint32_t ckind = rmeta & 3u;
-        const uint32_t cmeta = (((rmeta >> 2) & 3u) << 16) | (rmeta >> 4);
-        uint32_t cnseg = 0, mw = 0;
+        const uint32_t ckind = rmeta & 3u, calpha = (rmeta >> 4) & 0xFFu;
+        const uint32_t cxr = __shfl_sync(0xFFFFFFFFu, ra.y, bit), cyr = __shfl_sync(0xFFFFFFFFu, ra.z, bit);
+        uint32_t mw = 0;
         if (ckind == kFillAnalytic) {
+          uint32_t cnseg = 0;
           const uint32_t slot = strip_slot(f, __shfl_sync(0xFFFFFFFFu, rb.x, bit), __shfl_sync(0xFFFFFFFFu, rb.y, bit),
-                                           __shfl_sync(0xFFFFFFFFu, ra.z, bit), strip_row, tx, cnseg);
+                                           cyr, strip_row, tx, cnseg);
           mw = cnseg ? reinterpret_cast<const uint32_t*>(f.masks + size_t(cnseg - 1u) * kSlotPixels)[lane]
-                     : f.backdrop[size_t(slot) * kStripRows + prow];
+                     : uniform_mask(f.backdrop[size_t(slot) * kStripRows + prow], (rmeta >> 2) & 3u, calpha) * 0x01010101u;
         }
-        uint32_t m[4];
-        strip_masks(f, ckind, ci, cmeta, cnseg, mw, xp, y, m);
-        bool full = true;
-#pragma unroll
-        for (int k = 0; k < 4; k++) full &= !(row_ok && xp + k < cv.w) || m[k] == 255u;
+        else {
+          mw = box_masks(f, ckind, ci, calpha, cxr, cyr, xp, y);
+        }
+        const bool full = (mw | ~on_canvas) == 0xFFFFFFFFu;
         if (__all_sync(0xFFFFFFFFu, full)) { start = uint32_t(cb + bit); found = true; break; }
       }
       if (found) break;
@@ -1796,10 +1802,73 @@ __global__ void __launch_bounds__(kFineThreads) cull_kernel(FrameView f) {
   }
 }
 
-// 5 resident blocks per SM (48 registers, a few spilled): the composite waits on dependent loads,
-// and the extra warps hide more of them than the spills cost (curves frame 2.98 -> 2.95 ms; 6
-// blocks, 40 registers, measured the same as 5).
-__global__ void __launch_bounds__(kFineThreads, 5) fine_kernel(FrameView f) {
+// The four pixels of a lane composited with their sources and mask bytes. A zero mask byte leaves
+// its pixel as it is (SrcOver: the scaled source is 0 and d * 255 / 255 gives d; SrcCopy likewise),
+// so no pixel needs a branch.
+__device__ __forceinline__ void composite4(uint32_t pix[4], const uint32_t sv[4], uint32_t mw, bool src_copy) {
+  if (src_copy) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) pix[k] = px::src_copy(pix[k], sv[k], __byte_perm(mw, 0u, 0x4440u + k));
+  }
+  else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) pix[k] = px::src_over(pix[k], sv[k], __byte_perm(mw, 0u, 0x4440u + k));
+  }
+}
+
+// Sources of the lane's four pixels (those with a mask byte) for a gradient style.
+__device__ __forceinline__ void gradient4(const FrameView& f, uint32_t style, uint32_t fetch, bool dither, uint32_t row_state,
+                                          int xp, int y, uint32_t mw, uint32_t sv[4]) {
+  const DevStyle& st = f.styles[style];
+  const uint4 common = *reinterpret_cast<const uint4*>(&st.maxi);      // maxi, rori, con_maxi, con_rori
+  const uint32_t* lut = f.luts + st.lut_offset;
+  uint32_t idx[4];
+  if (fetch <= kFetchLinearRoR) {
+    const uint64_t dt = st.lin_dt;
+    uint64_t pt = st.lin_pt0 + uint64_t(uint32_t(y)) * st.lin_dy + uint64_t(uint32_t(xp)) * dt;
+#pragma unroll
+    for (int k = 0; k < 4; k++, pt += dt) idx[k] = px::grad_index(uint32_t(pt >> 32), fetch == kFetchLinearPad, common.x, common.y);
+  }
+  else {
+    const float4 rs = f.row_states[row_state];
+    if (fetch <= kFetchRadialRoR) {
+      const float2 r = *reinterpret_cast<const float2*>(&st.rad_bd);   // bd, ddd
+#pragma unroll
+      for (int k = 0; k < 4; k++) idx[k] = px::radial_index(r.x, r.y, rs.x, rs.y, rs.z, xp + k, fetch == kFetchRadialPad, common.x, common.y);
+    }
+    else {
+      const float4 q = *reinterpret_cast<const float4*>(st.con_q);
+      const float4 n = *reinterpret_cast<const float4*>(&st.con_n1);   // n1, n2, n4, offset
+      const float xx = st.con_xx;
+#pragma unroll
+      for (int k = 0; k < 4; k++) idx[k] = px::conic_index(q, n, xx, rs.x, rs.y, rs.z, xp + k, int32_t(common.z), common.w);
+    }
+  }
+  if (!dither) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) sv[k] = (mw >> (8 * k)) & 0xFFu ? __ldg(lut + idx[k]) : 0u;
+  }
+  else {
+    // 64-bit entries (lut_offset is even) + the ordered-dither threshold of each pixel
+    uint2 e[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      e[k] = (mw >> (8 * k)) & 0xFFu ? __ldg(reinterpret_cast<const uint2*>(lut) + idx[k]) : make_uint2(0u, 0u);
+#pragma unroll
+    for (int k = 0; k < 4; k++) sv[k] = px::dither_pixel(e[k], px::dither_threshold(xp + k, y));
+  }
+}
+
+// 32-entry chunks of the strip's command list: every lane tests one command's box and gathers what
+// the strip needs of it - a stored mask's index, or the four row masks of a slot no segment reaches, which
+// drops the command when they are all zero - so the loop over the chunk's commands, in painter's order,
+// only broadcasts. It is pipelined by one command: a command's source loads are under way while the
+// one before it is composited. Bound: instruction issue on full grids, and the latency of a strip's
+// chain of commands where few strips have long lists. The whole composite (with the cull pass), against
+// per-pixel branches, one command at a time and masks found in the loop: 512 canvases of the batch 8.4
+// -> 6.0 ms, 20,000 curve paths on 1920x1080 0.66 -> 0.46, 32 requests of up to 1024x1024 0.95 -> 0.56.
+// Four blocks per SM (64 registers): three (80) 6.6 ms on the batch, five (48, spilling) 6.2.
+__global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(FrameView f) {
   const int lane = threadIdx.x & 31;
   const int prow = lane >> 3;            // row within the strip
   const int pcol = (lane & 7) * 4;       // first of this lane's 4 columns
@@ -1822,8 +1891,8 @@ __global__ void __launch_bounds__(kFineThreads, 5) fine_kernel(FrameView f) {
     if (row0 >= cv.h) continue;
     const uint32_t strip_row = uint32_t(row0) >> kStripShift;
     int row1 = min(row0 + kStripRows, cv.h) - 1;     // last row of the strip inside the canvas
-    int y = row0 + prow, xp = x_base + pcol;
-    bool row_ok = y < cv.h;
+    const int y = row0 + prow, xp = x_base + pcol;
+    const uint32_t on_canvas = pixels_on_canvas(xp, y, cv);
     uint32_t* dst = cv.pixels + int64_t(y) * cv.stride + xp;
     // an A8 canvas: one byte per pixel, composited as the alpha byte of a 32-bit pixel (the
     // reference's P8_Alpha operators are its P32 operators' alpha lane); rows start at 16-byte
@@ -1831,7 +1900,7 @@ __global__ void __launch_bounds__(kFineThreads, 5) fine_kernel(FrameView f) {
     uint8_t* dst8 = reinterpret_cast<uint8_t*>(cv.pixels) + int64_t(y) * cv.stride + xp;
 
     uint32_t pix[4];
-    bool full = row_ok && (xp + 3 < cv.w);
+    const bool full = on_canvas == 0xFFFFFFFFu;
     if (cv.a8) {
       if (full) {
         const uint32_t v = *reinterpret_cast<const uint32_t*>(dst8);
@@ -1840,7 +1909,7 @@ __global__ void __launch_bounds__(kFineThreads, 5) fine_kernel(FrameView f) {
       }
       else {
 #pragma unroll
-        for (int k = 0; k < 4; k++) pix[k] = (row_ok && xp + k < cv.w) ? uint32_t(dst8[k]) << 24 : 0u;
+        for (int k = 0; k < 4; k++) pix[k] = ((on_canvas >> (8 * k)) & 1u) ? uint32_t(dst8[k]) << 24 : 0u;
       }
     }
     else if (full) {
@@ -1849,7 +1918,7 @@ __global__ void __launch_bounds__(kFineThreads, 5) fine_kernel(FrameView f) {
     }
     else {
 #pragma unroll
-      for (int k = 0; k < 4; k++) pix[k] = (row_ok && xp + k < cv.w) ? dst[k] : 0u;
+      for (int k = 0; k < 4; k++) pix[k] = ((on_canvas >> (8 * k)) & 1u) ? dst[k] : 0u;
     }
 
     const uint32_t row_id = (cv.row_base << (kTileShift - f.list_shift)) + (uint32_t(row0) >> f.list_shift);
@@ -1859,12 +1928,15 @@ __global__ void __launch_bounds__(kFineThreads, 5) fine_kernel(FrameView f) {
     const uint32_t strip_x = uint32_t(x_base) | (uint32_t(min(x_base + kTileW, cv.w) - 1) << 16);
 
     const uint32_t start = f.strip_start[unit];      // cull_kernel
+    uint32_t pend_mw = 0, pend[4] = {0u, 0u, 0u, 0u};   // the command to composite next
+    bool pend_copy = false;
 
     for (uint32_t base = start & ~31u; base < list_count; base += 32) {
       // commands of this chunk whose pixel bbox overlaps the strip, in painter's order: one pair
       // of list records per lane holds everything the tests and the slot lookup need
       uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
-      bool hit = false;
+      bool hit = false, stored = false;
+      uint32_t masks = 0;                            // index of the stored masks, or a mask byte per row
       if (base + lane < list_count && base + lane >= start) {
         // 8 bytes per entry to find the commands over the strip; their records only for those
         const uint2 bb = f.row_box[list_first + base + lane];
@@ -1874,123 +1946,81 @@ __global__ void __launch_bounds__(kFineThreads, 5) fine_kernel(FrameView f) {
           const uint4* rec = f.row_recs + 2u * (list_first + base + lane);
           ra = rec[0];
           rb = rec[1];
+          if ((ra.w & 3u) == kFillAnalytic) {
+            uint32_t nseg = 0;
+            const uint32_t slot = strip_slot(f, rb.x, rb.y, ra.z, strip_row, tx, nseg);
+            stored = nseg != 0u;
+            masks = nseg - 1u;
+            if (!stored) {
+              const uint4 bd = *reinterpret_cast<const uint4*>(f.backdrop + size_t(slot) * kStripRows);
+              const uint32_t flags = (ra.w >> 2) & 3u, alpha = (ra.w >> 4) & 0xFFu;
+              masks = uniform_mask(bd.x, flags, alpha) | (uniform_mask(bd.y, flags, alpha) << 8) |
+                      (uniform_mask(bd.z, flags, alpha) << 16) | (uniform_mask(bd.w, flags, alpha) << 24);
+              hit = masks != 0u;
+            }
+          }
         }
       }
-      const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, hit);
-      if (!ballot) continue;
-      // Each hit lane looks up its command's slot in parallel (one command per lane), so the
-      // painter's-order loop below only waits on the mask words.
-      uint32_t kind = 0, slot = 0xFFFFFFFFu, nseg = 0, meta = 0;   // meta: flags << 16 | alpha
-      if (hit) {
-        kind = ra.w & 3u;
-        meta = (((ra.w >> 2) & 3u) << 16) | (ra.w >> 4);
-        if (kind == kFillAnalytic) slot = strip_slot(f, rb.x, rb.y, ra.z, strip_row, tx, nseg);
-      }
-      uint32_t todo = ballot;
-      // the first command's mask word, then each next one's while the current one composites
+      uint32_t todo = __ballot_sync(0xFFFFFFFFu, hit);
+      if (!todo) continue;
+      const uint32_t stored_set = __ballot_sync(0xFFFFFFFFu, stored);
+      // the first command's mask word, then each next one's while the current one is under way
+      auto load_masks = [&](int from) -> uint32_t {
+        const uint32_t v = __shfl_sync(0xFFFFFFFFu, masks, from);
+        return (stored_set >> from) & 1u ? reinterpret_cast<const uint32_t*>(f.masks + size_t(v) * kSlotPixels)[lane]
+                                         : __byte_perm(v, 0u, 0x1111u * uint32_t(prow));
+      };
       int bit = __ffs(todo) - 1;
-      uint32_t next_mw = 0;
-      {
-        const uint32_t s0 = __shfl_sync(0xFFFFFFFFu, slot, bit), n0 = __shfl_sync(0xFFFFFFFFu, nseg, bit);
-        if (s0 != 0xFFFFFFFFu)
-          next_mw = n0 ? reinterpret_cast<const uint32_t*>(f.masks + size_t(n0 - 1u) * kSlotPixels)[lane]
-                       : f.backdrop[size_t(s0) * kStripRows + prow];
-      }
+      uint32_t next_mw = load_masks(bit);
       while (todo) {
         todo &= todo - 1;
-        const uint32_t ci = __shfl_sync(0xFFFFFFFFu, ra.x, bit);
-        const uint32_t ckind = __shfl_sync(0xFFFFFFFFu, kind, bit);
-        const uint32_t cmeta = __shfl_sync(0xFFFFFFFFu, meta, bit);
-        const uint32_t cnseg = __shfl_sync(0xFFFFFFFFu, nseg, bit);
-        const uint32_t cstyle = __shfl_sync(0xFFFFFFFFu, rb.z, bit);
-        const uint32_t crs = __shfl_sync(0xFFFFFFFFu, rb.w, bit);
-        const uint32_t cy0 = __shfl_sync(0xFFFFFFFFu, ra.z, bit) & 0xFFFFu;
-        const uint32_t mw = next_mw;
+        const uint32_t info = __shfl_sync(0xFFFFFFFFu, ra.w, bit);
+        const uint32_t style = __shfl_sync(0xFFFFFFFFu, rb.z, bit);
+        const uint32_t extra = __shfl_sync(0xFFFFFFFFu, rb.w, bit);      // colour, or first row state
+        const uint32_t yr = __shfl_sync(0xFFFFFFFFu, ra.z, bit);
+        uint32_t mw = next_mw;
+        if ((info & 3u) != kFillAnalytic)
+          mw = box_masks(f, info & 3u, __shfl_sync(0xFFFFFFFFu, ra.x, bit), (info >> 4) & 0xFFu,
+                         __shfl_sync(0xFFFFFFFFu, ra.y, bit), yr, xp, y);
         if (todo) {
-          const int nb = __ffs(todo) - 1;
-          const uint32_t s1 = __shfl_sync(0xFFFFFFFFu, slot, nb), n1 = __shfl_sync(0xFFFFFFFFu, nseg, nb);
-          if (s1 != 0xFFFFFFFFu)
-            next_mw = n1 ? reinterpret_cast<const uint32_t*>(f.masks + size_t(n1 - 1u) * kSlotPixels)[lane]
-                         : f.backdrop[size_t(s1) * kStripRows + prow];
-          bit = nb;
+          bit = __ffs(todo) - 1;
+          next_mw = load_masks(bit);
         }
-        uint32_t m[4];
-        strip_masks(f, ckind, ci, cmeta, cnseg, mw, xp, y, m);
-
-        if (row_ok && (m[0] | m[1] | m[2] | m[3]) && (cstyle & kRecSolid)) {
-          const bool src_copy = (cmeta >> 16) & 1u;
+        mw &= on_canvas;
+        if (!__any_sync(0xFFFFFFFFu, mw != 0u)) continue;
+        const uint32_t n = uint32_t(__popc((((mw & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | mw) & 0x80808080u));   // nonzero bytes
+        ops += n;
+        uint32_t sv[4] = {0u, 0u, 0u, 0u};
+        const uint32_t fetch = (info >> kRecFetchShift) & 15u;
+        if (style & kRecSolid) {
 #pragma unroll
-          for (int k = 0; k < 4; k++) {
-            if (m[k] && xp + k < cv.w) {
-              pix[k] = px::composite(pix[k], crs, m[k], src_copy);
-              ops++;
-            }
-          }
+          for (int k = 0; k < 4; k++) sv[k] = extra;
         }
-        else if (row_ok && (m[0] | m[1] | m[2] | m[3])) {
-          const DevCmd& cmd = f.cmds[ci];
-          const DevStyle& st = f.styles[cstyle];
-          const bool src_copy = (cmeta >> 16) & 1u;
-          px::RowState rs;
-          if (px::has_row_table(st.fetch)) {
-            const float4 t4 = f.row_states[crs + uint32_t(y - int(cy0))];
-            rs.f0 = t4.x; rs.f1 = t4.y; rs.f2 = t4.z;
-          }
-          else {
-            // the reference initializes its fetcher at the start of each band of an analytic fill
-            int fetch_y0 = ckind == kFillAnalytic ? max(cmd.box[1], (y / cv.band_height) * cv.band_height) : cmd.fetch_y0;
-            rs = px::row_state(st, y, fetch_y0);
-          }
-          uint32_t n = 0;
-          if (px::is_gradient(st.fetch)) {
-            // the 4 pixels' LUT indices first, so their 4 table loads are in flight together
-            const uint32_t* lut = f.luts + st.lut_offset;
-            uint32_t sv[4];
-            if (!st.dither) {
-#pragma unroll
-              for (int k = 0; k < 4; k++) {
-                const bool on = m[k] && xp + k < cv.w;
-                sv[k] = on ? __ldg(lut + px::gradient_index(st, rs, xp + k)) : 0u;
-              }
-            }
-            else {
-              // 64-bit entries (lut_offset is even) + the ordered-dither threshold of each pixel
-              uint2 e[4];
-#pragma unroll
-              for (int k = 0; k < 4; k++) {
-                const bool on = m[k] && xp + k < cv.w;
-                e[k] = on ? __ldg(reinterpret_cast<const uint2*>(lut) + px::gradient_index(st, rs, xp + k))
-                          : make_uint2(0u, 0u);
-              }
-#pragma unroll
-              for (int k = 0; k < 4; k++) sv[k] = px::dither_pixel(e[k], px::dither_threshold(xp + k, y));
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-              if (m[k] && xp + k < cv.w) {
-                pix[k] = px::composite(pix[k], sv[k], m[k], src_copy);
-                n++;
-              }
-            }
-          }
-          else {
-            // one copy of the fetch + composite code: the 4 pixels rotate through slot 0
+        else if (fetch <= kFetchConic) {
+          // a lane without masks may lie outside the command's rows: it reads no row state
+          if (mw) gradient4(f, style, fetch, info & kRecDither, extra + uint32_t(y) - (yr & 0xFFFFu), xp, y, mw, sv);
+        }
+        else {
+          pat_ops += n;
+          // one copy of the fetch code: the 4 pixels rotate through the last place
+          const DevStyle& st = f.styles[style];
+          const px::RowState rs = px::row_state(st, y, 0);
+          uint32_t m = mw;
 #pragma unroll 1
-            for (int k = 0; k < 4; k++) {
-              if (m[0] && xp + k < cv.w) {
-                uint32_t sv = px::fetch(st, rs, xp + k, f.luts, f.images) | st.src_or;
-                pix[0] = px::composite(pix[0], sv, m[0], src_copy);
-                n++;
-              }
-              uint32_t tp = pix[0]; pix[0] = pix[1]; pix[1] = pix[2]; pix[2] = pix[3]; pix[3] = tp;
-              uint32_t tm = m[0]; m[0] = m[1]; m[1] = m[2]; m[2] = m[3]; m[3] = tm;
-            }
+          for (int k = 0; k < 4; k++, m >>= 8) {
+            uint32_t v = 0;
+            if (m & 0xFFu) v = px::fetch(st, rs, xp + k, f.luts, f.images) | st.src_or;
+            sv[0] = sv[1]; sv[1] = sv[2]; sv[2] = sv[3]; sv[3] = v;
           }
-          ops += n;
-          pat_ops += st.fetch >= kFetchPatAlignedPad ? n : 0u;
         }
+        composite4(pix, pend, pend_mw, pend_copy);
+        pend_mw = mw;
+        pend_copy = (info >> 2) & 1u;
+#pragma unroll
+        for (int k = 0; k < 4; k++) pend[k] = sv[k];
       }
     }
+    composite4(pix, pend, pend_mw, pend_copy);
 
     if (cv.a8) {
       if (full) {
@@ -1999,7 +2029,7 @@ __global__ void __launch_bounds__(kFineThreads, 5) fine_kernel(FrameView f) {
       }
       else {
 #pragma unroll
-        for (int k = 0; k < 4; k++) if (row_ok && xp + k < cv.w) dst8[k] = uint8_t(pix[k] >> 24);
+        for (int k = 0; k < 4; k++) if ((on_canvas >> (8 * k)) & 1u) dst8[k] = uint8_t(pix[k] >> 24);
       }
     }
     else if (full) {
@@ -2007,7 +2037,7 @@ __global__ void __launch_bounds__(kFineThreads, 5) fine_kernel(FrameView f) {
     }
     else {
 #pragma unroll
-      for (int k = 0; k < 4; k++) if (row_ok && xp + k < cv.w) dst[k] = pix[k];
+      for (int k = 0; k < 4; k++) if ((on_canvas >> (8 * k)) & 1u) dst[k] = pix[k];
     }
   }
 

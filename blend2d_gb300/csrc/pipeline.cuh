@@ -28,24 +28,24 @@ __device__ __forceinline__ uint64_t div255(uint64_t u) {
 __device__ __forceinline__ uint64_t div256(uint64_t u) { return (u >> 8) & kLaneFF; }
 
 // The same per-channel arithmetic on two 16-bit lanes of a 32-bit word (every product and sum
-// stays below 2^16, so lanes never carry into each other).
-__device__ __forceinline__ uint32_t div255_2x16(uint32_t x) {
-  x += 0x00800080u;
-  return ((x + ((x >> 8) & 0x00FF00FFu)) >> 8) & 0x00FF00FFu;
-}
+// stays below 2^16, so lanes never carry into each other): x holds both lanes plus 0x00800080
+// (an addend of the multiplication that makes x); the quotients are bytes 1 and 3 of the result.
+__device__ __forceinline__ uint32_t div255_hi(uint32_t x) { return x + __byte_perm(x, 0u, 0x4341u); }
+// Bytes 1 and 3 of the red/blue and of the alpha/green word as a pixel.
+__device__ __forceinline__ uint32_t join(uint32_t rb, uint32_t ag) { return __byte_perm(rb, ag, 0x7351u); }
 
 // CompOp_SrcOver_Op / CompOp_SrcCopy_Op (compopgeneric_p.h:24-63) with a mask m in [0, 255].
-__device__ __forceinline__ uint32_t composite(uint32_t d, uint32_t s, uint32_t m, bool src_copy) {
-  const uint32_t kM = 0x00FF00FFu;
-  if (src_copy) {
-    uint32_t im = m ^ 0xFFu;
-    uint32_t rb = div255_2x16((d & kM) * im + (s & kM) * m);
-    uint32_t ag = div255_2x16(((d >> 8) & kM) * im + ((s >> 8) & kM) * m);
-    return rb | (ag << 8);
-  }
-  uint32_t sm = div255_2x16((s & kM) * m) | (div255_2x16(((s >> 8) & kM) * m) << 8);
-  uint32_t ia = (sm >> 24) ^ 0xFFu;
-  return sm + (div255_2x16((d & kM) * ia) | (div255_2x16(((d >> 8) & kM) * ia) << 8));
+__device__ __forceinline__ uint32_t src_copy(uint32_t d, uint32_t s, uint32_t m) {
+  const uint32_t kM = 0x00FF00FFu, kR = 0x00800080u, im = m ^ 0xFFu;
+  const uint32_t rb = div255_hi((d & kM) * im + ((s & kM) * m + kR));
+  const uint32_t ag = div255_hi(__byte_perm(d, 0u, 0x4341u) * im + (__byte_perm(s, 0u, 0x4341u) * m + kR));
+  return join(rb, ag);
+}
+__device__ __forceinline__ uint32_t src_over(uint32_t d, uint32_t s, uint32_t m) {
+  const uint32_t kM = 0x00FF00FFu, kR = 0x00800080u;
+  const uint32_t srb = div255_hi((s & kM) * m + kR), sag = div255_hi(__byte_perm(s, 0u, 0x4341u) * m + kR);
+  const uint32_t ia = (sag >> 24) ^ 0xFFu;
+  return join(srb, sag) + join(div255_hi((d & kM) * ia + kR), div255_hi(__byte_perm(d, 0u, 0x4341u) * ia + kR));
 }
 
 // x86 cvttss2si / cvtss2si semantics (INT_MIN for NaN and out-of-range values).
@@ -175,8 +175,6 @@ __device__ RowState row_state(const DevStyle& st, int y, int fetch_y0) {
   return r;
 }
 
-__device__ __forceinline__ bool is_gradient(uint32_t fetch) { return fetch >= kFetchLinearPad && fetch <= kFetchConic; }
-
 // Threshold of the 16x16 ordered-dither matrix (bayer_matrix_16x16, tables_p.h:449-473) at canvas
 // pixel (x, y), from the matrix's recursive construction instead of a table: the index interleaves
 // the bits of row and column, lowest bits most significant, each pair weighted by the 2x2 pattern
@@ -201,50 +199,42 @@ __device__ __forceinline__ uint32_t dither_pixel(uint2 v, uint32_t dd) {
   return (a << 24) | (r << 16) | (g << 8) | b;
 }
 
-// LUT index of pixel x of a gradient fetcher (linear, radial or conic): the fetchers' per-pixel
-// arithmetic up to the table lookup.
-__device__ __forceinline__ uint32_t gradient_index(const DevStyle& st, const RowState& r, int x) {
-  switch (st.fetch) {
-    case kFetchLinearPad: case kFetchLinearRoR: {
-      uint64_t pt = r.a64 + uint64_t(uint32_t(x)) * st.lin_dt;
-      return grad_index(uint32_t(pt >> 32), st.fetch == kFetchLinearPad, st.maxi, st.rori);
-    }
-    case kFetchRadialPad: case kFetchRadialRoR: {
-      float xf = float(x);
-      float sq_x = xf * xf;
-      float a = sqrtf(fabsf(sq_x * st.rad_ddd + (xf * r.f2 + r.f1)));
-      float v = (xf * st.rad_bd + r.f0) + a;
-      return grad_index(uint32_t(trunc_f(v)), st.fetch == kFetchRadialPad, st.maxi, st.rori);
-    }
-    default: {    // kFetchConic
-      float xf = float(x) * st.con_xx + r.f0;
-      float ax = fabsf(xf);
-      float ay = r.f1;
-      float xy_min = ay < ax ? ay : ax;
-      float xy_max = ax < ay ? ay : ax;
-      float s = __uint_as_float((ax == xy_min ? 0xFFFFFFFFu : 0u) & __float_as_uint(st.con_n4));
-      float p = xy_min / xy_max;
-      float p_sq = p * p;
-      float v = p_sq * st.con_q[3] + st.con_q[2];
-      v = v * p_sq + st.con_q[1];
-      v = v * p_sq + st.con_q[0];
-      v = fabsf(v * p + (-s));
-      v = fabsf(v - __uint_as_float(uint32_t(int32_t(__float_as_uint(xf)) >> 31) & __float_as_uint(st.con_n2)));
-      v = fabsf(v - r.f2) + st.con_offset;
-      int32_t ni = nearby_f(v);
-      return uint32_t(ni < st.con_maxi ? ni : st.con_maxi) & uint32_t(st.con_rori);
-    }
-  }
+// LUT index of pixel x of a radial / conic fetcher: its per-pixel arithmetic up to the table lookup.
+// f0..f2: the row state. (Linear: the fine stage steps the 32.32 position along its pixels.)
+__device__ __forceinline__ uint32_t radial_index(float bd, float ddd, float f0, float f1, float f2, int x, bool pad,
+                                                 uint32_t maxi, uint32_t rori) {
+  float xf = float(x);
+  float sq_x = xf * xf;
+  float a = sqrtf(fabsf(sq_x * ddd + (xf * f2 + f1)));
+  float v = (xf * bd + f0) + a;
+  return grad_index(uint32_t(trunc_f(v)), pad, maxi, rori);
 }
 
+// q: the polynomial; n: n1, n2, n4, offset.
+__device__ __forceinline__ uint32_t conic_index(const float4& q, const float4& n, float xx, float f0, float f1, float f2, int x,
+                                                int32_t maxi, uint32_t rori) {
+  float xf = float(x) * xx + f0;
+  float ax = fabsf(xf);
+  float ay = f1;
+  float xy_min = ay < ax ? ay : ax;
+  float xy_max = ax < ay ? ay : ax;
+  float s = __uint_as_float((ax == xy_min ? 0xFFFFFFFFu : 0u) & __float_as_uint(n.z));
+  float p = xy_min / xy_max;
+  float p_sq = p * p;
+  float v = p_sq * q.w + q.z;
+  v = v * p_sq + q.y;
+  v = v * p_sq + q.x;
+  v = fabsf(v * p + (-s));
+  v = fabsf(v - __uint_as_float(uint32_t(int32_t(__float_as_uint(xf)) >> 31) & __float_as_uint(n.y)));
+  v = fabsf(v - f2) + n.w;
+  int32_t ni = nearby_f(v);
+  return uint32_t(ni < maxi ? ni : maxi) & rori;
+}
+
+// Pattern fetchers (solid colours travel in the command lists, gradients have their own path).
 __device__ __forceinline__ uint32_t fetch(const DevStyle& st, const RowState& r, int x,
                                           const uint32_t* __restrict__ luts, const uint32_t* __restrict__ images) {
   switch (st.fetch) {
-    case kFetchSolid:
-      return st.solid;
-    case kFetchLinearPad: case kFetchLinearRoR: case kFetchRadialPad: case kFetchRadialRoR: case kFetchConic:
-      // 32-bit LUT only: the fine stage fetches gradients (dithered ones too) on its own path
-      return __ldg(luts + st.lut_offset + gradient_index(st, r, x));
     case kFetchPatAlignedPad: case kFetchPatAlignedRepeat: case kFetchPatAlignedRoR: {
       uint32_t kind = st.fetch - kFetchPatAlignedPad;
       int cx = pat_col(st, x, kind);
