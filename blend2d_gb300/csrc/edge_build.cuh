@@ -759,6 +759,39 @@ __device__ __forceinline__ PieceOutside piece_outside(const Pt* pts, int deg, co
   return (above ? l.x > eb.cx1 : f.x > eb.cx1 && l.x >= eb.cx1) ? kRightRun : kCrosses;
 }
 
+// floor(x * 128) of a coordinate in the clip box, 0 <= x < 2^24, with integer instructions.
+__device__ __forceinline__ int fixed7(double x) {
+  const uint64_t b = uint64_t(__double_as_longlong(x));
+  const uint32_t m = uint32_t(((b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) >> 21);   // top 32 bits of the mantissa
+  const int sh = 1047 - int(b >> 52);
+  return sh < 32 ? int(m >> sh) : 0;
+}
+
+// The flatness test of a node inside the clip box in 32 bits: 1 flat, 0 not flat, -1 too close to
+// tell. The decision has to be Mono::is_flat's, whose FP64 operations are two thirds of a node's; the
+// pipe they run on is the flattener's bound (2 operations per clock and SM). Here the coordinates
+// are whole 1/128 units (of 1/256 px), off by less than one, and so are their differences v = last -
+// first and a, b = control - first. Bounded control points stay in the node's box through every
+// split, so |a| and |b| are at most |v| + 1 per axis and a cross product is off by at most 2 (|vx| +
+// |vy|) + 4, and in FP32 by the roundings of two products and their difference, 2^-21 len, more. All of it is 0.05 of the tolerance's 51.2 units: about one node in a thousand is too close to tell.
+template<int DEG>
+__device__ __forceinline__ int flat_guess(const Pt* p) {
+  const int x0 = fixed7(p[0].x), y0 = fixed7(p[0].y);
+  const float vx = float(fixed7(p[DEG].x) - x0), vy = float(fixed7(p[DEG].y) - y0);
+  const float ax = float(fixed7(p[1].x) - x0), ay = float(fixed7(p[1].y) - y0);
+  float d = fabsf(vx * ay - vy * ax);
+  if (DEG == 3) {
+    const float bx = float(fixed7(p[2].x) - x0), by = float(fixed7(p[2].y) - y0);
+    d = fmaxf(d, fabsf(vx * by - vy * bx));
+  }
+  const float len = vx * vx + vy * vy;
+  const float err = 2.0f * (fabsf(vx) + fabsf(vy)) + 4.0f + len * 4.8e-7f;      // 2^-21 len
+  constexpr float kTol = float(0.20 * 256.0 * 128.0);
+  const float limit = kTol * kTol * len, hi = d + err, lo = d - err;
+  if (hi * hi <= limit * 0.999998f) return 1;
+  return lo > 0.0f && lo * lo > limit * 1.000002f ? 0 : -1;
+}
+
 // One node: true for a leaf, else its two halves (Mono::is_flat / split / push / pop).
 template<int DEG>
 __device__ __forceinline__ bool tree_step(const TreeNode<DEG>& n, double tol_sq, TreeNode<DEG>& left, TreeNode<DEG>& right) {
@@ -767,7 +800,8 @@ __device__ __forceinline__ bool tree_step(const TreeNode<DEG>& n, double tol_sq,
 #pragma unroll
   for (int i = 0; i <= DEG; i++) mc.p[i] = n.p[i];
   Step st;
-  if (mc.is_flat(st) || n.level == kStackLevels) return true;
+  const int guess = flat_guess<DEG>(n.p);
+  if (guess > 0 || n.level == kStackLevels || (guess < 0 && mc.is_flat(st))) return true;
   mc.split(st);
   if (DEG == 2) {
     left.p[0] = n.p[0]; left.p[1] = st.p01; left.p[2] = st.p012;

@@ -834,13 +834,17 @@ __global__ void __launch_bounds__(kCurveThreads) edge_pieces_kernel(FrameView f)
 // nodes, and the FP64 instructions (whose cost to the pipe does not depend on the active lanes)
 // serve more of them. The segments are those of the loop flattener, in another order; they are
 // appended for the warp with one atomic per step, and each lane accumulates the command bounds
-// finish_curve would for the run of segments it emits for one command.
+// finish_curve would for the run of segments it emits for one command. Bound: the FP64 pipe (a split's
+// 12 additions) and the latency of the exchange. The flatness test is decided in 32 bits
+// (eb::flat_guess) for all but one node in a thousand: 2.35 -> 1.68 ms on 512 canvases of the batch,
+// 0.32 -> 0.23 on 20,000 curve paths.
 
 // Idle lanes a warp of the tree flattener waits for before it takes new pieces, and its blocks per
-// SM: refills of 16, 24 and 32 lanes and 3, 4 and 6 blocks measured within 1 % of each other on the
-// batched workload (215.6-218.6 ms per step); 16 was the best on the curves frame (2.60 ms).
+// SM. With the 32-bit flatness test 3 blocks and refills of 16 lanes measured 19.42 ms on 512 canvases
+// of the batch and 1.863 ms on 20,000 curve paths, 4 and 8 19.36 and 1.851, 4 and 16 19.24 and 1.835,
+// 5 and 16 19.18 and 1.836, 5 and 24 19.18 and 1.833.
 constexpr int kTreeRefillLanes = 16;
-constexpr int kTreeBlocksPerSM = 3;
+constexpr int kTreeBlocksPerSM = 5;     // of each kind of curve
 
 template<int DEG>
 struct alignas(16) TreeXchg {
