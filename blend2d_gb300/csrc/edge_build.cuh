@@ -759,9 +759,11 @@ __device__ __forceinline__ PieceOutside piece_outside(const Pt* pts, int deg, co
   return (above ? l.x > eb.cx1 : f.x > eb.cx1 && l.x >= eb.cx1) ? kRightRun : kCrosses;
 }
 
-// floor(x * 128) of a coordinate in the clip box, 0 <= x < 2^24, with integer instructions.
+// floor(x * 128) of a coordinate in the clip box, 0 <= x < 2^24, with integer instructions. A curve's
+// split points may leave the box by a rounding error: 0 for a negative one.
 __device__ __forceinline__ int fixed7(double x) {
   const uint64_t b = uint64_t(__double_as_longlong(x));
+  if (b >> 63) return 0;
   const uint32_t m = uint32_t(((b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) >> 21);   // top 32 bits of the mantissa
   const int sh = 1047 - int(b >> 52);
   return sh < 32 ? int(m >> sh) : 0;
@@ -773,7 +775,8 @@ __device__ __forceinline__ int fixed7(double x) {
 // are whole 1/128 units (of 1/256 px), off by less than one, and so are their differences v = last -
 // first and a, b = control - first. Bounded control points stay in the node's box through every
 // split, so |a| and |b| are at most |v| + 1 per axis and a cross product is off by at most 2 (|vx| +
-// |vy|) + 4, and in FP32 by the roundings of two products and their difference, 2^-21 len, more. All of it is 0.05 of the tolerance's 51.2 units: about one node in a thousand is too close to tell.
+// |vy|) + 4, and in FP32 by the roundings of two products and their difference, 2^-21 len, more. All
+// of it is 0.05 of the tolerance's 51.2 units: about one node in a thousand is too close to tell.
 template<int DEG>
 __device__ __forceinline__ int flat_guess(const Pt* p) {
   const int x0 = fixed7(p[0].x), y0 = fixed7(p[0].y);

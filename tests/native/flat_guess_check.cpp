@@ -60,7 +60,8 @@ int main(int argc, char** argv) {
   std::uniform_real_distribution<double> u(0.0, 1.0);
   for (long it = 0; it < n; it++) {
     const double w = std::pow(65535.0, u(rng)), h = std::pow(65535.0, u(rng));
-    const double ox = u(rng) * (65535.0 - w), oy = u(rng) * (65535.0 - h);
+    // a fifth of the curves lie along the box's left or top side, where split points may fall outside
+    const double ox = rng() % 5 ? u(rng) * (65535.0 - w) : 0.0, oy = rng() % 5 ? u(rng) * (65535.0 - h) : 0.0;
     const int grid = int(rng() % 4);             // 0: any; whole, half, 1/256 pixels
     auto coord = [&](double o, double s) {
       double v = o + (u(rng) < 0.1 ? (rng() & 1u ? s : 0.0) : u(rng) * s);
@@ -73,6 +74,9 @@ int main(int argc, char** argv) {
     for (int i = 0; i < 4; i++) p[i] = Pt{coord(ox, w), coord(oy, h)};
     if (rng() % 8 == 0) p[1] = p[0];
     if (rng() % 8 == 0) p[2].y = p[1].y;
+    // starting or ending along the box's side: an extremum there, split off with a rounding error
+    if (rng() % 4 == 0) p[0].y = p[1].y = oy * 256.0;
+    if (rng() % 4 == 0) p[2].x = p[3].x = ox * 256.0;
     if (it & 1) {
       int nout = split_cubic(p);
       for (int k = 0; k < (nout ? nout : 3); k += 3) walk<3>(p + k, rng);
