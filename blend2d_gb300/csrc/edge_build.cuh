@@ -1283,36 +1283,39 @@ struct LaneCurve {
     }
   }
 
-  // One pass of the current loop's body. With kHandOver it returns true, having done nothing, at a
-  // node whose subtree no clip can reach (in an inside loop, ending within the box: its subdivision
-  // points lie between its ends) and that is far from flat: the caller may have the subtree's
-  // segments emitted elsewhere (a TreeNode of points mc.p, level mc.sp) and call skip_node, or call
-  // split_node to go on here. Squared distances fall to 1/16 with each split, so a node beyond 256
-  // times the limit has at least four leaves or so: fewer are not worth the hand-over.
-  template<bool kHandOver = false>
-  __device__ __forceinline__ bool step(Builder& eb) {
+  // One pass of the current loop's body. With kDefer it returns, having done nothing,
+  //  - kStepLeaf at a leaf: the caller runs leaf() when it suits the warp;
+  //  - kStepHand at a node whose subtree no clip can reach (in an inside loop, ending within the box:
+  //    its subdivision points lie between its ends) and that is far from flat: the caller may have
+  //    the subtree's segments emitted elsewhere (a TreeNode of points mc.p, level mc.sp) and call
+  //    skip_node, or call split_node to go on here. Squared distances fall to 1/16 with each split, so
+  //    a node beyond 256 times the limit has at least four leaves or so: fewer are not worth it.
+  enum StepResult : int { kStepOn = 0, kStepHand, kStepLeaf };
+  template<bool kDefer = false>
+  __device__ __forceinline__ StepResult step(Builder& eb) {
     switch (state) {
-      case kLsLTop: out = mc.first().x >= eb.cx1; if (out) { exit_loop(eb, true); return false; } break;
-      case kLsLLeft: out = mc.first().y >= eb.cy1; if (out) { exit_loop(eb, false); return false; } break;
-      case kLsRTop: out = mc.first().x <= eb.cx0; if (out) { exit_loop(eb, false); return false; } break;
-      case kLsRRight: out = mc.first().y >= eb.cy1; if (out) { exit_loop(eb, true); return false; } break;
+      case kLsLTop: out = mc.first().x >= eb.cx1; if (out) { exit_loop(eb, true); return kStepOn; } break;
+      case kLsLLeft: out = mc.first().y >= eb.cy1; if (out) { exit_loop(eb, false); return kStepOn; } break;
+      case kLsRTop: out = mc.first().x <= eb.cx0; if (out) { exit_loop(eb, false); return kStepOn; } break;
+      case kLsRRight: out = mc.first().y >= eb.cy1; if (out) { exit_loop(eb, true); return kStepOn; } break;
       default: break;
     }
     Step st;
     if (!mc.is_flat(st)) {
-      if (kHandOver && st.value > 256.0 * st.limit && mc.last().y < eb.cy1 &&
+      if (kDefer && st.value > 256.0 * st.limit && mc.last().y < eb.cy1 &&
           ((state == kLsLIn && mc.last().x <= eb.cx1) || (state == kLsRIn && mc.last().x >= eb.cx0)))
-        return true;
+        return kStepHand;
       mc.split(st);
       const Pt m = mc.step_mid(st);
       const bool discard = ((state == kLsLTop) | (state == kLsRTop)) ? (m.y <= eb.cy0)
                          : state == kLsLLeft ? (m.x <= eb.cx0)
                          : state == kLsRRight ? (m.x >= eb.cx1) : false;
-      if (discard) { mc.discard_and_advance(st); return false; }
-      if (mc.can_push()) { mc.push(st); return false; }
+      if (discard) { mc.discard_and_advance(st); return kStepOn; }
+      if (mc.can_push()) { mc.push(st); return kStepOn; }
     }
+    if (kDefer) return kStepLeaf;
     leaf(eb);
-    return false;
+    return kStepOn;
   }
 
   // The current node's subtree has been handed over: go on behind its last leaf.

@@ -570,6 +570,9 @@ constexpr uint32_t kSplitBlocksPerSM = 8;      // of each kind of curve
 // FP64 instructions whatever the number of lanes refilled. On the batched workload 24 and 28
 // measured 246-248 ms per step, 16 and 20 250 ms, 32 251 ms, 8 257 ms and 4 259 ms.
 constexpr uint32_t kPieceRefillLanes = 24;
+// ... and lanes at a leaf it waits for before it clips and emits them (8, 12, 16 and 20 measured 18.78,
+// 18.70, 18.65 and 18.58 ms on the same canvases, 1.827, 1.823, 1.822 and 1.829 ms on 20,000 curve paths).
+constexpr uint32_t kPieceLeafLanes = 16;
 
 // Curves in three kernels, each with the cubic curves in the first half of its blocks and the
 // quadratic and conic ones in the second, so that neither kind's tail waits for the other's and a
@@ -744,17 +747,26 @@ __device__ void flatten_clipped(FrameView& f, uint32_t blocks) {
   const uint32_t room = handed_room(f, n_cubic, n_quad), share = piece_share(n_items, blocks);
   const uint32_t* const list = f.piece_list + (DEG == 3 ? 0u : f.piece_capacity);
   uint32_t* queue = f.work_counter + W::kClipQueue;
+  using Lane = eb::LaneCurve<DEG, eb::CachedStack<DEG>>;
   eb::Builder b;
-  eb::LaneCurve<DEG, eb::CachedStack<DEG>> lc;
-  bool busy = false, exhausted = false;
+  Lane lc;
+  enum Phase : int { kIdle = 0, kStepping, kAtLeaf, kDone };
+  int phase = kIdle;
+  bool exhausted = false;
   uint32_t cur = 0, rows = 0;
+  // few pieces: no lane waits for others
+  const uint32_t refill_lanes = share == 32u ? kPieceRefillLanes : 33u, leaf_lanes = share == 32u ? kPieceLeafLanes : 1u;
 
   for (;;) {
     // hand the next pieces of the list to the idle lanes (one atomic per warp), once enough lanes
-    // are idle that the set-up's FP64 instructions serve several pieces at once
-    const uint32_t want = __ballot_sync(0xFFFFFFFFu, !busy && !exhausted);
-    const bool none = !__any_sync(0xFFFFFFFFu, busy);
-    if (want && ((share == 32u && uint32_t(__popc(want)) >= kPieceRefillLanes) || none)) {
+    // are idle that the set-up's and the ending's instructions serve several pieces at once
+    const uint32_t want = __ballot_sync(0xFFFFFFFFu, phase == kDone || (phase == kIdle && !exhausted));
+    const bool none = !__any_sync(0xFFFFFFFFu, phase == kStepping || phase == kAtLeaf);
+    if (want && (uint32_t(__popc(want)) >= refill_lanes || none)) {
+      if (phase == kDone) {
+        finish_curve(f, b, cur, rows);
+        phase = kIdle;
+      }
       const int leader = __ffs(want) - 1;
       const uint32_t take = none ? min(uint32_t(__popc(want)), share) : uint32_t(__popc(want));
       uint32_t base = 0;
@@ -762,7 +774,7 @@ __device__ void flatten_clipped(FrameView& f, uint32_t blocks) {
       base = __shfl_sync(0xFFFFFFFFu, base, leader);
       if (base >= n_items) exhausted = true;
       const uint32_t rank = uint32_t(__popc(want & lt));
-      if (!busy && !exhausted && rank < take) {
+      if (((want >> lane) & 1u) && !exhausted && rank < take) {
         const uint32_t t = base + rank;
         if (t >= n_items) {
           exhausted = true;
@@ -780,14 +792,26 @@ __device__ void flatten_clipped(FrameView& f, uint32_t blocks) {
             eb::Pt pts[DEG + 1];
 #pragma unroll
             for (int i = 0; i <= DEG; i++) pts[i] = eb::Pt{pc.p[i].x, pc.p[i].y};
-            busy = lc.begin_piece(b, pts, pc.any);
-            if (!busy) finish_curve(f, b, cur, rows);
+            phase = lc.begin_piece(b, pts, pc.any) ? kStepping : kDone;
           }
         }
       }
     }
-    if (__all_sync(0xFFFFFFFFu, !busy && exhausted)) break;   // the list is exhausted
-    const bool hand = busy && lc.template step<true>(b);
+    if (__all_sync(0xFFFFFFFFu, phase == kIdle && exhausted)) break;   // the list is exhausted
+    bool hand = false;
+    if (phase == kStepping) {
+      const int r = lc.template step<true>(b);
+      if (r == Lane::kStepLeaf) phase = kAtLeaf;
+      hand = r == Lane::kStepHand;
+    }
+    // leaves, where the clips are: together, when enough lanes stand at one or no lane can step on
+    const uint32_t leaves = __ballot_sync(0xFFFFFFFFu, phase == kAtLeaf);
+    if (leaves && (uint32_t(__popc(leaves)) >= leaf_lanes || !__any_sync(0xFFFFFFFFu, phase == kStepping))) {
+      if (phase == kAtLeaf) {
+        lc.leaf(b);
+        phase = kStepping;
+      }
+    }
     const uint32_t hands = __ballot_sync(0xFFFFFFFFu, hand);
     if (hands) {
       const int leader = __ffs(hands) - 1;
@@ -811,19 +835,24 @@ __device__ void flatten_clipped(FrameView& f, uint32_t blocks) {
         }
       }
     }
-    if (busy && lc.state == eb::kLsDone && !lc.next_piece(b, true)) {
-      finish_curve(f, b, cur, rows);
-      busy = false;
-    }
+    if (phase == kStepping && lc.state == eb::kLsDone && !lc.next_piece(b, true)) phase = kDone;
   }
   rows = __reduce_add_sync(0xFFFFFFFFu, rows);
   if (lane == 0 && rows) atomicAdd(f.totals + 1, rows);
 }
 
-__global__ void __launch_bounds__(kCurveThreads) edge_pieces_kernel(FrameView f) {
-  const uint32_t half = gridDim.x / 2u;
-  if (blockIdx.x >= half) flatten_clipped<2>(f, half);
-  else flatten_clipped<3>(f, half);
+// `few`: the blocks of each kind that work while the pieces are no more than four per lane of them;
+// more pieces bring in the launch's other blocks. Eight blocks an SM measured 18.20 ms against three's
+// 18.70 on 512 canvases of the batch (a million clipped pieces), but 1.862 against 1.823 on 20,000
+// curve paths (20,000 pieces).
+__global__ void __launch_bounds__(kCurveThreads) edge_pieces_kernel(FrameView f, uint32_t few) {
+  const uint32_t half = gridDim.x / 2u, block = blockIdx.x % half;
+  const bool quads = blockIdx.x >= half;
+  const uint32_t n = f.work_counter[quads ? CurveWords<2>::kClip : CurveWords<3>::kClip];
+  const uint32_t blocks = min(half, max(few, n / (4u * kCurveThreads)));
+  if (block >= blocks) return;
+  if (quads) flatten_clipped<2>(f, blocks);
+  else flatten_clipped<3>(f, blocks);
 }
 
 // The pieces the safe loop flattens (those of curves inside the clip box, and the inside pieces of
@@ -1588,8 +1617,8 @@ __global__ void row_fill_kernel(FrameView f, const uint32_t* row_canvas) {
 // slot (8-lane shuffle prefix per row from the backdrop) into 128 8-bit masks and leaves the cells
 // zero for its next slots. No barrier wider than the warp. Bound: issue slots (57 % of cycles), about
 // half of them the sweeps. Measured against one block per 64 slots running the reference's DDA on
-// items sorted by its code paths: 0.58 -> 0.34 ms on 1920x1080 with 20,000 curve paths, the whole
-// pass 10.1 -> 5.2 ms on 512 canvases of the batch.
+// items sorted by its code paths, the whole pass with its slot layout: 0.82 -> 0.35 ms on 1920x1080 with
+// 20,000 curve paths, 9.7 -> 4.0 ms on 512 canvases of the batch.
 // ---------------------------------------------------------------------------------------------
 
 constexpr int kStripsPerTile = kTileH / kStripRows;
@@ -2214,7 +2243,7 @@ int launch_edges(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st) {
   if (!f.num_cmds) return 0;
   const int sms = device_sms();
   static const int max_per_sm = max_blocks_per_sm(edge_pieces_kernel, kCurveThreads);
-  const int per_sm = cfg.cubic_blocks_per_sm > 0 && cfg.cubic_blocks_per_sm < max_per_sm ? cfg.cubic_blocks_per_sm : max_per_sm;
+  const int few_per_sm = cfg.cubic_blocks_per_sm > 0 && cfg.cubic_blocks_per_sm < max_per_sm ? cfg.cubic_blocks_per_sm : max_per_sm;
   const uint32_t eb = cfg.edge_block == 64 || cfg.edge_block == 256 ? uint32_t(cfg.edge_block) : 128u;
   // four commands a warp once one each would be more than a wave of blocks
   const uint32_t per_warp = f.num_cmds > uint32_t(sms) * 8u * kClassifyWarps ? kClassifyMax : 1u;
@@ -2225,7 +2254,8 @@ int launch_edges(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st) {
   curve_split_kernel<<<2 * split_grid, 128, 0, st>>>(f);
   // as many warps as there may be pieces, up to the grids' limits
   const uint32_t pgrid = cdiv(f.piece_capacity ? f.piece_capacity : 1, kCurveThreads / 32);
-  edge_pieces_kernel<<<2 * min(pgrid, uint32_t(sms * per_sm)), kCurveThreads, 0, st>>>(f);
+  edge_pieces_kernel<<<2 * min(pgrid, uint32_t(sms * max_per_sm)), kCurveThreads, 0, st>>>(
+      f, min(pgrid, uint32_t(sms * few_per_sm)));
   edge_tree_kernel<<<2 * min(pgrid, uint32_t(sms * kTreeBlocksPerSM)), kCurveThreads, 0, st>>>(f);
   return 5;
 }
@@ -2268,11 +2298,14 @@ int launch_coverage(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st
   int k = 1;
   slot_layout_kernel<<<cdiv(f.num_cmdrows, kLayoutWarps * kLayoutSlots), 32 * kLayoutWarps, 0, st>>>(f);
   k += launch_seg_bin<true>(f, st);
-  const int per_sm = cfg.cover_blocks_per_sm > 0 ? cfg.cover_blocks_per_sm : 16;
-  // by frame: scenes of long edges (many strip rows per segment) have few work items per slot,
-  // where smaller groups keep more of them in flight per SM
-  const int slots = cfg.cover_slots ? cfg.cover_slots : (f.num_seglist > 16u * f.num_segs ? 32 : 64);
-  const int grid = sms * per_sm;
+  // far more blocks than fit at once, so that long groups even out (12, 16, 24, 32 and 64 an SM: 4.79, 4.34,
+  // 4.19, 4.16 and 4.01 ms on the batch's canvases), but none without a group
+  const int per_sm = cfg.cover_blocks_per_sm > 0 ? cfg.cover_blocks_per_sm : 64;
+  // 8 slots a warp: 16 (64 a block) leave less shared memory for other warps, 4 fewer work items than
+  // lanes. The pass at 16, 32 and 64 slots a block: 5.44, 4.37 and 4.66 ms on 512 canvases of the batch,
+  // 0.41, 0.36 and 0.41 on 20,000 curve paths.
+  const int slots = cfg.cover_slots ? cfg.cover_slots : 32;
+  const int grid = int(min(uint32_t(sms * per_sm), cdiv(f.mask_capacity, uint32_t(slots))));
   if (slots == 16) coverage_kernel<16 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f);
   else if (slots == 64) coverage_kernel<64 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f);
   else coverage_kernel<32 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f);

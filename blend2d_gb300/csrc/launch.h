@@ -11,11 +11,11 @@ namespace blgpu {
 
 // Launch shapes the autotuner chooses between (0 = the default for that field).
 struct LaunchConfig {
-  int cover_slots = 0;            // slots with segments per coverage block (16, 32 or 64; 0 = by frame)
+  int cover_slots = 0;            // slots with segments per coverage block (16, 32 or 64; 0 = 32)
   int cover_blocks_per_sm = 0;    // coverage grid: blocks per SM (0 = as many as fit)
   int fine_blocks_per_sm = 0;     // composite grid: blocks per SM (0 = as many as fit)
   int edge_block = 128;           // threads per block of the per-item edge builder (64/128/256)
-  int cubic_blocks_per_sm = 3;    // lane-scheduled curve-piece flattener: blocks per SM (0 = as many as fit)
+  int cubic_blocks_per_sm = 3;    // clipped curve pieces' flattener: blocks per SM while they are few (0 = as many as fit)
   int no_occlusion_cull = 0;      // 1: the composite starts every strip at its first command
   int max_segments = 0;           // > 0: cap of the segment array (frames needing more fail)
   int graph_frames = 0;           // 1: frames run as a captured graph over capacity-sized arrays

@@ -87,7 +87,9 @@ static bool same(const Pt* pts, uint32_t any, double w, double h, std::mt19937_6
   LaneCurve<DEG, CachedStack<DEG>> lh;
   busy = lh.begin_piece(c, pts, any);
   while (busy) {
-    if (lh.template step<true>(c)) {
+    const int r = lh.template step<true>(c);
+    if (r == LaneCurve<DEG, CachedStack<DEG>>::kStepLeaf) lh.leaf(c);
+    if (r == LaneCurve<DEG, CachedStack<DEG>>::kStepHand) {
       if (rng() % 8 == 0) { g_refused++; lh.split_node(c); }
       else {
         g_handed++;
