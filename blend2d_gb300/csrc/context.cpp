@@ -243,12 +243,15 @@ struct BLGpuContext {
     xrgb_read = xrgb_read && cs.hs.dev.fetch >= kFetchPatAlignedPad;
     if (!xrgb_read && cs.frame_gen == frame->generation) return cs.frame_index;
     if (xrgb_read && cs.frame_gen_x == frame->generation) return cs.frame_index_x;
-    DevStyle d = cs.hs.dev;
+    // written once, straight into the frame's (page-locked) array
+    const size_t at = frame->styles.size();
+    frame->styles.push_back(cs.hs.dev);
+    DevStyle& d = frame->styles[at];
     d.src_or = xrgb_read ? 0xFF000000u : 0u;
     if (d.lut_size) {
       if (d.dither) frame->lut_words = (frame->lut_words + 1u) & ~1u;   // 8-byte aligned entries
       DevLutJob job{};
-      job.style = uint32_t(frame->styles.size());
+      job.style = uint32_t(at);
       job.stop_first = uint32_t(frame->stops.size());
       job.stop_count = uint32_t(cs.hs.stops.size());
       job.lut_offset = frame->lut_words;
@@ -260,7 +263,6 @@ struct BLGpuContext {
       frame->lut_words += d.dither ? 2u * d.lut_size : d.lut_size;
     }
     if (cs.has_image) d.src_offset += frame->add_image(cs.image);
-    frame->styles.push_back(d);
     if (xrgb_read) {
       cs.frame_gen_x = frame->generation;
       cs.frame_index_x = uint32_t(frame->styles.size() - 1);

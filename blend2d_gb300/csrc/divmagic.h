@@ -19,25 +19,15 @@ struct DivMagic {
   int32_t s;       // post-shift; -1: the divisor is 1 (remainder 0)
 };
 
-// Magic number and shift for a divisor d >= 1.
+// Magic number and shift for a divisor d >= 1 (Granlund and Montgomery, "Division by Invariant Integers
+// using Multiplication", 1994, section 5): with l = ceil(log2 d), m = floor(2^(31 + l) / d) + 1 - 2^32 and
+// shift l - 1, the quotient is n plus the high product, shifted, plus 1 for a negative n. One division
+// (a search for the smallest shift took 30 steps for the 2^31 - 1 that stands for "no wrap").
 inline DivMagic div_magic(int32_t d) {
   if (d == 1) return DivMagic{0, -1};
-  const uint32_t two31 = 0x80000000u;
-  const uint32_t ad = uint32_t(d);
-  const uint32_t anc = two31 - 1u - two31 % ad;    // |nc|
-  int p = 31;
-  uint32_t q1 = two31 / anc, r1 = two31 - q1 * anc;
-  uint32_t q2 = two31 / ad, r2 = two31 - q2 * ad;
-  uint32_t delta;
-  do {
-    p++;
-    q1 *= 2u; r1 *= 2u;
-    if (r1 >= anc) { q1++; r1 -= anc; }
-    q2 *= 2u; r2 *= 2u;
-    if (r2 >= ad) { q2++; r2 -= ad; }
-    delta = ad - r2;
-  } while (q1 < delta || (q1 == delta && r1 == 0));
-  return DivMagic{int32_t(q2 + 1u), p - 32};
+  int32_t l = 1;
+  while (l < 31 && (int32_t(1) << l) < d) l++;
+  return DivMagic{int32_t(uint32_t((uint64_t(1) << (31 + l)) / uint32_t(d) + 1u)), l - 1};
 }
 
 BLGPU_HD int32_t mulhi_s32(int32_t a, int32_t b) {
