@@ -311,7 +311,8 @@ struct FrameView {
   uint32_t* cmdrow_base;       // [num_cmds + 1]: first (cmd, strip row, tile column) slot
   uint32_t* slot_mask;         // [num_cmdrows + 1] the slot's segment count (binning), then 1 + index of its masks; 0 = no segments
   uint32_t* mask_cursor;       // [non-empty slots] the mask's first work item; past its last one after the items are placed
-  uint4* mask_info;            // [non-empty slots] {x of the slot's first column, its first row, flags << 16 | alpha, slot}
+  uint4* mask_info;            // [non-empty slots] {the slot's last column | last row << 16 on the canvas (their multiples of
+                               //   32 and 4 are its first ones), command, flags << 16 | alpha, slot}
   uint2* entries;              // coverage work items {segment, mask index}, grouped by mask in mask order
   uint32_t mask_capacity;      // slots the masks array holds
   uint8_t* masks;              // [non-empty slots][kStripRows * kTileW]: analytic masks from the coverage pass
@@ -328,6 +329,7 @@ struct FrameView {
                                //   style word has bit 31 set and the colour replaces the row state
   uint32_t* row_copies;        // [num_rows] SrcCopy commands in each tile row's list
   uint32_t* strip_start;       // [num_tiles * strips per tile] first list entry the composite needs (occlusion)
+  uint32_t* strip_cmd;         // the same as a command: no command of the canvas before it shows in the strip
   uint32_t* tile_order;        // tile processing order for the persistent fine kernel
   uint32_t* tile_canvas;       // canvas index per global tile
   uint32_t* work_counter;      // [0] fine work queue, [1] items, [2] cubics, [21] quads, [23] / [25] cubic / quadratic

@@ -1292,6 +1292,7 @@ __global__ void cmd_tiles_kernel(FrameView f, uint32_t* cmdrow_counts_per_cmd, u
 // (32 a warp: 0.23 + 0.19); 27,000 segments of large shapes on 1023x767 0.18 + 0.18 -> 0.02 + 0.05
 // ms (32 a warp: 0.05 + 0.11).
 constexpr int kBinWarps = 8;
+constexpr int kStripsPerTile = kTileH / kStripRows;
 
 template<bool kScatter>
 __global__ void __launch_bounds__(32 * kBinWarps) seg_bin_kernel(FrameView f, uint32_t per_warp) {
@@ -1351,7 +1352,7 @@ __global__ void __launch_bounds__(32 * kBinWarps) seg_bin_kernel(FrameView f, ui
       }
       else {
         const uint32_t m = f.slot_mask[slot] - 1u;
-        if (m >= f.mask_capacity) continue;    // reported by the layout
+        if (m >= f.mask_capacity) continue;    // no masks: nothing below a covering command (or too many, reported)
         const uint32_t pos = atomicAdd(&f.mask_cursor[m], 1u);
         if (pos >= f.num_seglist) { atomicOr(f.error_flags, kErrSeglist); continue; }
         f.entries[pos] = make_uint2(par.w, m);
@@ -1385,26 +1386,45 @@ __device__ __forceinline__ uint32_t slot_command(const FrameView& f, uint32_t x,
   return lo;
 }
 
-// Lays out the slots after the count pass, in one pass over them: the backdrop deltas become
-// prefixes over the tile columns of every (command, strip row), and the slots with segments get
-// their mask index, the mask's record and its first work item. A warp takes the (command, strip
-// row)s that begin in its kLayoutSlots slots, whole, 32 slots at a time (a segmented scan: several
-// narrow rows or a part of a wide one), and a block takes its masks and work items from one 64-bit
-// counter with one atomic, so masks and items come in the same order and need no scan over the
-// frame. Bound: the slot arrays' bytes (20 B read per slot, backdrops written where they change).
-// In place of one warp per command for the prefix, two frame-wide scans, a flag and a compaction
-// pass over the slots: 2.4 -> 0.48 ms for the 46 M slots of 20,000 pattern quads on 4096x4096 (1.1 GB
-// read), 0.36 -> 0.02 ms for large shapes on 1023x767, and 8 to 12 launches fewer.
-constexpr int kLayoutWarps = 8;
-constexpr uint32_t kLayoutSlots = 128;
+// The commands of 32 consecutive slots from `it` on (each lane's is returned), found from command `c` at
+// or before them: those after it whose first slot is not beyond the lane's. Leaves c at the last
+// lane's command.
+__device__ __forceinline__ uint32_t slot_commands(const FrameView& f, uint32_t& c, uint32_t it, uint32_t end,
+                                                  uint32_t num_cmds, int lane) {
+  const uint32_t s = it + uint32_t(lane), last = min(it + 31u, end - 1u);
+  uint32_t mine = c;
+  for (;;) {
+    const uint32_t k = c + 1u + uint32_t(lane);
+    const uint32_t b = k < num_cmds ? f.cmdrow_base[k] : 0xFFFFFFFFu;
+    if (__shfl_sync(0xFFFFFFFFu, b, 0) > last) break;
+    uint32_t pos = 0;
+#pragma unroll
+    for (int step = 16; step; step >>= 1)
+      if (__shfl_sync(0xFFFFFFFFu, b, int(pos) + step - 1) <= s) pos += uint32_t(step);
+    const uint32_t b31 = __shfl_sync(0xFFFFFFFFu, b, 31);
+    if (pos == 31u && b31 <= s) pos = 32u;
+    if (mine == c) mine = c + pos;             // later rounds only move the lanes beyond this one's commands
+    if (b31 > last) break;
+    c += 32u;
+  }
+  c = __shfl_sync(0xFFFFFFFFu, mine, 31);
+  return mine;
+}
 
-__global__ void __launch_bounds__(32 * kLayoutWarps) slot_layout_kernel(FrameView f) {
+// After the count pass, in two passes over the slots with the occlusion pass between them (it needs
+// the prefixes, and tells which slots need no masks). First the backdrop deltas become prefixes over the
+// tile columns of every (command, strip row). A warp takes the (command, strip row)s that begin in its
+// kPrefixSlots slots, whole, 32 slots at a time (a segmented scan: several narrow rows or a part of a
+// wide one). Bound: the backdrops' bytes (16 B read per slot, written where they change).
+constexpr int kLayoutWarps = 8;
+constexpr uint32_t kLayoutSlots = 128, kPrefixSlots = 256;
+
+__global__ void __launch_bounds__(32 * kLayoutWarps) backdrop_prefix_kernel(FrameView f) {
   if (frame_skipped(f)) return;
-  __shared__ uint32_t masks_of[kLayoutWarps], items_of[kLayoutWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t n = frame_slots(f), num_cmds = f.counts[kCntCmds];
-  const uint64_t x0 = (uint64_t(blockIdx.x) * kLayoutWarps + uint32_t(w)) * kLayoutSlots;
-  if (x0 - uint64_t(w) * kLayoutSlots >= n) return;   // whole blocks leave together
+  const uint64_t x0 = (uint64_t(blockIdx.x) * kLayoutWarps + uint32_t(w)) * kPrefixSlots;
+  if (x0 >= n) return;
   // the first (command, strip row) beginning at or after x; `c` its command if it is inside one
   uint32_t c = 0;
   auto row_start = [&](uint64_t x) -> uint32_t {
@@ -1415,16 +1435,80 @@ __global__ void __launch_bounds__(32 * kLayoutWarps) slot_layout_kernel(FrameVie
     const uint32_t past = (uint32_t(x) - f.cmdrow_base[c]) % ntx;
     return past ? min(n, uint32_t(x) + ntx - past) : uint32_t(x);
   };
-  const uint32_t end = row_start(x0 + kLayoutSlots);
+  const uint32_t end = row_start(x0 + kPrefixSlots);
   const uint32_t begin = row_start(x0);        // leaves c at x0's command: at or before begin's
-  uint32_t my_masks = 0, my_items = 0;
-  for (uint32_t s = begin + uint32_t(lane); s < end; s += 32) {
-    const uint32_t k = f.slot_mask[s];
-    my_masks += k ? 1u : 0u;
-    my_items += k;
+  uint4 carry = make_uint4(0u, 0u, 0u, 0u);    // the last slot's prefix of the slots before
+  for (uint32_t it = begin; it < end; it += 32) {
+    const uint32_t s = it + uint32_t(lane);
+    const bool on = s < end;
+    const uint4 v = on ? *reinterpret_cast<const uint4*>(f.backdrop + size_t(s) * kStripRows) : make_uint4(0u, 0u, 0u, 0u);
+    if (!__any_sync(0xFFFFFFFFu, (v.x | v.y | v.z | v.w | carry.x | carry.y | carry.z | carry.w) != 0u)) continue;
+    const uint32_t mine = slot_commands(f, c, it, end, num_cmds, lane);
+    uint32_t col = 0;
+    if (on) {
+      const uint32_t ctx = f.cmd_tile_x[mine];
+      col = (s - f.cmdrow_base[mine]) % ((ctx >> 16) - (ctx & 0xFFFFu) + 1u);
+    }
+    uint4 p = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t px = __shfl_up_sync(0xFFFFFFFFu, p.x, o), py = __shfl_up_sync(0xFFFFFFFFu, p.y, o);
+      const uint32_t pz = __shfl_up_sync(0xFFFFFFFFu, p.z, o), pw = __shfl_up_sync(0xFFFFFFFFu, p.w, o);
+      if (lane >= o && col >= uint32_t(o)) { p.x += px; p.y += py; p.z += pz; p.w += pw; }
+    }
+    if (col > uint32_t(lane)) { p.x += carry.x; p.y += carry.y; p.z += carry.z; p.w += carry.w; }
+    if (on && (p.x != v.x || p.y != v.y || p.z != v.z || p.w != v.w))
+      *reinterpret_cast<uint4*>(f.backdrop + size_t(s) * kStripRows) = p;
+    carry = make_uint4(__shfl_sync(0xFFFFFFFFu, p.x, 31), __shfl_sync(0xFFFFFFFFu, p.y, 31),
+                       __shfl_sync(0xFFFFFFFFu, p.z, 31), __shfl_sync(0xFFFFFFFFu, p.w, 31));
   }
-  my_masks = __reduce_add_sync(0xFFFFFFFFu, my_masks);
-  my_items = __reduce_add_sync(0xFFFFFFFFu, my_items);
+}
+
+// Then the slots with segments that no later command covers (cull_kernel) get their mask index, the
+// mask's record and its first work item, in place of the segment count; the others get none. A warp
+// takes 128 slots and a block its masks and work items from one 64-bit counter with one atomic, so masks
+// and items come in the same order and need no scan over the frame. Bound: the counts' bytes and the
+// command look-up. Both passes in place of one warp per command for the prefix, two frame-wide scans and
+// a flag and a compaction pass over the slots: 2.4 -> 0.51 ms for the 46 M slots of 20,000
+// pattern quads on 4096x4096, 0.36 -> 0.03 ms for large shapes on 1023x767, and 8 to 12 launches fewer.
+__global__ void __launch_bounds__(32 * kLayoutWarps) slot_compact_kernel(FrameView f) {
+  if (frame_skipped(f)) return;
+  constexpr int kSteps = int(kLayoutSlots) / 32;
+  __shared__ uint32_t masks_of[kLayoutWarps], items_of[kLayoutWarps];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t n = frame_slots(f), num_cmds = f.counts[kCntCmds];
+  const uint64_t x0 = (uint64_t(blockIdx.x) * kLayoutWarps + uint32_t(w)) * kLayoutSlots;
+  if (x0 - uint64_t(w) * kLayoutSlots >= n) return;   // whole blocks leave together
+  uint32_t count[kSteps], mine[kSteps], my_masks = 0, my_items = 0;
+#pragma unroll
+  for (int k = 0; k < kSteps; k++) {
+    const uint64_t s = x0 + uint64_t(32 * k + lane);
+    count[k] = s < n ? f.slot_mask[s] : 0u;
+    my_items |= count[k];
+  }
+  if (!__syncthreads_or(int(my_items != 0u))) return;         // no slot of the block has segments
+  uint32_t c = __any_sync(0xFFFFFFFFu, my_items != 0u) ? slot_command(f, uint32_t(x0), num_cmds, lane) : 0u;
+  my_items = 0;
+#pragma unroll
+  for (int k = 0; k < kSteps; k++) {
+    mine[k] = 0;
+    if (!__any_sync(0xFFFFFFFFu, count[k] != 0u)) continue;
+    const uint32_t it = uint32_t(x0) + 32u * uint32_t(k);
+    mine[k] = slot_commands(f, c, it, n, num_cmds, lane);
+    if (count[k]) {
+      const uint32_t ctx = f.cmd_tile_x[mine[k]], tx0 = ctx & 0xFFFFu, ntx = (ctx >> 16) - tx0 + 1u;
+      const uint32_t local = it + uint32_t(lane) - f.cmdrow_base[mine[k]], row = local / ntx;
+      const uint32_t sr = ((f.cmd_yr[mine[k]] & 0xFFFFu) >> kStripShift) + row;
+      const DevCanvas& cv = f.canvases[f.cmds[mine[k]].canvas];
+      const uint32_t tile = cv.tile_base + (sr >> (kTileShift - kStripShift)) * uint32_t(cv.tiles_x) + tx0 + local - row * ntx;
+      if (mine[k] < f.strip_cmd[tile * kStripsPerTile + (sr & (kStripsPerTile - 1u))]) {
+        f.slot_mask[it + uint32_t(lane)] = 0u;
+        count[k] = 0u;
+      }
+    }
+    my_masks += uint32_t(__popc(__ballot_sync(0xFFFFFFFFu, count[k] != 0u)));
+    my_items += __reduce_add_sync(0xFFFFFFFFu, count[k]);
+  }
   if (lane == 0) { masks_of[w] = my_masks; items_of[w] = my_items; }
   __syncthreads();
   if (w == 0) {
@@ -1444,74 +1528,36 @@ __global__ void __launch_bounds__(32 * kLayoutWarps) slot_layout_kernel(FrameVie
   }
   __syncthreads();
   uint32_t mask_at = masks_of[w], item_at = items_of[w];
-
-  uint4 carry = make_uint4(0u, 0u, 0u, 0u);    // the last slot's prefix of the slots before
-  for (uint32_t it = begin; it < end; it += 32) {
-    const uint32_t s = it + uint32_t(lane);
-    const bool on = s < end;
-    // the slots' commands: those after `c` whose first slot is not beyond the slot
-    uint32_t mine = c;
-    for (;;) {
-      const uint32_t k = c + 1u + uint32_t(lane);
-      const uint32_t b = k < num_cmds ? f.cmdrow_base[k] : 0xFFFFFFFFu;
-      const uint32_t b0 = __shfl_sync(0xFFFFFFFFu, b, 0), b31 = __shfl_sync(0xFFFFFFFFu, b, 31);
-      if (b0 > min(it + 31u, end - 1u)) { break; }
-      uint32_t pos = 0;
 #pragma unroll
-      for (int step = 16; step; step >>= 1)
-        if (__shfl_sync(0xFFFFFFFFu, b, int(pos) + step - 1) <= s) pos += uint32_t(step);
-      if (pos == 31u && b31 <= s) pos = 32u;
-      if (mine == c) mine = c + pos;           // later rounds only move the lanes beyond this one's commands
-      if (b31 > min(it + 31u, end - 1u)) break;
-      c += 32u;
-    }
-    c = __shfl_sync(0xFFFFFFFFu, mine, 31);
-    uint32_t count = 0, col = 0, tx = 0, sr = 0;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (on) {
-      const uint32_t ctx = f.cmd_tile_x[mine];
-      const uint32_t ntx = (ctx >> 16) - (ctx & 0xFFFFu) + 1u, local = s - f.cmdrow_base[mine];
-      count = f.slot_mask[s];
-      v = *reinterpret_cast<const uint4*>(f.backdrop + size_t(s) * kStripRows);
-      sr = local / ntx;
-      col = local - sr * ntx;
-      tx = (ctx & 0xFFFFu) + col;
-    }
-    if (__any_sync(0xFFFFFFFFu, (v.x | v.y | v.z | v.w | carry.x | carry.y | carry.z | carry.w) != 0u)) {
-      uint4 p = v;
+  for (int k = 0; k < kSteps; k++) {
+    const uint32_t some = __ballot_sync(0xFFFFFFFFu, count[k] != 0u);
+    if (!some) continue;
+    uint32_t incl = count[k];
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t px = __shfl_up_sync(0xFFFFFFFFu, p.x, o), py = __shfl_up_sync(0xFFFFFFFFu, p.y, o);
-        const uint32_t pz = __shfl_up_sync(0xFFFFFFFFu, p.z, o), pw = __shfl_up_sync(0xFFFFFFFFu, p.w, o);
-        if (lane >= o && col >= uint32_t(o)) { p.x += px; p.y += py; p.z += pz; p.w += pw; }
-      }
-      if (col > uint32_t(lane)) { p.x += carry.x; p.y += carry.y; p.z += carry.z; p.w += carry.w; }
-      if (on && (p.x != v.x || p.y != v.y || p.z != v.z || p.w != v.w))
-        *reinterpret_cast<uint4*>(f.backdrop + size_t(s) * kStripRows) = p;
-      carry = make_uint4(__shfl_sync(0xFFFFFFFFu, p.x, 31), __shfl_sync(0xFFFFFFFFu, p.y, 31),
-                         __shfl_sync(0xFFFFFFFFu, p.z, 31), __shfl_sync(0xFFFFFFFFu, p.w, 31));
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += t;
     }
-    const uint32_t some = __ballot_sync(0xFFFFFFFFu, count != 0u);
-    if (some) {
-      uint32_t incl = count;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += t;
+    if (count[k]) {
+      const uint32_t s = uint32_t(x0) + 32u * uint32_t(k) + uint32_t(lane), m = mine[k];
+      const uint32_t idx = mask_at + uint32_t(__popc(some & ((1u << lane) - 1u)));
+      f.slot_mask[s] = idx + 1u;
+      if (idx < f.mask_capacity) {
+        const uint32_t ctx = f.cmd_tile_x[m], tx0 = ctx & 0xFFFFu, ntx = (ctx >> 16) - tx0 + 1u;
+        const uint32_t local = s - f.cmdrow_base[m], row = local / ntx;
+        const uint32_t x = (tx0 + local - row * ntx) << kTileShift;
+        const uint32_t y = (((f.cmd_yr[m] & 0xFFFFu) >> kStripShift) + row) << kStripShift;
+        const DevCmd& cmd = f.cmds[m];
+        const DevCanvas& cv = f.canvases[cmd.canvas];
+        f.mask_cursor[idx] = item_at + incl - count[k];
+        // what the coverage pass needs of the slot
+        f.mask_info[idx] = make_uint4((x + min(uint32_t(cv.w) - x, uint32_t(kTileW)) - 1u) |
+                                          ((y + min(uint32_t(cv.h) - y, uint32_t(kStripRows)) - 1u) << 16),
+                                      m, (cmd.flags << 16) | cmd.alpha, s);
       }
-      if (count) {
-        const uint32_t idx = mask_at + uint32_t(__popc(some & ((1u << lane) - 1u)));
-        f.slot_mask[s] = idx + 1u;
-        if (idx < f.mask_capacity) {
-          f.mask_cursor[idx] = item_at + incl - count;
-          // what the coverage pass needs of the slot
-          f.mask_info[idx] = make_uint4(tx << kTileShift, (((f.cmd_yr[mine] & 0xFFFFu) >> kStripShift) + sr) << kStripShift,
-                                        (f.cmds[mine].flags << 16) | f.cmds[mine].alpha, s);
-        }
-      }
-      mask_at += uint32_t(__popc(some));
-      item_at += __shfl_sync(0xFFFFFFFFu, incl, 31);
     }
+    mask_at += uint32_t(__popc(some));
+    item_at += __shfl_sync(0xFFFFFFFFu, incl, 31);
   }
 }
 
@@ -1621,9 +1667,9 @@ __global__ void row_fill_kernel(FrameView f, const uint32_t* row_canvas) {
 // 20,000 curve paths, 9.7 -> 4.0 ms on 512 canvases of the batch.
 // ---------------------------------------------------------------------------------------------
 
-constexpr int kStripsPerTile = kTileH / kStripRows;
 constexpr int kFineWarps = kFineThreads / 32;
 constexpr int kFineBlocksPerSM = 4;
+constexpr uint32_t kCullBlocksPerSM = 8;
 constexpr int kSlotPixels = kStripRows * kTileW;
 constexpr int kCoverWarps = 4;
 
@@ -1631,8 +1677,8 @@ template<int kSlots>
 __global__ void __launch_bounds__(32 * kCoverWarps) coverage_kernel(FrameView f) {
   __shared__ __align__(16) uint32_t cells_all[kCoverWarps][kSlots][kSlotPixels];
   __shared__ __align__(16) uint32_t bd_all[kCoverWarps][kSlots][kStripRows];
-  __shared__ int2 org_all[kCoverWarps][kSlots];       // x of the slot's first column, its first row
-  __shared__ uint32_t meta_all[kCoverWarps][kSlots];  // command flags << 16 | alpha
+  __shared__ uint32_t org_all[kCoverWarps][kSlots];   // the slot's last column and row on the canvas
+  __shared__ uint2 meta_all[kCoverWarps][kSlots];     // command flags << 16 | alpha, command
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (frame_skipped(f)) return;
   const uint32_t all_masks = f.work_counter[kMaskAlloc + 1], num_masks = min(all_masks, f.mask_capacity);
@@ -1642,8 +1688,8 @@ __global__ void __launch_bounds__(32 * kCoverWarps) coverage_kernel(FrameView f)
   if (first >= groups) return;
   uint32_t(*cells)[kSlotPixels] = cells_all[warp];
   uint32_t(*bd)[kStripRows] = bd_all[warp];
-  int2* org = org_all[warp];
-  uint32_t* meta = meta_all[warp];
+  uint32_t* org = org_all[warp];
+  uint2* meta = meta_all[warp];
 #pragma unroll
   for (int j = 0; j < kSlots; j++) *reinterpret_cast<uint4*>(&cells[j][lane * 4]) = make_uint4(0u, 0u, 0u, 0u);
 
@@ -1652,8 +1698,8 @@ __global__ void __launch_bounds__(32 * kCoverWarps) coverage_kernel(FrameView f)
     const int nk = int(min(uint32_t(kSlots), num_masks - m0));
     if (lane < nk) {
       const uint4 info = f.mask_info[m0 + uint32_t(lane)];
-      org[lane] = make_int2(int(info.x), int(info.y));
-      meta[lane] = info.z;
+      org[lane] = info.x;
+      meta[lane] = make_uint2(info.z, info.y);
       *reinterpret_cast<uint4*>(bd[lane]) = *reinterpret_cast<const uint4*>(f.backdrop + size_t(info.w) * kStripRows);
     }
     // a mask's cursor now stands at the end of its items, where the next mask's begin
@@ -1662,14 +1708,17 @@ __global__ void __launch_bounds__(32 * kCoverWarps) coverage_kernel(FrameView f)
     for (uint32_t e = e0 + uint32_t(lane); e < e1; e += 32) {
       const uint2 it = f.entries[e];
       const int j = int(it.y - m0);
-      ras::WindowSink sink{cells[j], bd[j], org[j].x};
-      ras::segment_to_window(f.segs[it.x], f.seg_meta[it.x] & 1u, org[j].y, kStripRows, sink);
+      const uint32_t o = org[j];
+      ras::WindowSink sink{cells[j], bd[j], int(o & 0xFFFFu & ~uint32_t(kTileW - 1))};
+      ras::segment_to_window(f.segs[it.x], f.seg_meta[it.x] & 1u, int((o >> 16) & ~uint32_t(kStripRows - 1)), kStripRows, sink);
     }
     __syncwarp();
     // sweep: lane covers row lane / 8, columns (lane % 8) * 4 .. + 3 of the slot
     const int prow = lane >> 3;
+    uint32_t covers = 0;                       // bit j: slot j hides everything before its command
     for (int j = 0; j < nk; j++) {
-      const uint32_t flags = meta[j] >> 16, alpha = meta[j] & 0xFFFFu;
+      const uint2 mt = meta[j];
+      const uint32_t flags = mt.x >> 16, alpha = mt.x & 0xFFFFu;
       uint4* cell4 = reinterpret_cast<uint4*>(&cells[j][lane * 4]);
       const uint4 cv4 = *cell4;
       *cell4 = make_uint4(0u, 0u, 0u, 0u);
@@ -1688,6 +1737,21 @@ __global__ void __launch_bounds__(32 * kCoverWarps) coverage_kernel(FrameView f)
       cov += cv4.z; m |= px::calc_mask(cov, rule, alpha) << 16;
       cov += cv4.w; m |= px::calc_mask(cov, rule, alpha) << 24;
       reinterpret_cast<uint32_t*>(f.masks + size_t(m0 + uint32_t(j)) * kSlotPixels)[lane] = m;
+      if ((flags & 1u) && alpha == 255u) {
+        // an opaque SrcCopy command that covers every pixel of the slot on the canvas: none before it
+        // shows there (what the occlusion pass could not see without the masks)
+        const uint32_t o = org[j];
+        const int cols = int(o & uint32_t(kTileW - 1)) + 1 - (lane & 7) * 4;          // of the lane's four
+        const uint32_t on = prow > int((o >> 16) & uint32_t(kStripRows - 1)) || cols <= 0 ? 0u
+                          : cols >= 4 ? 0xFFFFFFFFu : (1u << (8 * cols)) - 1u;
+        if (__all_sync(0xFFFFFFFFu, (m | ~on) == 0xFFFFFFFFu)) covers |= 1u << j;
+      }
+    }
+    if (lane < nk && ((covers >> lane) & 1u)) {      // a lane per covering slot: one latency for all of them
+      const uint32_t o = org[lane], cmd = meta[lane].y, sr = (o >> 16) >> kStripShift;
+      const DevCanvas& cv = f.canvases[f.cmds[cmd].canvas];
+      const uint32_t tile = cv.tile_base + (sr >> (kTileShift - kStripShift)) * uint32_t(cv.tiles_x) + ((o & 0xFFFFu) >> kTileShift);
+      atomicMax(&f.strip_cmd[tile * kStripsPerTile + (sr & (kStripsPerTile - 1u))], cmd);
     }
     __syncwarp();
   }
@@ -1759,79 +1823,104 @@ __device__ __forceinline__ uint32_t pixels_on_canvas(int xp, int y, const DevCan
 }
 
 // Occlusion, per strip: a SrcCopy command whose mask is 255 on every pixel of the strip writes its
-// source there whatever is below (CompOp_SrcCopy with m = 255 gives the source exactly), so the
-// composite pass can start at the last such command of the strip's list. Looked for from the end
-// of the list, in rows with SrcCopy commands besides a first clear; 0 elsewhere.
+// source there whatever is below (CompOp_SrcCopy with m = 255 gives the source exactly), so nothing
+// before the last such command of the strip's list shows: slot_compact_kernel gives the slots before it no
+// masks and the composite starts at it. Such a command is found before any mask is rasterized: a box
+// that covers the strip, or a path in whose slot no segment lies and whose carried-in coverage is full.
+// (A path with segments in the slot that cover it all the same shows in its masks: coverage_kernel
+// raises strip_cmd for the composite.)
+//
+// One warp per tile looks through the tile's list from the end, 32 entries at a time, for opaque SrcCopy
+// commands over all its columns, and tests four of them on all eight strips at once, until every strip
+// has one; in rows with SrcCopy commands besides a first clear. Bound: the latency of the list reads and
+// slot look-ups. One warp per strip, one candidate at a time, took 1.19 ms on 512 canvases of the batch
+// (0.43 this way), and after the coverage pass, so that every slot had masks: coverage kernel 3.6 -> 2.4
+// ms there, and 1.0 -> 0.06 ms for 20,000 pattern quads on 4096x4096, where the pass itself went from 0.08
+// to 0.26.
 __global__ void __launch_bounds__(kFineThreads) cull_kernel(FrameView f) {
   const int lane = threadIdx.x & 31;
-  const int prow = lane >> 3;
-  const int pcol = (lane & 7) * 4;
   if (frame_skipped(f)) return;
-  const uint32_t num_units = f.counts[kCntTiles] * kStripsPerTile;
+  const uint32_t num_tiles = f.counts[kCntTiles];
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); unit < num_units; unit += warps) {
-    const uint32_t tile = f.tile_order[unit / kStripsPerTile];
-    const int strip = int(unit % kStripsPerTile);
+  const uint32_t row_log2 = kTileShift - f.list_shift;           // list rows per tile
+  const int strips = kStripsPerTile >> row_log2;                  // strips per list row
+  for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < num_tiles; tile += warps) {
     const DevCanvas cv = f.canvases[f.tile_canvas[tile]];
     const uint32_t local = tile - cv.tile_base;
     const int tx = int(local % uint32_t(cv.tiles_x)), ty = int(local / uint32_t(cv.tiles_x));
-    const int x_base = tx * kTileW;
-    const int row0 = ty * kTileH + strip * kStripRows;
-    const uint32_t row_id = (cv.row_base << (kTileShift - f.list_shift)) + (uint32_t(row0) >> f.list_shift);
-    if (row0 >= cv.h || f.row_copies[row_id] < 2) {
-      if (lane == 0) f.strip_start[unit] = 0;
-      continue;
-    }
-    const uint32_t strip_row = uint32_t(row0) >> kStripShift;
-    const int row1 = min(row0 + kStripRows, cv.h) - 1;
-    const int y = row0 + prow, xp = x_base + pcol;
-    const uint32_t on_canvas = pixels_on_canvas(xp, y, cv);
-    const uint32_t list_first = f.row_offsets[row_id];
-    const uint32_t list_count = f.row_counts[row_id];
-    const uint32_t strip_y = uint32_t(row0) | (uint32_t(row1) << 16);
-    const uint32_t strip_x = uint32_t(x_base) | (uint32_t(min(x_base + kTileW, cv.w) - 1) << 16);
-    uint32_t start = 0;
-    for (int cb = int((list_count - 1u) & ~31u); cb >= 0; cb -= 32) {
-      uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
-      bool cand = false;
-      if (uint32_t(cb + lane) < list_count) {
-        // the box first; the records only for commands that cover the whole strip
-        const uint2 bb = f.row_box[list_first + uint32_t(cb + lane)];
-        cand = (bb.x & 0xFFFFu) <= (strip_x & 0xFFFFu) && (bb.x >> 16) >= (strip_x >> 16) &&
-               (bb.y & 0xFFFFu) <= (strip_y & 0xFFFFu) && (bb.y >> 16) >= (strip_y >> 16);
-        if (cand) {
-          const uint4* rec = f.row_recs + 2u * (list_first + uint32_t(cb + lane));
-          ra = rec[0];
-          rb = rec[1];
-          cand = ((ra.w >> 2) & 1u) && ((ra.w >> 4) & 0xFFu) == 255u;
+    const uint32_t x0 = uint32_t(tx) << kTileShift, x1 = uint32_t(min(int(x0) + kTileW, cv.w) - 1);
+    const int s = lane & 7, q = lane >> 3;                        // strip of the list row, candidate of four
+    for (uint32_t lr = 0; lr < (1u << row_log2); lr++) {
+      const uint32_t row_id = ((cv.row_base + uint32_t(ty)) << row_log2) + lr;
+      const int top = (ty << kTileShift) + int(lr << f.list_shift);     // the list row's first pixel row
+      const int sy0 = top + s * kStripRows, sy1 = min(sy0 + kStripRows, cv.h) - 1;
+      const bool real = s < strips && sy0 < cv.h;
+      uint32_t open = __ballot_sync(0xFFFFFFFFu, real) & 0xFFu;   // strips still without a covering command
+      uint32_t start = 0, start_cmd = 0;                          // of strip `lane`, for lanes below `strips`
+      if (top >= cv.h || f.row_copies[row_id] < 2) open = 0;
+      const uint32_t list_first = open ? f.row_offsets[row_id] : 0u, list_count = open ? f.row_counts[row_id] : 0u;
+      for (int cb = int((list_count - 1u) & ~31u); open && cb >= 0; cb -= 32) {
+        uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
+        bool cand = false;
+        if (uint32_t(cb + lane) < list_count) {
+          // the box first; the records only for commands over all columns
+          const uint2 bb = f.row_box[list_first + uint32_t(cb + lane)];
+          cand = (bb.x & 0xFFFFu) <= x0 && (bb.x >> 16) >= x1;
+          if (cand) {
+            const uint4* rec = f.row_recs + 2u * (list_first + uint32_t(cb + lane));
+            ra = rec[0];
+            rb = rec[1];
+            cand = ((ra.w >> 2) & 1u) && ((ra.w >> 4) & 0xFFu) == 255u && (ra.w & 3u) != kFillMaskA;
+          }
+        }
+        uint32_t todo = __ballot_sync(0xFFFFFFFFu, cand);
+        while (todo && open) {
+          // the next four candidates, the last one of the list first
+          int at = -1;
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const int bit = 31 - __clz(todo);                     // -1 when there is none left
+            if (q == j) at = bit;
+            if (bit >= 0) todo &= ~(1u << bit);
+          }
+          const int from = at < 0 ? 0 : at;
+          const uint32_t ci = __shfl_sync(0xFFFFFFFFu, ra.x, from), yr = __shfl_sync(0xFFFFFFFFu, ra.z, from);
+          const uint32_t meta = __shfl_sync(0xFFFFFFFFu, ra.w, from);
+          const uint32_t slot0 = __shfl_sync(0xFFFFFFFFu, rb.x, from), tcols = __shfl_sync(0xFFFFFFFFu, rb.y, from);
+          bool full = at >= 0 && ((open >> s) & 1u) && int(yr & 0xFFFFu) <= sy0 && int(yr >> 16) >= sy1;
+          if (full && (meta & 3u) == kFillAnalytic) {
+            uint32_t nseg = 0;
+            const uint32_t slot = strip_slot(f, slot0, tcols, yr, uint32_t(sy0) >> kStripShift, tx, nseg);
+            full = nseg == 0u;
+            if (full) {
+              const uint4 bd = *reinterpret_cast<const uint4*>(f.backdrop + size_t(slot) * kStripRows);
+              const uint32_t rows[4] = {bd.x, bd.y, bd.z, bd.w};
+#pragma unroll
+              for (int r = 0; r < 4; r++)
+                full &= sy0 + r > sy1 || uniform_mask(rows[r], (meta >> 2) & 3u, 255u) == 255u;
+            }
+          }
+          else if (full && (meta & 3u) == kFillBoxU) {
+            // fractional borders thin only the box's first and last columns and rows: the strip's corners tell
+            const int32_t* box = f.cmds[ci].box;
+            full = px::box_u_mask(box, 255u, int(x0), sy0) == 255u && px::box_u_mask(box, 255u, int(x1), sy0) == 255u &&
+                   px::box_u_mask(box, 255u, int(x0), sy1) == 255u && px::box_u_mask(box, 255u, int(x1), sy1) == 255u;
+          }
+          const uint32_t found = __ballot_sync(0xFFFFFFFFu, full);
+          const uint32_t mine = (found >> s) & 0x01010101u;       // the candidates that cover strip s
+          const int first = mine ? (__ffs(mine) - 1) >> 3 : 0;
+          const int hit_at = __shfl_sync(0xFFFFFFFFu, at, first * 8);
+          const uint32_t hit_cmd = __shfl_sync(0xFFFFFFFFu, ci, first * 8);
+          if (mine && ((open >> s) & 1u)) { start = uint32_t(cb + hit_at); start_cmd = hit_cmd; }
+          open &= ~((found | (found >> 8) | (found >> 16) | (found >> 24)) & 0xFFu);
         }
       }
-      uint32_t todo = __ballot_sync(0xFFFFFFFFu, cand);
-      bool found = false;
-      while (todo) {
-        const int bit = 31 - __clz(todo);
-        todo &= ~(1u << bit);
-        const uint32_t ci = __shfl_sync(0xFFFFFFFFu, ra.x, bit);
-        const uint32_t rmeta = __shfl_sync(0xFFFFFFFFu, ra.w, bit);
-        const uint32_t ckind = rmeta & 3u, calpha = (rmeta >> 4) & 0xFFu;
-        const uint32_t cxr = __shfl_sync(0xFFFFFFFFu, ra.y, bit), cyr = __shfl_sync(0xFFFFFFFFu, ra.z, bit);
-        uint32_t mw = 0;
-        if (ckind == kFillAnalytic) {
-          uint32_t cnseg = 0;
-          const uint32_t slot = strip_slot(f, __shfl_sync(0xFFFFFFFFu, rb.x, bit), __shfl_sync(0xFFFFFFFFu, rb.y, bit),
-                                           cyr, strip_row, tx, cnseg);
-          mw = cnseg ? reinterpret_cast<const uint32_t*>(f.masks + size_t(cnseg - 1u) * kSlotPixels)[lane]
-                     : uniform_mask(f.backdrop[size_t(slot) * kStripRows + prow], (rmeta >> 2) & 3u, calpha) * 0x01010101u;
-        }
-        else {
-          mw = box_masks(f, ckind, ci, calpha, cxr, cyr, xp, y);
-        }
-        const bool full = (mw | ~on_canvas) == 0xFFFFFFFFu;
-        if (__all_sync(0xFFFFFFFFu, full)) { start = uint32_t(cb + bit); found = true; break; }
+      if (lane < strips) {
+        const uint32_t unit = tile * kStripsPerTile + lr * uint32_t(strips) + uint32_t(lane);
+        f.strip_start[unit] = start;
+        f.strip_cmd[unit] = start_cmd;
       }
-      if (found) break;
     }
-    if (lane == 0) f.strip_start[unit] = start;
   }
 }
 
@@ -1960,7 +2049,8 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
     const uint32_t strip_y = uint32_t(row0) | (uint32_t(row1) << 16);
     const uint32_t strip_x = uint32_t(x_base) | (uint32_t(min(x_base + kTileW, cv.w) - 1) << 16);
 
-    const uint32_t start = f.strip_start[unit];      // cull_kernel
+    const uint32_t start = f.strip_start[tile * kStripsPerTile + uint32_t(strip)];      // cull_kernel
+    const uint32_t cover = f.strip_cmd[tile * kStripsPerTile + uint32_t(strip)];        // ... and coverage_kernel
     uint32_t pend_mw = 0, pend[4] = {0u, 0u, 0u, 0u};   // the command to composite next
     bool pend_copy = false;
 
@@ -1979,7 +2069,8 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
           const uint4* rec = f.row_recs + 2u * (list_first + base + lane);
           ra = rec[0];
           rb = rec[1];
-          if ((ra.w & 3u) == kFillAnalytic) {
+          hit = ra.x >= cover;
+          if (hit && (ra.w & 3u) == kFillAnalytic) {
             uint32_t nseg = 0;
             const uint32_t slot = strip_slot(f, rb.x, rb.y, ra.z, strip_row, tx, nseg);
             stored = nseg != 0u;
@@ -2290,14 +2381,27 @@ int fine_grid_size(int blocks_per_sm) {
   return sms * (blocks_per_sm > 0 && blocks_per_sm < max_per_sm ? blocks_per_sm : max_per_sm);
 }
 
-// Coverage pass: lay out the slots (backdrop prefixes, masks, work items), place the work items,
-// rasterize and sweep. Called after the binning count pass.
+// Coverage pass: backdrop prefixes, occlusion, masks and work items of the slots that show, rasterize and
+// sweep. Called after the binning count pass and the command lists.
 int launch_coverage(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st) {
-  if (!f.num_cmdrows) return 0;
   const int sms = device_sms();
-  int k = 1;
-  slot_layout_kernel<<<cdiv(f.num_cmdrows, kLayoutWarps * kLayoutSlots), 32 * kLayoutWarps, 0, st>>>(f);
-  k += launch_seg_bin<true>(f, st);
+  int k = 0;
+  const uint32_t layout_grid = cdiv(f.num_cmdrows, kLayoutWarps * kLayoutSlots);
+  if (f.num_cmdrows) {
+    backdrop_prefix_kernel<<<cdiv(f.num_cmdrows, kLayoutWarps * kPrefixSlots), 32 * kLayoutWarps, 0, st>>>(f);
+    k++;
+  }
+  if (cfg.no_occlusion_cull) {
+    cudaMemsetAsync(f.strip_start, 0, sizeof(uint32_t) * size_t(f.num_tiles) * kStripsPerTile, st);
+    cudaMemsetAsync(f.strip_cmd, 0, sizeof(uint32_t) * size_t(f.num_tiles) * kStripsPerTile, st);
+  }
+  else if (f.num_tiles) {
+    cull_kernel<<<min(uint32_t(sms) * kCullBlocksPerSM, cdiv(f.num_tiles, kFineWarps)), kFineThreads, 0, st>>>(f);
+    k++;
+  }
+  if (!f.num_cmdrows) return k;
+  slot_compact_kernel<<<layout_grid, 32 * kLayoutWarps, 0, st>>>(f);
+  k += 1 + launch_seg_bin<true>(f, st);
   // far more blocks than fit at once, so that long groups even out (12, 16, 24, 32 and 64 an SM: 4.79, 4.34,
   // 4.19, 4.16 and 4.01 ms on the batch's canvases), but none without a group
   const int per_sm = cfg.cover_blocks_per_sm > 0 ? cfg.cover_blocks_per_sm : 64;
@@ -2326,14 +2430,8 @@ int launch_fine(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st) {
   int grid = fine_grid_size(cfg.fine_blocks_per_sm);
   uint32_t max_blocks = (f.num_tiles * kStripsPerTile + kFineWarps - 1) / kFineWarps;
   if (uint32_t(grid) > max_blocks) grid = int(max_blocks);
-  if (cfg.no_occlusion_cull) {
-    cudaMemsetAsync(f.strip_start, 0, sizeof(uint32_t) * size_t(f.num_tiles) * kStripsPerTile, st);
-  }
-  else {
-    cull_kernel<<<grid, kFineThreads, 0, st>>>(f);
-  }
   fine_kernel<<<grid, kFineThreads, 0, st>>>(f);
-  return cfg.no_occlusion_cull ? 1 : 2;
+  return 1;
 }
 
 }  // namespace blgpu
