@@ -721,16 +721,23 @@ int Runtime::enqueue_count_half(cudaStream_t st) {
 int Runtime::enqueue_render_half(cudaStream_t st, bool timed) {
   const FrameView& f = view;
   int k = launch_frame_gate(f, st);
+  // The gradients' row states (a conic's is a serial FP64 chain of up to a band of rows, or of the whole
+  // box) are read by the composite only: on the side stream, beside the binning and coverage passes.
+  if (f.num_row_states) {
+    cudaEventRecord(fork_ev, st);
+    cudaStreamWaitEvent(side, fork_ev, 0);
+    k += launch_row_states(f, side);
+    cudaEventRecord(join_ev, side);
+  }
   cudaMemsetAsync(f.slot_mask, 0, sizeof(uint32_t) * (f.num_cmdrows + 1), st);
   cudaMemsetAsync(f.backdrop, 0, sizeof(uint32_t) * kStripRows * (size_t(f.num_cmdrows) + 1), st);
   k += launch_bin_count(f, st);
   k += launch_rows_and_tiles(f, row_canvas, st);
-  k += launch_row_states(f, st);
   // the fine stage: coverage (masks of analytic fills) + composite, timed together
   if (timed) cudaEventRecord(ev[1], st);
   k += launch_coverage(f, cfg, st);
   if (timed) cudaEventRecord(ev[4], st);
-  if (f.num_lut_jobs) cudaStreamWaitEvent(st, join_ev, 0);     // the composite reads the LUTs
+  if (f.num_lut_jobs || f.num_row_states) cudaStreamWaitEvent(st, join_ev, 0);     // the composite reads the LUTs and row states
   k += launch_fine(f, cfg, st);
   if (timed) cudaEventRecord(ev[2], st);
   return k;
