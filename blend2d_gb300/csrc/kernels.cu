@@ -1194,6 +1194,68 @@ __global__ void scan_add_kernel(uint32_t* out, const uint32_t* block_offsets, ui
     if (i < n) out[i] += add;
 }
 
+// The frame's four scans - slots, gradient row states and conic row runs per command, list entries per
+// list row - with their totals, together: one launch of a block per array while the longest has at
+// most kScanSmall elements, else three launches over all four. Each array on its own, with a launch
+// for its total, took 8 launches on small frames and 16 on larger ones, at 2 to 3 us each.
+struct ScanJobs {
+  const uint32_t* in[4];
+  uint32_t* out[4];
+  uint32_t* total[4];
+  uint32_t* sums[4];                   // a word per tile of kScanTile elements
+  uint32_t n[4];
+};
+constexpr uint32_t kScanSmall = 16384;
+constexpr int kScanWide = 1024;        // threads of the blocks that walk a whole array
+
+// One array (in may equal out), by one block; the total goes to `total`.
+__device__ __forceinline__ void scan_by_block(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* total, uint32_t* smem) {
+  uint32_t carry = 0;
+  for (uint32_t first = 0; first < n; first += uint32_t(kScanWide * kScanItems)) {
+    const uint32_t base = first + threadIdx.x * kScanItems;
+    uint32_t v[kScanItems], sum = 0, all;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) { v[k] = base + k < n ? in[base + k] : 0u; sum += v[k]; }
+    uint32_t off = carry + block_exclusive_scan(sum, smem, all);
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) { if (base + k < n) out[base + k] = off; off += v[k]; }
+    carry += all;
+  }
+  if (threadIdx.x == 0 && total) *total = carry;
+}
+
+__global__ void __launch_bounds__(kScanWide) scan_arrays_kernel(ScanJobs j, int of_sums) {
+  __shared__ uint32_t smem[32];
+  const int a = blockIdx.x;
+  if (of_sums) scan_by_block(j.sums[a], j.sums[a], (j.n[a] + kScanTile - 1) / kScanTile, j.total[a], smem);
+  else scan_by_block(j.in[a], j.out[a], j.n[a], j.total[a], smem);
+}
+
+__global__ void __launch_bounds__(kScanThreads) scan_arrays_tiles_kernel(ScanJobs j) {
+  __shared__ uint32_t smem[32];
+  const int a = blockIdx.y;
+  const uint32_t n = j.n[a], base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+  if (blockIdx.x * kScanTile >= n) return;
+  uint32_t v[kScanItems], sum = 0, total;
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) { v[k] = base + k < n ? j.in[a][base + k] : 0u; sum += v[k]; }
+  uint32_t off = block_exclusive_scan(sum, smem, total);
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) { if (base + k < n) j.out[a][base + k] = off; off += v[k]; }
+  if (threadIdx.x == 0) j.sums[a][blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kScanThreads) scan_arrays_add_kernel(ScanJobs j) {
+  const int a = blockIdx.y;
+  const uint32_t n = j.n[a];
+  if (blockIdx.x * kScanTile >= n) return;
+  const uint32_t add = j.sums[a][blockIdx.x];
+  uint32_t i = blockIdx.x * kScanTile + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++, i += kScanThreads)
+    if (i < n) j.out[a][i] += add;
+}
+
 // ---------------------------------------------------------------------------------------------
 // K2 - binning
 // ---------------------------------------------------------------------------------------------
@@ -1213,9 +1275,29 @@ __global__ void frame_gate_kernel(FrameView f) {
 
 __device__ __forceinline__ bool frame_skipped(const FrameView& f) { return f.work_counter[kSkipWord] != 0u; }
 
-// Tile ranges of every command (empty commands get 0xFFFFFFFF) and its number of tile rows.
-__global__ void cmd_tiles_kernel(FrameView f, uint32_t* cmdrow_counts_per_cmd, uint32_t* row_counts) {
+// Tile/row bookkeeping: canvas of every global tile and list row, identity processing order.
+__device__ __forceinline__ void tile_setup(const FrameView& f, uint32_t i, uint32_t* row_canvas) {
+  const uint32_t num_canvases = f.counts[kCntCanvases];
+  // binary search the canvas owning tile i / row i
+  if (i < f.counts[kCntTiles]) {
+    uint32_t lo = 0, hi = num_canvases - 1;
+    while (lo < hi) { uint32_t mid = (lo + hi + 1) >> 1; if (f.canvases[mid].tile_base <= i) lo = mid; else hi = mid - 1; }
+    f.tile_canvas[i] = lo;
+    f.tile_order[i] = i;
+  }
+  const uint32_t log2 = kTileShift - f.list_shift;
+  if (i < (f.counts[kCntRows] << log2)) {
+    uint32_t lo = 0, hi = num_canvases - 1;
+    while (lo < hi) { uint32_t mid = (lo + hi + 1) >> 1; if ((f.canvases[mid].row_base << log2) <= i) lo = mid; else hi = mid - 1; }
+    row_canvas[i] = lo;
+  }
+}
+
+// Tile ranges of every command (empty commands get 0xFFFFFFFF) and its number of tile rows; the same
+// launch does the tiles' and list rows' bookkeeping.
+__global__ void cmd_tiles_kernel(FrameView f, uint32_t* cmdrow_counts_per_cmd, uint32_t* row_counts, uint32_t* row_canvas) {
   uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  tile_setup(f, c, row_canvas);
   if (c >= f.counts[kCntCmds]) {
     // entries beyond the frame's commands (up to the capacity the scans run over) count nothing
     if (c < f.num_cmds) { cmdrow_counts_per_cmd[c] = 0; f.rs_count[c] = 0; f.rb_count[c] = 0; }
@@ -2241,25 +2323,6 @@ __global__ void conic_rows_kernel(FrameView f) {
   }
 }
 
-// Tile/row bookkeeping: canvas of every global tile and tile row, identity processing order.
-__global__ void tile_setup_kernel(FrameView f, uint32_t* row_canvas) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t num_canvases = f.counts[kCntCanvases];
-  // binary search the canvas owning tile i / row i
-  if (i < f.counts[kCntTiles]) {
-    uint32_t lo = 0, hi = num_canvases - 1;
-    while (lo < hi) { uint32_t mid = (lo + hi + 1) >> 1; if (f.canvases[mid].tile_base <= i) lo = mid; else hi = mid - 1; }
-    f.tile_canvas[i] = lo;
-    f.tile_order[i] = i;
-  }
-  const uint32_t log2 = kTileShift - f.list_shift;
-  if (i < (f.counts[kCntRows] << log2)) {
-    uint32_t lo = 0, hi = num_canvases - 1;
-    while (lo < hi) { uint32_t mid = (lo + hi + 1) >> 1; if ((f.canvases[mid].row_base << log2) <= i) lo = mid; else hi = mid - 1; }
-    row_canvas[i] = lo;
-  }
-}
-
 }  // namespace blgpu
 
 // =============================================================================================
@@ -2295,24 +2358,6 @@ uint32_t scan_temp_words(uint32_t n) {
 
 __global__ void total_kernel(const uint32_t* counts, const uint32_t* offsets, uint32_t n, uint32_t* total) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *total = n ? offsets[n - 1] + counts[n - 1] : 0u;
-}
-
-// totals[k] += sum(in[0..n)) (totals zeroed by the caller).
-__global__ void sum_kernel(const uint32_t* in, uint32_t n, uint32_t* total) {
-  __shared__ uint32_t smem[32];
-  uint32_t v = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v += in[i];
-  uint32_t t;
-  block_exclusive_scan(v, smem, t);
-  if (threadIdx.x == 0) atomicAdd(total, t);
-}
-
-int launch_sum(const uint32_t* in, uint32_t n, uint32_t* total, cudaStream_t st) {
-  if (!n) return 0;
-  uint32_t blocks = cdiv(n, 1024);
-  if (blocks > 1024) blocks = 1024;
-  sum_kernel<<<blocks, 1024, 0, st>>>(in, n, total);
-  return 1;
 }
 
 int launch_total(const uint32_t* counts, const uint32_t* offsets, uint32_t n, uint32_t* total, cudaStream_t st) {
@@ -2354,10 +2399,32 @@ int launch_edges(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st) {
   return 5;
 }
 
-int launch_cmd_tiles(const FrameView& f, uint32_t* cmdrow_counts_per_cmd, cudaStream_t st) {
-  if (!f.num_cmds) return 0;
-  cmd_tiles_kernel<<<cdiv(f.num_cmds, 256), 256, 0, st>>>(f, cmdrow_counts_per_cmd, f.row_counts);
+int launch_cmd_tiles(const FrameView& f, uint32_t* cmdrow_counts_per_cmd, uint32_t* row_canvas, cudaStream_t st) {
+  const uint32_t list_rows = f.num_rows << (kTileShift - f.list_shift);
+  const uint32_t n = max(f.num_cmds, max(f.num_tiles, list_rows));
+  if (!n) return 0;
+  cmd_tiles_kernel<<<cdiv(n, 256), 256, 0, st>>>(f, cmdrow_counts_per_cmd, f.row_counts, row_canvas);
   return 1;
+}
+
+uint32_t frame_scan_words(uint32_t n) { return 4u * (cdiv(n, kScanTile) + 1u); }
+
+int launch_frame_scans(const FrameView& f, const uint32_t* cmdrow_per_cmd, uint32_t* tmp, cudaStream_t st) {
+  const uint32_t list_rows = f.num_rows << (kTileShift - f.list_shift);
+  const uint32_t longest = max(f.num_cmds, list_rows), tiles = cdiv(longest, kScanTile);
+  const ScanJobs j{{cmdrow_per_cmd, f.row_counts, f.rs_count, f.rb_count},
+                   {f.cmdrow_base, f.row_offsets, f.rs_base, f.rb_base},
+                   {f.totals + 2, f.totals + 3, f.totals + 4, f.totals + 6},
+                   {tmp, tmp + tiles, tmp + 2 * tiles, tmp + 3 * tiles},
+                   {f.num_cmds, list_rows, f.num_cmds, f.num_cmds}};
+  if (longest <= kScanSmall) {
+    scan_arrays_kernel<<<4, kScanWide, 0, st>>>(j, 0);
+    return 1;
+  }
+  scan_arrays_tiles_kernel<<<dim3(tiles, 4), kScanThreads, 0, st>>>(j);
+  scan_arrays_kernel<<<4, kScanWide, 0, st>>>(j, 1);
+  scan_arrays_add_kernel<<<dim3(tiles, 4), kScanThreads, 0, st>>>(j);
+  return 3;
 }
 
 template<bool kScatter>
@@ -2369,13 +2436,11 @@ static int launch_seg_bin(const FrameView& f, cudaStream_t st) {
 }
 int launch_bin_count(const FrameView& f, cudaStream_t st) { return launch_seg_bin<false>(f, st); }
 
-int launch_rows_and_tiles(const FrameView& f, uint32_t* row_canvas, cudaStream_t st) {
-  int k = 0;
+int launch_rows(const FrameView& f, uint32_t* row_canvas, cudaStream_t st) {
   const uint32_t list_rows = f.num_rows << (kTileShift - f.list_shift);
-  uint32_t n = f.num_tiles > list_rows ? f.num_tiles : list_rows;
-  if (n) { tile_setup_kernel<<<cdiv(n, 256), 256, 0, st>>>(f, row_canvas); k++; }
-  if (list_rows) { row_fill_kernel<<<list_rows, 512, 0, st>>>(f, row_canvas); k++; }
-  return k;
+  if (!list_rows) return 0;
+  row_fill_kernel<<<list_rows, 512, 0, st>>>(f, row_canvas);
+  return 1;
 }
 
 int fine_grid_size(int blocks_per_sm) {

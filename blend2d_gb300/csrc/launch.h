@@ -31,13 +31,15 @@ inline uint32_t list_shift_of(const LaunchConfig& c) {
 int exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* tmp, cudaStream_t st);
 uint32_t scan_temp_words(uint32_t n);
 int launch_total(const uint32_t* counts, const uint32_t* offsets, uint32_t n, uint32_t* total, cudaStream_t st);
-int launch_sum(const uint32_t* in, uint32_t n, uint32_t* total, cudaStream_t st);
 
 int launch_lut(const FrameView& f, cudaStream_t st);
 int launch_edges(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st);
-int launch_cmd_tiles(const FrameView& f, uint32_t* cmdrow_counts_per_cmd, cudaStream_t st);
+int launch_cmd_tiles(const FrameView& f, uint32_t* cmdrow_counts_per_cmd, uint32_t* row_canvas, cudaStream_t st);
+// The frame's scans and their totals; `tmp` holds frame_scan_words(longest array) words.
+int launch_frame_scans(const FrameView& f, const uint32_t* cmdrow_per_cmd, uint32_t* tmp, cudaStream_t st);
+uint32_t frame_scan_words(uint32_t n);
 int launch_bin_count(const FrameView& f, cudaStream_t st);
-int launch_rows_and_tiles(const FrameView& f, uint32_t* row_canvas, cudaStream_t st);
+int launch_rows(const FrameView& f, uint32_t* row_canvas, cudaStream_t st);
 int launch_fine(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st);
 int launch_row_states(const FrameView& f, cudaStream_t st);
 int launch_frame_gate(const FrameView& f, cudaStream_t st);

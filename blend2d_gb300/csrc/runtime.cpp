@@ -537,7 +537,6 @@ BLGpuResult Runtime::upload_frame(const Frame& fr, const FrameSizes* caps) {
     v.cmdrow_base = L.take<uint32_t>(nc + 1);
     // command-list rows: room for the smallest list-row height
     const size_t list_rows = (size_t(z.rows) << kMaxListLog2) + 1;
-    v.row_counts = L.take<uint32_t>(list_rows);
     v.row_offsets = L.take<uint32_t>(list_rows);
     v.row_copies = L.take<uint32_t>(list_rows);
     v.strip_start = L.take<uint32_t>((size_t(z.tiles) + 1) * (kTileH / kStripRows));
@@ -548,7 +547,8 @@ BLGpuResult Runtime::upload_frame(const Frame& fr, const FrameSizes* caps) {
     // [0] work queue, [1] line items, [2] cubic curves, [3] their queue, [4..12) totals,
     // [12..16) error flags, [16..20) pixel ops (2 x u64), [21] quadratic / conic curves, [22] their
     // queue
-    v.work_counter = L.take<uint32_t>(kCounterWords);
+    v.work_counter = L.take<uint32_t>(kCounterWords + list_rows);        // cleared together with row_counts
+    v.row_counts = v.work_counter + kCounterWords;
     v.totals = v.work_counter + 4;
     v.error_flags = v.work_counter + 12;
     v.pixel_ops = reinterpret_cast<unsigned long long*>(v.work_counter + 16);
@@ -556,7 +556,7 @@ BLGpuResult Runtime::upload_frame(const Frame& fr, const FrameSizes* caps) {
     v.rs_base = L.take<uint32_t>(nc + 1);
     v.rb_count = L.take<uint32_t>(nc + 1);
     v.rb_base = L.take<uint32_t>(nc + 1);
-    scan_tmp = L.take<uint32_t>(scan_temp_words(std::max<uint32_t>(nc + 1, (z.rows << kMaxListLog2) + 1)));
+    scan_tmp = L.take<uint32_t>(frame_scan_words(std::max<uint32_t>(nc, z.rows << kMaxListLog2)));
     return staged_end;
   };
 
@@ -690,8 +690,8 @@ int Runtime::enqueue_count_half(cudaStream_t st) {
   const FrameView& f = view;
   const uint32_t list_rows = f.num_rows << (kTileShift - f.list_shift);
   int k = 0;
-  cudaMemsetAsync(f.work_counter, 0, sizeof(uint32_t) * kCounterWords, st);
-  cudaMemsetAsync(f.row_counts, 0, sizeof(uint32_t) * (list_rows + 1), st);
+  // the counters, and the list rows' entry counts behind them
+  cudaMemsetAsync(f.work_counter, 0, sizeof(uint32_t) * (kCounterWords + list_rows + 1), st);
   if (f.num_lut_jobs) {
     cudaEventRecord(fork_ev, st);
     cudaStreamWaitEvent(side, fork_ev, 0);
@@ -704,23 +704,16 @@ int Runtime::enqueue_count_half(cudaStream_t st) {
     k += launch_stroke_emit(f, st);
   }
   k += launch_edges(f, cfg, st);
-  k += launch_cmd_tiles(f, cmdrow_per_cmd, st);
-  k += exclusive_scan(cmdrow_per_cmd, f.cmdrow_base, f.num_cmds, scan_tmp, st);
-  k += launch_total(cmdrow_per_cmd, f.cmdrow_base, f.num_cmds, f.totals + 2, st);
-  k += exclusive_scan(f.row_counts, f.row_offsets, list_rows, scan_tmp, st);
-  k += launch_total(f.row_counts, f.row_offsets, list_rows, f.totals + 3, st);
-  k += exclusive_scan(f.rs_count, f.rs_base, f.num_cmds, scan_tmp, st);
-  k += launch_total(f.rs_count, f.rs_base, f.num_cmds, f.totals + 4, st);
-  k += exclusive_scan(f.rb_count, f.rb_base, f.num_cmds, scan_tmp, st);
-  k += launch_total(f.rb_count, f.rb_base, f.num_cmds, f.totals + 6, st);
+  k += launch_cmd_tiles(f, cmdrow_per_cmd, row_canvas, st);
+  k += launch_frame_scans(f, cmdrow_per_cmd, scan_tmp, st);
   return k;
 }
 
 // Rendering half: segments binned into (command, strip, tile) slots, row command lists, the
 // coverage pass, the composite pass.
-int Runtime::enqueue_render_half(cudaStream_t st, bool timed) {
+int Runtime::enqueue_render_half(cudaStream_t st, bool timed, bool gated) {
   const FrameView& f = view;
-  int k = launch_frame_gate(f, st);
+  int k = gated ? launch_frame_gate(f, st) : 0;
   // The gradients' row states (a conic's is a serial FP64 chain of up to a band of rows, or of the whole
   // box) are read by the composite only: on the side stream, beside the binning and coverage passes.
   if (f.num_row_states) {
@@ -729,10 +722,10 @@ int Runtime::enqueue_render_half(cudaStream_t st, bool timed) {
     k += launch_row_states(f, side);
     cudaEventRecord(join_ev, side);
   }
-  cudaMemsetAsync(f.slot_mask, 0, sizeof(uint32_t) * (f.num_cmdrows + 1), st);
-  cudaMemsetAsync(f.backdrop, 0, sizeof(uint32_t) * kStripRows * (size_t(f.num_cmdrows) + 1), st);
+  // the slots' backdrops, and their segment counts behind them
+  cudaMemsetAsync(f.backdrop, 0, sizeof(uint32_t) * (kStripRows + 1) * (size_t(f.num_cmdrows) + 1), st);
   k += launch_bin_count(f, st);
-  k += launch_rows_and_tiles(f, row_canvas, st);
+  k += launch_rows(f, row_canvas, st);
   // the fine stage: coverage (masks of analytic fills) + composite, timed together
   if (timed) cudaEventRecord(ev[1], st);
   k += launch_coverage(f, cfg, st);
@@ -747,8 +740,8 @@ int Runtime::enqueue_render_half(cudaStream_t st, bool timed) {
 // work items), and each has one block of masks.
 static void plan_dynamic(Layout& L, FrameView& v, const FrameTotals& t) {
   const uint32_t slots = std::min(t.cmdrows, t.seglist);
-  v.slot_mask = L.take<uint32_t>(size_t(t.cmdrows) + 1);
-  v.backdrop = L.take<uint32_t>((size_t(t.cmdrows) + 1) * kStripRows);
+  v.backdrop = L.take<uint32_t>((size_t(t.cmdrows) + 1) * (kStripRows + 1));   // cleared together
+  v.slot_mask = v.backdrop + (size_t(t.cmdrows) + 1) * kStripRows;
   v.entries = L.take<uint2>(size_t(t.seglist) + 1);
   v.mask_cursor = L.take<uint32_t>(size_t(slots) + 1);
   v.mask_info = L.take<uint4>(size_t(slots) + 1);
@@ -947,7 +940,7 @@ BLGpuResult Runtime::run_graph(const Frame& fr) {
     cudaGraph_t g = nullptr;
     BLGPU_CHECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     int launches = enqueue_count_half(stream);
-    launches += enqueue_render_half(stream, false);
+    launches += enqueue_render_half(stream, false, true);
     cudaError_t e = cudaStreamEndCapture(stream, &g);
     if (e != cudaSuccess) return cuda_result(e);
     e = cudaGraphInstantiate(&graph, g, 0);
@@ -1058,7 +1051,7 @@ BLGpuResult Runtime::run_eager(const Frame& fr) {
   planned_list_shift = list_shift_of(cfg);
   last_frame_bytes = in_bytes + stroke_bytes + measure.off + uint64_t(totals.segs) * (sizeof(DevSeg) + sizeof(uint32_t));
 
-  launches += enqueue_render_half(stream, true);
+  launches += enqueue_render_half(stream, true, false);
   BLGPU_CHECK(cudaGetLastError());
   BLGPU_CHECK(cudaEventRecord(ev[3], stream));
   // error flags and pixel-op counters in one read-back
@@ -1131,7 +1124,6 @@ BLGpuResult Runtime::run_noalloc(const Frame& fr) {
     a_cmdrow_per_cmd = L.take<uint32_t>(nc + 1);
     v.cmdrow_base = L.take<uint32_t>(nc + 1);
     const size_t list_rows = (size_t(fr.rows) << kMaxListLog2) + 1;
-    v.row_counts = L.take<uint32_t>(list_rows);
     v.row_offsets = L.take<uint32_t>(list_rows);
     v.row_copies = L.take<uint32_t>(list_rows);
     v.strip_start = L.take<uint32_t>((size_t(fr.tiles) + 1) * (kTileH / kStripRows));
@@ -1139,7 +1131,8 @@ BLGpuResult Runtime::run_noalloc(const Frame& fr) {
     a_row_canvas = L.take<uint32_t>(list_rows);
     v.tile_order = L.take<uint32_t>(fr.tiles + 1);
     v.tile_canvas = L.take<uint32_t>(fr.tiles + 1);
-    v.work_counter = L.take<uint32_t>(kCounterWords);
+    v.work_counter = L.take<uint32_t>(kCounterWords + list_rows);        // cleared together with row_counts
+    v.row_counts = v.work_counter + kCounterWords;
     v.totals = v.work_counter + 4;
     v.error_flags = v.work_counter + 12;
     v.pixel_ops = reinterpret_cast<unsigned long long*>(v.work_counter + 16);
@@ -1147,7 +1140,7 @@ BLGpuResult Runtime::run_noalloc(const Frame& fr) {
     v.rs_base = L.take<uint32_t>(nc + 1);
     v.rb_count = L.take<uint32_t>(nc + 1);
     v.rb_base = L.take<uint32_t>(nc + 1);
-    a_scan_tmp = L.take<uint32_t>(scan_temp_words(std::max<uint32_t>(nc + 1, (fr.rows << kMaxListLog2) + 1)));
+    a_scan_tmp = L.take<uint32_t>(frame_scan_words(std::max<uint32_t>(nc, fr.rows << kMaxListLog2)));
     v.counts = L.take<uint32_t>(kCntWords);
   };
   Layout L;
@@ -1229,7 +1222,7 @@ BLGpuResult Runtime::run_noalloc(const Frame& fr) {
     D.off = dyn_begin;
     plan_dynamic(D, view, t);
     if (D.off > kNoAllocArenaBytes) { r = BLGPU_ERROR_DATA_TOO_LARGE; break; }
-    launches += enqueue_render_half(stream, false);
+    launches += enqueue_render_half(stream, false, false);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(host_totals + 20, view.error_flags, 4, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
@@ -1279,7 +1272,7 @@ BLGpuResult Runtime::replay(bool use_graph) {
   if (!use_graph) {
     BLGPU_CHECK(cudaEventRecord(ev[0], stream));
     int launches = enqueue_count_half(stream);
-    launches += enqueue_render_half(stream, true);
+    launches += enqueue_render_half(stream, true, view_by_caps);
     BLGPU_CHECK(cudaGetLastError());
     BLGPU_CHECK(cudaEventRecord(ev[3], stream));
     stats.kernel_launches = uint64_t(launches);
@@ -1292,7 +1285,7 @@ BLGpuResult Runtime::replay(bool use_graph) {
     cudaGraph_t g = nullptr;
     BLGPU_CHECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     int launches = enqueue_count_half(stream);
-    launches += enqueue_render_half(stream, false);
+    launches += enqueue_render_half(stream, false, view_by_caps);
     cudaError_t e = cudaStreamEndCapture(stream, &g);
     if (e != cudaSuccess) return cuda_result(e);
     e = cudaGraphInstantiate(&graph, g, 0);

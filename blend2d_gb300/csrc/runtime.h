@@ -259,7 +259,8 @@ struct Runtime {
 
  private:
   int enqueue_count_half(cudaStream_t st);
-  int enqueue_render_half(cudaStream_t st, bool timed);
+  // `gated`: the arrays are sized by capacities, which the counting half's totals may exceed.
+  int enqueue_render_half(cudaStream_t st, bool timed, bool gated);
   BLGpuResult prepare_strokes(const Frame& fr, FrameView& v, uint32_t& outline_verts);
   // Fills host_counts with the frame's sizes and copies them to `dev` on the stream.
   cudaError_t put_counts(const Frame& fr, uint32_t* dev);
