@@ -59,6 +59,8 @@ enum ErrorFlag : uint32_t {
 constexpr int kSkipWord = 27;
 // work_counter[kMaskAlloc], [kMaskAlloc + 1]: work items and masks handed out, one 64-bit counter.
 constexpr int kMaskAlloc = 32;
+// work_counter[kSpilled], [kSpillQueue]: strips the composite left to its tail launch, and their queue.
+constexpr int kSpilled = 40, kSpillQueue = 41;
 
 enum FetchKind : uint32_t {
   kFetchSolid = 0,
@@ -330,6 +332,7 @@ struct FrameView {
   uint32_t* row_copies;        // [num_rows] SrcCopy commands in each tile row's list
   uint32_t* strip_start;       // [num_tiles * strips per tile] first list entry the composite needs (occlusion)
   uint32_t* strip_cmd;         // the same as a command: no command of the canvas before it shows in the strip
+  uint32_t* spilled;           // [num_tiles * strips per tile] strips whose list the composite's tail launch finishes
   uint32_t* tile_order;        // tile processing order for the persistent fine kernel
   uint32_t* tile_canvas;       // canvas index per global tile
   uint32_t* work_counter;      // [0] fine work queue, [1] items, [2] cubics, [21] quads, [23] / [25] cubic / quadratic

@@ -1861,8 +1861,9 @@ __global__ void __launch_bounds__(32 * kCoverWarps) coverage_kernel(FrameView f)
 // lane from the coverage pass, box fills compute theirs, then fetch + SrcOver/SrcCopy.
 // ---------------------------------------------------------------------------------------------
 
-// Masks of the lane's four pixels as bytes of a word, for a command without stored masks: boxes from
-// their rectangles.
+// Masks of the lane's PX pixels (from xp on) as bytes of a word, for a command without stored masks:
+// boxes from their rectangles.
+template<int PX>
 __device__ __forceinline__ uint32_t box_masks(const FrameView& f, uint32_t kind, uint32_t ci, uint32_t alpha, uint32_t xr,
                                               uint32_t yr, int xp, int y) {
   uint32_t w = 0;
@@ -1870,7 +1871,7 @@ __device__ __forceinline__ uint32_t box_masks(const FrameView& f, uint32_t kind,
     const int x0 = int(xr & 0xFFFFu), x1 = int(xr >> 16);
     if (y >= int(yr & 0xFFFFu) && y <= int(yr >> 16)) {
 #pragma unroll
-      for (int k = 0; k < 4; k++) w |= (xp + k >= x0 && xp + k <= x1) ? alpha << (8 * k) : 0u;
+      for (int k = 0; k < PX; k++) w |= (xp + k >= x0 && xp + k <= x1) ? alpha << (8 * k) : 0u;
     }
     return w;
   }
@@ -1882,7 +1883,7 @@ __device__ __forceinline__ uint32_t box_masks(const FrameView& f, uint32_t kind,
     const uint8_t* row = reinterpret_cast<const uint8_t*>(f.images) +
                          ((uint64_t(cmd.xform) << 32) | cmd.geom_first) + int64_t(y - cmd.box[1]) * cmd.geom_count;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
+    for (int k = 0; k < PX; k++) {
       if (in_y && xp + k >= cmd.box[0] && xp + k < cmd.box[2]) {
         uint32_t v = __ldg(row + (xp + k - cmd.box[0]));
         if (alpha < 255u) v = ((v * alpha + 0x80u) * 0x101u) >> 16;
@@ -1892,7 +1893,7 @@ __device__ __forceinline__ uint32_t box_masks(const FrameView& f, uint32_t kind,
     return w;
   }
 #pragma unroll
-  for (int k = 0; k < 4; k++) w |= px::box_u_mask(cmd.box, alpha, xp + k, y) << (8 * k);
+  for (int k = 0; k < PX; k++) w |= px::box_u_mask(cmd.box, alpha, xp + k, y) << (8 * k);
   return w;
 }
 
@@ -1912,9 +1913,10 @@ __device__ __forceinline__ uint32_t strip_slot(const FrameView& f, uint32_t slot
   return slot;
 }
 
-// The bytes of a lane's mask word whose pixels lie on the canvas.
+// The bytes of a lane's mask word whose PX pixels lie on the canvas.
+template<int PX>
 __device__ __forceinline__ uint32_t pixels_on_canvas(int xp, int y, const DevCanvas& cv) {
-  const int n = y < cv.h ? min(max(cv.w - xp, 0), 4) : 0;
+  const int n = y < cv.h ? min(max(cv.w - xp, 0), PX) : 0;
   return n == 4 ? 0xFFFFFFFFu : (1u << (8 * n)) - 1u;
 }
 
@@ -2020,85 +2022,107 @@ __global__ void __launch_bounds__(kFineThreads) cull_kernel(FrameView f) {
   }
 }
 
-// The four pixels of a lane composited with their sources and mask bytes. A zero mask byte leaves
+// The PX pixels of a lane composited with their sources and mask bytes. A zero mask byte leaves
 // its pixel as it is (SrcOver: the scaled source is 0 and d * 255 / 255 gives d; SrcCopy likewise),
 // so no pixel needs a branch.
-__device__ __forceinline__ void composite4(uint32_t pix[4], const uint32_t sv[4], uint32_t mw, bool src_copy) {
+template<int PX>
+__device__ __forceinline__ void composite(uint32_t pix[PX], const uint32_t sv[PX], uint32_t mw, bool src_copy) {
   if (src_copy) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) pix[k] = px::src_copy(pix[k], sv[k], __byte_perm(mw, 0u, 0x4440u + k));
+    for (int k = 0; k < PX; k++) pix[k] = px::src_copy(pix[k], sv[k], __byte_perm(mw, 0u, 0x4440u + k));
   }
   else {
 #pragma unroll
-    for (int k = 0; k < 4; k++) pix[k] = px::src_over(pix[k], sv[k], __byte_perm(mw, 0u, 0x4440u + k));
+    for (int k = 0; k < PX; k++) pix[k] = px::src_over(pix[k], sv[k], __byte_perm(mw, 0u, 0x4440u + k));
   }
 }
 
-// Sources of the lane's four pixels (those with a mask byte) for a gradient style.
-__device__ __forceinline__ void gradient4(const FrameView& f, uint32_t style, uint32_t fetch, bool dither, uint32_t row_state,
-                                          int xp, int y, uint32_t mw, uint32_t sv[4]) {
+// Sources of the lane's PX pixels (those with a mask byte) for a gradient style.
+template<int PX>
+__device__ __forceinline__ void gradient_sources(const FrameView& f, uint32_t style, uint32_t fetch, bool dither, uint32_t row_state,
+                                          int xp, int y, uint32_t mw, uint32_t sv[PX]) {
   const DevStyle& st = f.styles[style];
   const uint4 common = *reinterpret_cast<const uint4*>(&st.maxi);      // maxi, rori, con_maxi, con_rori
   const uint32_t* lut = f.luts + st.lut_offset;
-  uint32_t idx[4];
+  uint32_t idx[PX];
   if (fetch <= kFetchLinearRoR) {
     const uint64_t dt = st.lin_dt;
     uint64_t pt = st.lin_pt0 + uint64_t(uint32_t(y)) * st.lin_dy + uint64_t(uint32_t(xp)) * dt;
 #pragma unroll
-    for (int k = 0; k < 4; k++, pt += dt) idx[k] = px::grad_index(uint32_t(pt >> 32), fetch == kFetchLinearPad, common.x, common.y);
+    for (int k = 0; k < PX; k++, pt += dt) idx[k] = px::grad_index(uint32_t(pt >> 32), fetch == kFetchLinearPad, common.x, common.y);
   }
   else {
     const float4 rs = f.row_states[row_state];
     if (fetch <= kFetchRadialRoR) {
       const float2 r = *reinterpret_cast<const float2*>(&st.rad_bd);   // bd, ddd
 #pragma unroll
-      for (int k = 0; k < 4; k++) idx[k] = px::radial_index(r.x, r.y, rs.x, rs.y, rs.z, xp + k, fetch == kFetchRadialPad, common.x, common.y);
+      for (int k = 0; k < PX; k++) idx[k] = px::radial_index(r.x, r.y, rs.x, rs.y, rs.z, xp + k, fetch == kFetchRadialPad, common.x, common.y);
     }
     else {
       const float4 q = *reinterpret_cast<const float4*>(st.con_q);
       const float4 n = *reinterpret_cast<const float4*>(&st.con_n1);   // n1, n2, n4, offset
       const float xx = st.con_xx;
 #pragma unroll
-      for (int k = 0; k < 4; k++) idx[k] = px::conic_index(q, n, xx, rs.x, rs.y, rs.z, xp + k, int32_t(common.z), common.w);
+      for (int k = 0; k < PX; k++) idx[k] = px::conic_index(q, n, xx, rs.x, rs.y, rs.z, xp + k, int32_t(common.z), common.w);
     }
   }
   if (!dither) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) sv[k] = (mw >> (8 * k)) & 0xFFu ? __ldg(lut + idx[k]) : 0u;
+    for (int k = 0; k < PX; k++) sv[k] = (mw >> (8 * k)) & 0xFFu ? __ldg(lut + idx[k]) : 0u;
   }
   else {
     // 64-bit entries (lut_offset is even) + the ordered-dither threshold of each pixel
-    uint2 e[4];
+    uint2 e[PX];
 #pragma unroll
-    for (int k = 0; k < 4; k++)
+    for (int k = 0; k < PX; k++)
       e[k] = (mw >> (8 * k)) & 0xFFu ? __ldg(reinterpret_cast<const uint2*>(lut) + idx[k]) : make_uint2(0u, 0u);
 #pragma unroll
-    for (int k = 0; k < 4; k++) sv[k] = px::dither_pixel(e[k], px::dither_threshold(xp + k, y));
+    for (int k = 0; k < PX; k++) sv[k] = px::dither_pixel(e[k], px::dither_threshold(xp + k, y));
   }
 }
+
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 // 32-entry chunks of the strip's command list: every lane tests one command's box and gathers what
 // the strip needs of it - a stored mask's index, or the four row masks of a slot no segment reaches, which
 // drops the command when they are all zero - so the loop over the chunk's commands, in painter's order,
-// only broadcasts. It is pipelined by one command: a command's source loads are under way while the
+// only broadcasts, and has the stored masks, the style and the row states it will read brought to the
+// L1 (composite of 512 canvases of the batch 5.07 -> 4.44 ms: a load from the L2 is as long as a command's
+// arithmetic). The loop is pipelined by one command: a command's source loads are under way while the
 // one before it is composited. Bound: instruction issue on full grids, and the latency of a strip's
 // chain of commands where few strips have long lists. The whole composite (with the cull pass), against
 // per-pixel branches, one command at a time and masks found in the loop: 512 canvases of the batch 8.4
 // -> 6.0 ms, 20,000 curve paths on 1920x1080 0.66 -> 0.46, 32 requests of up to 1024x1024 0.95 -> 0.56.
 // Four blocks per SM (64 registers): three (80) 6.6 ms on the batch, five (48, spilling) 6.2.
+//
+// A warp takes a strip, four pixels a lane. With a tail launch to follow (kSpill), a warp that has come
+// through kSpillHits commands while no strip is left to start, and has a good part of its list before it,
+// writes its pixels back and leaves the rest to four warps of that launch (kTail), a row of the strip
+// and one pixel a lane each, so that a few strips with long lists do not run alone. That pays where
+// strips differ, in frames of several canvases: composite of 512 canvases of the batch 4.44 -> 4.07 ms, 32
+// requests of up to 1024x1024 0.45 -> 0.43; on one canvas the strips' lists are alike and the launch costs 6 to 14
+// us (20,000 curve paths 0.451 -> 0.465). Rows from the start, for frames of few strips, were slower (2,000
+// polygons on 512x512 0.041 -> 0.055): a command costs a warp nearly as much for 32 pixels as for 128.
+enum FineMode : int { kStrips = 0, kSpill = 1, kTail = 2 };
+constexpr uint32_t kSpillHits = 64, kSpillLeft = 64;
+
+template<int kMode>
 __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(FrameView f) {
+  constexpr int PX = kMode == kTail ? 1 : 4;
   const int lane = threadIdx.x & 31;
-  const int prow = lane >> 3;            // row within the strip
-  const int pcol = (lane & 7) * 4;       // first of this lane's 4 columns
+  const int pcol = PX == 4 ? (lane & 7) * 4 : lane;     // first of this lane's columns
   uint32_t ops = 0, pat_ops = 0;         // composited pixels of this lane (all strips)
   if (frame_skipped(f)) return;
-  const uint32_t num_units = f.counts[kCntTiles] * kStripsPerTile;
+  const uint32_t num_strips = f.counts[kCntTiles] * kStripsPerTile;
+  const uint32_t num_units = kMode == kTail ? f.work_counter[kSpilled] * kStripRows : num_strips;
 
   for (;;) {
     uint32_t unit = 0;
-    if (lane == 0) unit = atomicAdd(f.work_counter, 1u);
+    if (lane == 0) unit = atomicAdd(f.work_counter + (kMode == kTail ? kSpillQueue : 0), 1u);
     unit = __shfl_sync(0xFFFFFFFFu, unit, 0);
     if (unit >= num_units) break;
+    const int prow = kMode == kTail ? int(unit % kStripRows) : lane >> 3;     // row within the strip
+    if (kMode == kTail) unit = f.spilled[unit / kStripRows];
     uint32_t tile = f.tile_order[unit / kStripsPerTile];
     int strip = int(unit % kStripsPerTile);
     const DevCanvas cv = f.canvases[f.tile_canvas[tile]];
@@ -2110,33 +2134,34 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
     const uint32_t strip_row = uint32_t(row0) >> kStripShift;
     int row1 = min(row0 + kStripRows, cv.h) - 1;     // last row of the strip inside the canvas
     const int y = row0 + prow, xp = x_base + pcol;
-    const uint32_t on_canvas = pixels_on_canvas(xp, y, cv);
+    const uint32_t on_canvas = pixels_on_canvas<PX>(xp, y, cv);
+    if (kMode == kTail && y >= cv.h) continue;
     uint32_t* dst = cv.pixels + int64_t(y) * cv.stride + xp;
     // an A8 canvas: one byte per pixel, composited as the alpha byte of a 32-bit pixel (the
     // reference's P8_Alpha operators are its P32 operators' alpha lane); rows start at 16-byte
     // boundaries and xp is a multiple of 4, so 4 pixels are one aligned word
     uint8_t* dst8 = reinterpret_cast<uint8_t*>(cv.pixels) + int64_t(y) * cv.stride + xp;
 
-    uint32_t pix[4];
-    const bool full = on_canvas == 0xFFFFFFFFu;
+    uint32_t pix[PX];
+    const bool full = PX == 4 && on_canvas == 0xFFFFFFFFu;
     if (cv.a8) {
       if (full) {
         const uint32_t v = *reinterpret_cast<const uint32_t*>(dst8);
 #pragma unroll
-        for (int k = 0; k < 4; k++) pix[k] = ((v >> (8 * k)) & 0xFFu) << 24;
+        for (int k = 0; k < PX; k++) pix[k] = ((v >> (8 * k)) & 0xFFu) << 24;
       }
       else {
 #pragma unroll
-        for (int k = 0; k < 4; k++) pix[k] = ((on_canvas >> (8 * k)) & 1u) ? uint32_t(dst8[k]) << 24 : 0u;
+        for (int k = 0; k < PX; k++) pix[k] = ((on_canvas >> (8 * k)) & 1u) ? uint32_t(dst8[k]) << 24 : 0u;
       }
     }
     else if (full) {
       uint4 v = *reinterpret_cast<const uint4*>(dst);
-      pix[0] = v.x; pix[1] = v.y; pix[2] = v.z; pix[3] = v.w;
+      pix[0] = v.x; pix[1 % PX] = v.y; pix[2 % PX] = v.z; pix[3 % PX] = v.w;
     }
     else {
 #pragma unroll
-      for (int k = 0; k < 4; k++) pix[k] = ((on_canvas >> (8 * k)) & 1u) ? dst[k] : 0u;
+      for (int k = 0; k < PX; k++) pix[k] = ((on_canvas >> (8 * k)) & 1u) ? dst[k] : 0u;
     }
 
     const uint32_t row_id = (cv.row_base << (kTileShift - f.list_shift)) + (uint32_t(row0) >> f.list_shift);
@@ -2147,10 +2172,20 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
 
     const uint32_t start = f.strip_start[tile * kStripsPerTile + uint32_t(strip)];      // cull_kernel
     const uint32_t cover = f.strip_cmd[tile * kStripsPerTile + uint32_t(strip)];        // ... and coverage_kernel
-    uint32_t pend_mw = 0, pend[4] = {0u, 0u, 0u, 0u};   // the command to composite next
+    uint32_t pend_mw = 0, pend[PX] = {};   // the command to composite next
     bool pend_copy = false;
+    uint32_t done = 0;                               // commands composited
 
     for (uint32_t base = start & ~31u; base < list_count; base += 32) {
+      if (kMode == kSpill && done >= kSpillHits && list_count - base >= kSpillLeft &&
+          *reinterpret_cast<volatile const uint32_t*>(f.work_counter) >= num_units) {
+        // no strip is waiting to be started: the rest of this one's list goes to four warps
+        if (lane == 0) {
+          f.strip_start[tile * kStripsPerTile + uint32_t(strip)] = base;
+          f.spilled[atomicAdd(f.work_counter + kSpilled, 1u)] = unit;
+        }
+        break;
+      }
       // commands of this chunk whose pixel bbox overlaps the strip, in painter's order: one pair
       // of list records per lane holds everything the tests and the slot lookup need
       uint4 ra = make_uint4(0u, 0u, 0u, 0u), rb = ra;
@@ -2171,12 +2206,27 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
             const uint32_t slot = strip_slot(f, rb.x, rb.y, ra.z, strip_row, tx, nseg);
             stored = nseg != 0u;
             masks = nseg - 1u;
-            if (!stored) {
+            if (stored) {
+              prefetch_l1(f.masks + size_t(masks) * kSlotPixels);
+            }
+            else {
               const uint4 bd = *reinterpret_cast<const uint4*>(f.backdrop + size_t(slot) * kStripRows);
               const uint32_t flags = (ra.w >> 2) & 3u, alpha = (ra.w >> 4) & 0xFFu;
               masks = uniform_mask(bd.x, flags, alpha) | (uniform_mask(bd.y, flags, alpha) << 8) |
                       (uniform_mask(bd.z, flags, alpha) << 16) | (uniform_mask(bd.w, flags, alpha) << 24);
               hit = masks != 0u;
+            }
+          }
+          if (hit && !(rb.z & kRecSolid)) {
+            // what the loop will read of the style, while the other commands' turns last
+            const char* st = reinterpret_cast<const char*>(f.styles + rb.z);
+            prefetch_l1(st);
+            prefetch_l1(st + 64);
+            const uint32_t fetch = (ra.w >> kRecFetchShift) & 15u;
+            if (fetch >= kFetchPatAlignedPad) { prefetch_l1(st + 192); prefetch_l1(st + 256); }
+            else if (px::has_row_table(fetch)) {
+              prefetch_l1(st + 128);
+              prefetch_l1(f.row_states + rb.w + (max(uint32_t(row0), ra.z & 0xFFFFu) - (ra.z & 0xFFFFu)));
             }
           }
         }
@@ -2187,11 +2237,15 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
       // the first command's mask word, then each next one's while the current one is under way
       auto load_masks = [&](int from) -> uint32_t {
         const uint32_t v = __shfl_sync(0xFFFFFFFFu, masks, from);
+        if (PX == 1)
+          return (stored_set >> from) & 1u ? f.masks[size_t(v) * kSlotPixels + uint32_t(prow) * kTileW + uint32_t(lane)]
+                                           : (v >> (8 * prow)) & 0xFFu;
         return (stored_set >> from) & 1u ? reinterpret_cast<const uint32_t*>(f.masks + size_t(v) * kSlotPixels)[lane]
                                          : __byte_perm(v, 0u, 0x1111u * uint32_t(prow));
       };
       int bit = __ffs(todo) - 1;
       uint32_t next_mw = load_masks(bit);
+      done += uint32_t(__popc(todo));
       while (todo) {
         todo &= todo - 1;
         const uint32_t info = __shfl_sync(0xFFFFFFFFu, ra.w, bit);
@@ -2200,7 +2254,7 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
         const uint32_t yr = __shfl_sync(0xFFFFFFFFu, ra.z, bit);
         uint32_t mw = next_mw;
         if ((info & 3u) != kFillAnalytic)
-          mw = box_masks(f, info & 3u, __shfl_sync(0xFFFFFFFFu, ra.x, bit), (info >> 4) & 0xFFu,
+          mw = box_masks<PX>(f, info & 3u, __shfl_sync(0xFFFFFFFFu, ra.x, bit), (info >> 4) & 0xFFu,
                          __shfl_sync(0xFFFFFFFFu, ra.y, bit), yr, xp, y);
         if (todo) {
           bit = __ffs(todo) - 1;
@@ -2210,15 +2264,15 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
         if (!__any_sync(0xFFFFFFFFu, mw != 0u)) continue;
         const uint32_t n = uint32_t(__popc((((mw & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | mw) & 0x80808080u));   // nonzero bytes
         ops += n;
-        uint32_t sv[4] = {0u, 0u, 0u, 0u};
+        uint32_t sv[PX] = {};
         const uint32_t fetch = (info >> kRecFetchShift) & 15u;
         if (style & kRecSolid) {
 #pragma unroll
-          for (int k = 0; k < 4; k++) sv[k] = extra;
+          for (int k = 0; k < PX; k++) sv[k] = extra;
         }
         else if (fetch <= kFetchConic) {
           // a lane without masks may lie outside the command's rows: it reads no row state
-          if (mw) gradient4(f, style, fetch, info & kRecDither, extra + uint32_t(y) - (yr & 0xFFFFu), xp, y, mw, sv);
+          if (mw) gradient_sources<PX>(f, style, fetch, info & kRecDither, extra + uint32_t(y) - (yr & 0xFFFFu), xp, y, mw, sv);
         }
         else {
           pat_ops += n;
@@ -2227,37 +2281,38 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
           const px::RowState rs = px::row_state(st, y, 0);
           uint32_t m = mw;
 #pragma unroll 1
-          for (int k = 0; k < 4; k++, m >>= 8) {
+          for (int k = 0; k < PX; k++, m >>= 8) {
             uint32_t v = 0;
             if (m & 0xFFu) v = px::fetch(st, rs, xp + k, f.luts, f.images) | st.src_or;
-            sv[0] = sv[1]; sv[1] = sv[2]; sv[2] = sv[3]; sv[3] = v;
+            for (int j = 0; j + 1 < PX; j++) sv[j] = sv[j + 1];
+            sv[PX - 1] = v;
           }
         }
-        composite4(pix, pend, pend_mw, pend_copy);
+        composite<PX>(pix, pend, pend_mw, pend_copy);
         pend_mw = mw;
         pend_copy = (info >> 2) & 1u;
 #pragma unroll
-        for (int k = 0; k < 4; k++) pend[k] = sv[k];
+        for (int k = 0; k < PX; k++) pend[k] = sv[k];
       }
     }
-    composite4(pix, pend, pend_mw, pend_copy);
+    composite<PX>(pix, pend, pend_mw, pend_copy);
 
     if (cv.a8) {
       if (full) {
-        *reinterpret_cast<uint32_t*>(dst8) = (pix[0] >> 24) | ((pix[1] >> 24) << 8) | ((pix[2] >> 24) << 16) |
-                                             (pix[3] & 0xFF000000u);
+        *reinterpret_cast<uint32_t*>(dst8) = (pix[0] >> 24) | ((pix[1 % PX] >> 24) << 8) | ((pix[2 % PX] >> 24) << 16) |
+                                             (pix[3 % PX] & 0xFF000000u);
       }
       else {
 #pragma unroll
-        for (int k = 0; k < 4; k++) if ((on_canvas >> (8 * k)) & 1u) dst8[k] = uint8_t(pix[k] >> 24);
+        for (int k = 0; k < PX; k++) if ((on_canvas >> (8 * k)) & 1u) dst8[k] = uint8_t(pix[k] >> 24);
       }
     }
     else if (full) {
-      *reinterpret_cast<uint4*>(dst) = make_uint4(pix[0], pix[1], pix[2], pix[3]);
+      *reinterpret_cast<uint4*>(dst) = make_uint4(pix[0], pix[1 % PX], pix[2 % PX], pix[3 % PX]);
     }
     else {
 #pragma unroll
-      for (int k = 0; k < 4; k++) if ((on_canvas >> (8 * k)) & 1u) dst[k] = pix[k];
+      for (int k = 0; k < PX; k++) if ((on_canvas >> (8 * k)) & 1u) dst[k] = pix[k];
     }
   }
 
@@ -2443,9 +2498,10 @@ int launch_rows(const FrameView& f, uint32_t* row_canvas, cudaStream_t st) {
   return 1;
 }
 
-int fine_grid_size(int blocks_per_sm) {
+template<int kMode>
+static int fine_grid_size(int blocks_per_sm) {
   const int sms = device_sms();
-  static const int max_per_sm = max_blocks_per_sm(fine_kernel, kFineThreads);
+  static const int max_per_sm = max_blocks_per_sm(fine_kernel<kMode>, kFineThreads);
   return sms * (blocks_per_sm > 0 && blocks_per_sm < max_per_sm ? blocks_per_sm : max_per_sm);
 }
 
@@ -2495,10 +2551,14 @@ int launch_row_states(const FrameView& f, cudaStream_t st) {
 // work_counter must be zero on entry.
 int launch_fine(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st) {
   if (!f.num_tiles) return 0;
-  int grid = fine_grid_size(cfg.fine_blocks_per_sm);
-  uint32_t max_blocks = (f.num_tiles * kStripsPerTile + kFineWarps - 1) / kFineWarps;
-  if (uint32_t(grid) > max_blocks) grid = int(max_blocks);
-  fine_kernel<<<grid, kFineThreads, 0, st>>>(f);
+  const uint32_t strips = f.num_tiles * kStripsPerTile;
+  const uint32_t needed = cdiv(strips, kFineWarps);
+  if (f.num_canvases > 1) {
+    fine_kernel<kSpill><<<min(uint32_t(fine_grid_size<kSpill>(cfg.fine_blocks_per_sm)), needed), kFineThreads, 0, st>>>(f);
+    fine_kernel<kTail><<<min(uint32_t(fine_grid_size<kTail>(cfg.fine_blocks_per_sm)), needed * kStripRows), kFineThreads, 0, st>>>(f);
+    return 2;
+  }
+  fine_kernel<kStrips><<<min(uint32_t(fine_grid_size<kStrips>(cfg.fine_blocks_per_sm)), needed), kFineThreads, 0, st>>>(f);
   return 1;
 }
 

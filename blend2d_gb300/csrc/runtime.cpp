@@ -541,6 +541,7 @@ BLGpuResult Runtime::upload_frame(const Frame& fr, const FrameSizes* caps) {
     v.row_copies = L.take<uint32_t>(list_rows);
     v.strip_start = L.take<uint32_t>((size_t(z.tiles) + 1) * (kTileH / kStripRows));
     v.strip_cmd = L.take<uint32_t>((size_t(z.tiles) + 1) * (kTileH / kStripRows));
+    v.spilled = L.take<uint32_t>((size_t(z.tiles) + 1) * (kTileH / kStripRows));
     row_canvas = L.take<uint32_t>(list_rows);
     v.tile_order = L.take<uint32_t>(z.tiles + 1);
     v.tile_canvas = L.take<uint32_t>(z.tiles + 1);
@@ -1128,6 +1129,7 @@ BLGpuResult Runtime::run_noalloc(const Frame& fr) {
     v.row_copies = L.take<uint32_t>(list_rows);
     v.strip_start = L.take<uint32_t>((size_t(fr.tiles) + 1) * (kTileH / kStripRows));
     v.strip_cmd = L.take<uint32_t>((size_t(fr.tiles) + 1) * (kTileH / kStripRows));
+    v.spilled = L.take<uint32_t>((size_t(fr.tiles) + 1) * (kTileH / kStripRows));
     a_row_canvas = L.take<uint32_t>(list_rows);
     v.tile_order = L.take<uint32_t>(fr.tiles + 1);
     v.tile_canvas = L.take<uint32_t>(fr.tiles + 1);
