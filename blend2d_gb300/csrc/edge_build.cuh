@@ -538,6 +538,78 @@ __device__ int split_cubic(Pt* c) {
   return int(out - c);
 }
 
+// split_quad and split_cubic in steps for lanes that share a warp's curves: the curve's polynomial, a
+// set of candidate parameters, the cuts made of all candidates, and one piece between two cuts. The
+// operations and their order are those of the functions above; which lane does which step does not
+// matter to any of them.
+constexpr double kNoCut = 2.0;               // a candidate that is none (cuts lie in (0, 1))
+
+template<int DEG> struct Poly;
+template<> struct Poly<3> { Pt a, b, c, d; };
+template<> struct Poly<2> { Pt a, b, c; };
+
+__device__ __forceinline__ Poly<3> curve_poly(Pt c0, Pt c1, Pt c2, Pt c3) {
+  const Pt v1{c1.x - c0.x, c1.y - c0.y}, v2{c2.x - c1.x, c2.y - c1.y}, v3{c3.x - c2.x, c3.y - c2.y};
+  return Poly<3>{Pt{v3.x - v2.x - v2.x + v1.x, v3.y - v2.y - v2.y + v1.y}, Pt{3.0 * (v2.x - v1.x), 3.0 * (v2.y - v1.y)},
+                 Pt{3.0 * v1.x, 3.0 * v1.y}, c0};
+}
+__device__ __forceinline__ Poly<2> curve_poly(Pt c0, Pt c1, Pt c2) {
+  const Pt v1{c1.x - c0.x, c1.y - c0.y}, v2{c2.x - c1.x, c2.y - c1.y};
+  return Poly<2>{Pt{v2.x - v1.x, v2.y - v1.y}, Pt{v1.x + v1.x, v1.y + v1.y}, c0};
+}
+
+// Candidate sets of a cubic: 0 the cusp, 1 the inflections, 2 and 3 the extrema in x and y. At most two
+// values each; the derivative's coefficients are 3 a, 2 b and c exactly as split_cubic computes them (6
+// (v2 - v1) is 3 (v2 - v1) doubled).
+constexpr int kCubicSets = 4, kCubicCands = 7;
+__device__ __forceinline__ void cubic_candidates(const Poly<3>& p, int set, double out[2]) {
+  const double kAfter0 = 1e-40, kBefore1 = 0.999999999999999889;
+  out[0] = out[1] = kNoCut;
+  double ts[3];
+  int n;
+  if (set == 0) {
+    const double t = (cross(p.c, p.a) / cross(p.b, p.a)) * -0.5;
+    ts[0] = t;
+    n = int((t > 0.0) & (t < 1.0));
+  }
+  else {
+    double a, b, c;
+    if (set == 1) { a = cross(p.b, p.a) * 6.0; b = cross(p.c, p.a) * 6.0; c = cross(p.c, p.b) * 2.0; }
+    else if (set == 2) { a = 3.0 * p.a.x; b = 2.0 * p.b.x; c = p.c.x; }
+    else { a = 3.0 * p.a.y; b = 2.0 * p.b.y; c = p.c.y; }
+    n = quad_roots(ts, a, b, c, kAfter0, kBefore1);
+  }
+  if (n > 0) out[0] = ts[0];
+  if (n > 1) out[1] = ts[1];
+}
+
+// The point of the polynomial at t, and the piece between the cuts t0 and t1, which begins at `from` (the
+// curve's first point or the point at t0) and ends at `to` (the point at t1 or the curve's last one). A
+// curve without cuts is its own only piece.
+__device__ __forceinline__ Pt poly_point(const Poly<3>& p, double t) {
+  return Pt{((p.a.x * t + p.b.x) * t + p.c.x) * t + p.d.x, ((p.a.y * t + p.b.y) * t + p.c.y) * t + p.d.y};
+}
+__device__ __forceinline__ Pt poly_point(const Poly<2>& p, double t) {
+  return Pt{(p.a.x * t + p.b.x) * t + p.c.x, (p.a.y * t + p.b.y) * t + p.c.y};
+}
+__device__ __forceinline__ void poly_piece(const Poly<3>& p, double t0, double t1, Pt from, Pt to, Pt out[4]) {
+  const double k1Div3 = 1.0 / 3.0;
+  const double dt = (t1 - t0) * k1Div3;
+  const Pt cp1{((p.a.x * (t0 * 3.0) + p.b.x * 2.0) * t0 + p.c.x) * dt, ((p.a.y * (t0 * 3.0) + p.b.y * 2.0) * t0 + p.c.y) * dt};
+  const Pt cp2{((p.a.x * (t1 * 3.0) + p.b.x * 2.0) * t1 + p.c.x) * dt, ((p.a.y * (t1 * 3.0) + p.b.y * 2.0) * t1 + p.c.y) * dt};
+  out[0] = from;
+  out[1] = Pt{from.x + cp1.x, from.y + cp1.y};
+  out[2] = Pt{to.x - cp2.x, to.y - cp2.y};
+  out[3] = to;
+}
+__device__ __forceinline__ void poly_piece(const Poly<2>& p, double t0, double t1, Pt from, Pt to, Pt out[3]) {
+  const double dt = (t1 - t0) * 0.5;
+  const Pt cp{(p.a.x * (t1 * 2.0) + p.b.x) * dt, (p.a.y * (t1 * 2.0) + p.b.y) * dt};
+  out[0] = from;
+  out[1] = Pt{to.x - cp.x, to.y - cp.y};
+  out[2] = to;
+}
+
 struct Step { double value, limit; Pt p01, p12, p23, p012, p123, p0123; };
 
 __device__ __forceinline__ Pt mid(Pt a, Pt b) { return Pt{(a.x + b.x) * 0.5, (a.y + b.y) * 0.5}; }

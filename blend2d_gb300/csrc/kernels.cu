@@ -565,7 +565,7 @@ __device__ __forceinline__ void finish_curve(FrameView& f, eb::Builder& b, uint3
 // the batched workload (piece kernel 10.8 -> 14.2 ms): the shared-memory carve-out shrinks the L1
 // that the stacks' and the segment sinks' local memory hits in.
 constexpr int kCurveThreads = 128;
-constexpr uint32_t kSplitBlocksPerSM = 8;      // of each kind of curve
+constexpr uint32_t kSplitBlocksPerSM = 6;      // of each kind of curve
 // Idle lanes a warp waits for before it takes new pieces: each refill's set-up costs the warp its
 // FP64 instructions whatever the number of lanes refilled. On the batched workload 24 and 28
 // measured 246-248 ms per step, 16 and 20 250 ms, 32 251 ms, 8 257 ms and 4 259 ms.
@@ -578,137 +578,291 @@ constexpr uint32_t kPieceLeafLanes = 16;
 // quadratic and conic ones in the second, so that neither kind's tail waits for the other's and a
 // frame without one kind loses blocks that leave at once, not launches. (Not alternating blocks: the
 // even ones go to one half of the SMs, and a frame of cubics alone took twice as long.)
-// curve_split_kernel: one thread per curve does
-// curve_to's set-up (transform, clip flags, a curve entirely on one side of the clip box, the split
-// into monotonic pieces: the divergent, FP64-heavy part) with every lane converged on it, and
-// writes the pieces. edge_pieces_kernel flattens the clipped pieces lane-scheduled, so taking a new
-// piece is cheap and the lanes' subdivision steps stay together; edge_tree_kernel then flattens what
-// no clip touches. A piece is built by its own
-// builder: the border runs a curve accumulates are vertical lines at the clip box's x0/x1 whose
-// cells add up the same whether the runs of consecutive pieces are merged or not.
+// curve_split_kernel does curve_to's set-up - transform, clip flags, a curve entirely on one side of the
+// clip box, the split into monotonic pieces - and writes the pieces. edge_pieces_kernel flattens the clipped
+// pieces lane-scheduled; edge_tree_kernel then flattens what no clip touches. A piece is built by its own
+// builder: the border runs a curve accumulates are vertical lines at the clip box's x0/x1 whose cells add
+// up the same whether the runs of consecutive pieces are merged or not.
+//
+// In curve_split_kernel a warp takes up to 32 curves and its lanes share their work: a lane per curve for
+// the transform, the polynomial and the sorting of its cuts, a lane per (curve, candidate set) for
+// the roots, a lane per piece for the pieces, whatever curve they belong to. A thread per curve ran the
+// piece loop as often as the warp's most divided curve asks (8 times for 3.4 pieces on average), and in a
+// small frame went through all of it alone. Frames with few curves give each warp fewer. Bound: the FP64
+// pipe. 512 canvases of the batch 2.13 -> 1.77 ms, 20,000 curve paths 0.22 -> 0.19, a 64x64 icon 0.048 ->
+// 0.016 (4, 5, 6 and 8 blocks an SM measured alike).
+constexpr int kSplitWarps = 4;
+
 template<int DEG>
-__device__ void split_curves(FrameView& f, uint32_t block, uint32_t blocks) {
+struct SplitShared {
+  static constexpr int kCands = DEG == 3 ? eb::kCubicCands : 2;
+  double pt[2 * (DEG + 1)][32];      // the curves' points
+  double poly[2 * DEG][32];          // their polynomials without the constant term (the first point)
+  double t[kCands][32];              // their candidates, then their cuts in order
+  uint32_t end[32];                  // pieces of the curves up to and with this one
+  uint32_t cuts[32];
+  uint32_t cmd[32];
+  uint32_t any[32];
+};
+
+// One vertical run at a side of the clip box per lane that has one (Builder::emit_left / emit_right of a
+// builder that accumulated y0 to y1): segment, bounds, binning bound.
+__device__ __forceinline__ void emit_runs(FrameView& f, bool has, int x, double y0, double y1, uint32_t cmd, int lane, uint32_t& rows) {
+  const int a = has ? eb::trunc_i(y0) : 0, b = has ? eb::trunc_i(y1) : 0;
+  has = a != b;
+  const uint32_t set = __ballot_sync(0xFFFFFFFFu, has);
+  if (!set) return;
+  uint32_t base = 0;
+  if (lane == __ffs(set) - 1) base = atomicAdd(f.totals + 0, uint32_t(__popc(set)));
+  base = __shfl_sync(0xFFFFFFFFu, base, __ffs(set) - 1) + uint32_t(__popc(set & ((1u << lane) - 1u)));
+  if (!has) return;
+  const int ya = min(a, b), yb = max(a, b);
+  if (base < f.seg_capacity) {
+    f.segs[base] = DevSeg{x, ya, x, yb};
+    f.seg_meta[base] = (cmd << 1) | uint32_t(a > b);
+  }
+  const uint32_t strips = (uint32_t((yb - 1) >> 8) >> kStripShift) - (uint32_t(ya >> 8) >> kStripShift) + 1u;
+  rows += uint32_t(((((x + 256) >> 8) + 1) >> kTileShift) - (((x - 256) >> 8) >> kTileShift) + 1) + 3u * strips;
+  int4* bb = f.cmd_bbox + cmd;
+  atomicMin(&bb->x, x);
+  atomicMin(&bb->y, ya);
+  atomicMax(&bb->z, x);
+  atomicMax(&bb->w, yb);
+  atomicOr(&f.cmds_rw[cmd].status, kCmdHasSegments);
+}
+
+template<int DEG>
+__device__ __forceinline__ eb::Poly<DEG> shared_poly(const SplitShared<DEG>& sh, int j) {
+  auto term = [&](int i) { return eb::Pt{sh.poly[2 * i][j], sh.poly[2 * i + 1][j]}; };
+  const eb::Pt c0{sh.pt[0][j], sh.pt[1][j]};
+  if constexpr (DEG == 3) return eb::Poly<3>{term(0), term(1), term(2), c0};
+  else return eb::Poly<2>{term(0), term(1), c0};
+}
+
+template<int DEG>
+__device__ void split_curves(FrameView& f, SplitShared<DEG>& sh, uint32_t block, uint32_t blocks) {
   using W = CurveWords<DEG>;
+  constexpr int kCands = SplitShared<DEG>::kCands;
   const int lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
   const uint32_t n_cubic = min(f.work_counter[CurveWords<3>::kCurves], f.item_capacity);
   const uint32_t n_items = DEG == 3 ? n_cubic : min(f.work_counter[CurveWords<2>::kCurves], f.item_capacity - n_cubic);
+  const uint32_t warps = blocks * kSplitWarps;
+  const uint32_t share = min(32u, (n_items + warps - 1u) / warps);      // curves a warp takes at a time
   uint32_t* const list = f.piece_list + (DEG == 3 ? 0u : f.piece_capacity);
   uint32_t rows = 0;
-  for (uint32_t t = block * blockDim.x + threadIdx.x; t - uint32_t(lane) < n_items; t += blocks * blockDim.x) {
-    uint32_t keep = 0, safe = 0, cmd_i = 0;       // bit k: piece k goes on; flattens as by the safe loop
-    eb::Pt spline[DEG == 3 ? 25 : 7];
-    uint32_t any = 0;
-    if (t < n_items) {
-      const DevItem it = f.curve_items[DEG == 3 ? t : f.item_capacity - 1u - t];
+  for (uint32_t first = (block * kSplitWarps + (threadIdx.x >> 5)) * share; first < n_items; first += warps * share) {
+    const int count = int(min(share, n_items - first));
+    // a lane per curve: transform and clip flags (LaneCurve::prepare's set-up)
+    uint32_t pieces = 0, cmd_i = 0;
+    double run0 = 0.0, run1 = 0.0;
+    int run_x = 0;
+    bool run = false;
+    if (lane < count) {
+      const DevItem it = f.curve_items[DEG == 3 ? first + uint32_t(lane) : f.item_capacity - 1u - (first + uint32_t(lane))];
       const DevCmd& cmd = f.cmds[it.cmd];
       const DevXform& xf = f.xforms[cmd.xform];
       eb::Builder b;
       init_builder(b, f.canvases[cmd.canvas]);
-      b.sink.init(f.segs, f.seg_meta, f.totals + 0, f.seg_capacity, it.cmd);
       eb::Src src;
       src.xy = f.verts + 2ull * cmd.geom_first;
       src.affine = xf.affine != 0;
       src.m00 = xf.m[0]; src.m01 = xf.m[1]; src.m10 = xf.m[2]; src.m11 = xf.m[3]; src.m20 = xf.m[4]; src.m21 = xf.m[5];
-      const eb::Pt p0 = src.tf(int(it.a));
-      spline[1] = src.tf(int(it.b));
-      if (DEG == 3) { spline[2] = src.tf(int(it.b) + 1); spline[DEG] = src.tf(int(it.b) + 2); }
-      else spline[DEG] = src.tf(int(it.b) + (it.kind == kItemConic ? 2 : 1));
+      eb::Pt pts[DEG + 1];
+      pts[0] = src.tf(int(it.a));
+      pts[1] = src.tf(int(it.b));
+      if (DEG == 3) pts[2] = src.tf(int(it.b) + 1);
+      pts[DEG] = src.tf(int(it.b) + (DEG == 3 || it.kind == kItemConic ? 2 : 1));
       cmd_i = it.cmd;
-      // curve_to's set-up (LaneCurve::prepare, restated on this thread's own spline)
-      const uint32_t p0_flags = b.fxy(p0);
-      uint32_t common = p0_flags;
-      any = p0_flags;
+      uint32_t common = 15u, any = 0;
 #pragma unroll
-      for (int i = 1; i <= DEG; i++) { const uint32_t fl = b.fxy(spline[i]); common &= fl; any |= fl; }
+      for (int i = 0; i <= DEG; i++) {
+        const uint32_t fl = b.fxy(pts[i]);
+        common &= fl;
+        any |= fl;
+        sh.pt[2 * i][lane] = pts[i].x;
+        sh.pt[2 * i + 1][lane] = pts[i].y;
+      }
+      sh.cmd[lane] = cmd_i;
+      sh.any[lane] = any;
       if (common) {
         if (!(common & (eb::CF_Y0 | eb::CF_Y1))) {
-          const double y0 = eb::dclamp(p0.y, b.cy0, b.cy1), y1 = eb::dclamp(spline[DEG].y, b.cy0, b.cy1);
-          if (common & eb::CF_X0) b.acc_left(y0, y1); else b.acc_right(y0, y1);
+          run = true;
+          run_x = (common & eb::CF_X0) ? b.icx0 : b.icx1;
+          run0 = eb::dclamp(pts[0].y, b.cy0, b.cy1);
+          run1 = eb::dclamp(pts[DEG].y, b.cy0, b.cy1);
         }
-        finish_curve(f, b, it.cmd, rows);
       }
       else {
-        spline[0] = p0;
-        int nout = DEG == 3 ? eb::split_cubic(spline) : eb::split_quad(spline);
-        if (nout == 0) nout = DEG;
-        bool runs = false;
-        for (int k = 0; k < nout / DEG; k++) {
-          if (any) {
-            // pieces outside the clip box end here, with at most a run at its side
-            double y0, y1;
-            uint32_t sign;
-            const eb::PieceOutside where = eb::piece_outside(spline + k * DEG, DEG, b, y0, y1, sign);
-            if (where == eb::kLeftRun) b.acc_left_s(y0, y1, sign);
-            else if (where == eb::kRightRun) b.acc_right_s(y0, y1, sign);
-            runs |= where >= eb::kLeftRun;
-            if (where != eb::kCrosses) continue;
-          }
-          keep |= 1u << k;
-          if (eb::piece_flattens_safe(spline + k * DEG, DEG, any, b)) safe |= 1u << k;
+        pieces = 1;
+        eb::Pt terms[DEG];
+        if constexpr (DEG == 3) {
+          const eb::Poly<3> p = eb::curve_poly(pts[0], pts[1], pts[2], pts[3]);
+          terms[0] = p.a; terms[1] = p.b; terms[2] = p.c;
         }
-        if (runs) finish_curve(f, b, it.cmd, rows);
+        else {
+          const eb::Poly<2> p = eb::curve_poly(pts[0], pts[1], pts[2]);
+          terms[0] = p.a; terms[1] = p.b;
+        }
+#pragma unroll
+        for (int i = 0; i < DEG; i++) { sh.poly[2 * i][lane] = terms[i].x; sh.poly[2 * i + 1][lane] = terms[i].y; }
       }
     }
-    const uint32_t npieces = uint32_t(__popc(keep));
-    // one atomic per warp for the pieces of its curves
-    uint32_t incl = npieces;
+    emit_runs(f, run, run_x, run0, run1, cmd_i, lane, rows);
+    const uint32_t live = __ballot_sync(0xFFFFFFFFu, pieces != 0u);
+    if (!live) continue;
+    __syncwarp();
+    // a lane per (curve, candidate set)
+    constexpr int kSets = DEG == 3 ? eb::kCubicSets : 2;
+    for (int task = lane; task < kSets * count; task += 32) {
+      const int set = task / count, j = task - set * count;
+      if (!((live >> j) & 1u)) continue;
+      if constexpr (DEG == 3) {
+        double c[2];
+        eb::cubic_candidates(shared_poly<3>(sh, j), set, c);
+        if (set == 0) sh.t[0][j] = c[0];
+        else { sh.t[2 * set - 1][j] = c[0]; sh.t[2 * set][j] = c[1]; }
+      }
+      else {
+        const double a = sh.pt[set][j], b = sh.pt[2 + set][j], c = sh.pt[4 + set][j];
+        sh.t[set][j] = (a - b) / (a - b * 2.0 + c);
+      }
+    }
+    __syncwarp();
+    // a lane per curve: its cuts in order, each once
+    if (pieces) {
+      uint32_t n = 0;
+      if constexpr (DEG == 3) {
+        // positive doubles order like their bits
+        unsigned long long v[kCands];
+#pragma unroll
+        for (int k = 0; k < kCands; k++) v[k] = (unsigned long long)__double_as_longlong(sh.t[k][lane]);
+#pragma unroll
+        for (int i = 1; i < kCands; i++) {
+#pragma unroll
+          for (int k = i; k > 0; k--) {
+            const unsigned long long lo = min(v[k - 1], v[k]), hi = max(v[k - 1], v[k]);
+            v[k - 1] = lo;
+            v[k] = hi;
+          }
+        }
+        const unsigned long long none = (unsigned long long)__double_as_longlong(eb::kNoCut);
+        unsigned long long last = 0;
+#pragma unroll
+        for (int k = 0; k < kCands; k++) {
+          if (v[k] != none && v[k] != last) { sh.t[n][lane] = __longlong_as_double((long long)v[k]); n++; }
+          last = v[k];
+        }
+      }
+      else {
+        const double ex = sh.t[0][lane], ey = sh.t[1][lane];
+        const double t0 = eb::dmin(ex, ey), t1 = eb::dmax(ex, ey);
+        if ((t0 > 0.0) & (t0 < 1.0)) sh.t[n++][lane] = t0;
+        if ((t1 > eb::dmax(t0, 0.0)) & (t1 < 1.0)) sh.t[n++][lane] = t1;
+      }
+      sh.cuts[lane] = n;
+      pieces = n + 1u;
+    }
+    uint32_t end = pieces;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= o) incl += v;
+      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, end, o);
+      if (lane >= o) end += v;
     }
-    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    uint32_t base = 0;
-    if (lane == 31 && total) base = atomicAdd(f.work_counter + W::kPieces, total);
-    base = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - npieces;
-    uint32_t idx = base;
-    for (uint32_t todo = keep; todo; todo &= todo - 1u, idx++) {
-      const int k = __ffs(todo) - 1;
-      if (idx >= f.piece_capacity) { atomicOr(f.error_flags, kErrPieces); break; }
-      DevPiece pc;
+    sh.end[lane] = end;
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, end, 31);
+    __syncwarp();
+    // a lane per piece; its first point is the last one of the piece before it, on the lane below or
+    // of the last lane's piece of the step before
+    eb::Pt carry{0.0, 0.0};
+    for (uint32_t at0 = 0; at0 < total; at0 += 32) {
+      const uint32_t at = at0 + uint32_t(lane);
+      const bool on = at < total;
+      int j = 0;
+      if (on) {
 #pragma unroll
-      for (int i = 0; i <= DEG; i++) pc.p[i] = make_double2(spline[k * DEG + i].x, spline[k * DEG + i].y);
-      pc.cmd = cmd_i;
-      pc.any = any;
-      pc.node = 0u;
-      f.pieces[DEG == 3 ? idx : f.piece_capacity - 1u - idx] = pc;
-    }
-    {
-      // pieces the safe loop flattens listed from the front of the kind's list, the others from its
-      // back (one atomic per warp for each), in the pieces' order
-      const uint32_t n_safe = uint32_t(__popc(safe)), n_clip = npieces - n_safe;
-      uint32_t is = n_safe, ic = n_clip;
+        for (int step = 16; step; step >>= 1)
+          if (sh.end[j + step - 1] <= at) j += step;
+      }
+      eb::Pt out[DEG + 1];
+      bool keep = false, safe = false;
+      run = false;
+      cmd_i = sh.cmd[j];
+      const uint32_t any = sh.any[j];
+      const uint32_t n = on ? sh.cuts[j] : 0u, k = on ? at - (j ? sh.end[j - 1] : 0u) : 0u;
+      const eb::Poly<DEG> p = shared_poly<DEG>(sh, j);
+      const double t1 = k < n ? sh.t[k][j] : 1.0;
+      eb::Pt to{sh.pt[2 * DEG][j], sh.pt[2 * DEG + 1][j]};
+      if (k < n) to = eb::poly_point(p, t1);
+      eb::Pt from{__shfl_up_sync(0xFFFFFFFFu, to.x, 1), __shfl_up_sync(0xFFFFFFFFu, to.y, 1)};
+      if (lane == 0) from = carry;
+      carry = eb::Pt{__shfl_sync(0xFFFFFFFFu, to.x, 31), __shfl_sync(0xFFFFFFFFu, to.y, 31)};
+      if (k == 0) from = eb::Pt{sh.pt[0][j], sh.pt[1][j]};
+      if (on) {
+        if (n == 0) {
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t vs = __shfl_up_sync(0xFFFFFFFFu, is, o), vc = __shfl_up_sync(0xFFFFFFFFu, ic, o);
-        if (lane >= o) { is += vs; ic += vc; }
+          for (int i = 0; i <= DEG; i++) out[i] = eb::Pt{sh.pt[2 * i][j], sh.pt[2 * i + 1][j]};
+        }
+        else {
+          eb::poly_piece(p, k ? sh.t[k - 1][j] : 0.0, t1, from, to, out);
+        }
+        eb::Builder b;
+        init_builder(b, f.canvases[f.cmds[cmd_i].canvas]);
+        keep = true;
+        if (any) {
+          // pieces outside the clip box end here, with at most a run at its side
+          uint32_t sign;
+          const eb::PieceOutside where = eb::piece_outside(out, DEG, b, run0, run1, sign);
+          keep = where == eb::kCrosses;
+          run = where >= eb::kLeftRun;
+          run_x = where == eb::kLeftRun ? b.icx0 : b.icx1;
+          if (sign) { const double t = run0; run0 = run1; run1 = t; }
+        }
+        safe = keep && eb::piece_flattens_safe(out, DEG, any, b);
       }
-      const uint32_t ts = __shfl_sync(0xFFFFFFFFu, is, 31), tc = __shfl_sync(0xFFFFFFFFu, ic, 31);
-      uint32_t bs = 0, bc = 0;
-      if (lane == 31) {
-        if (ts) bs = atomicAdd(f.work_counter + W::kSafe, ts);
-        if (tc) bc = atomicAdd(f.work_counter + W::kClip, tc);
-      }
-      bs = __shfl_sync(0xFFFFFFFFu, bs, 31) + is - n_safe;
-      bc = __shfl_sync(0xFFFFFFFFu, bc, 31) + ic - n_clip;
-      uint32_t ks = 0, kc = 0;
-      idx = base;
-      for (uint32_t todo = keep; todo; todo &= todo - 1u, idx++) {
-        if (idx >= f.piece_capacity) break;
-        const uint32_t at = DEG == 3 ? idx : f.piece_capacity - 1u - idx;
-        if ((safe >> (__ffs(todo) - 1)) & 1u) list[bs + ks++] = at;
-        else list[f.piece_capacity - 1u - (bc + kc++)] = at;
+      emit_runs(f, run, run_x, run0, run1, cmd_i, lane, rows);
+      // one atomic per step for the pieces, the safe ones (listed from the front of the kind's list) and
+      // the others (from its back)
+      const uint32_t kept = __ballot_sync(0xFFFFFFFFu, keep), safes = __ballot_sync(0xFFFFFFFFu, safe);
+      const uint32_t clips = kept & ~safes;
+      if (!kept) continue;
+      uint32_t place = 0;
+      if (lane == 0) place = atomicAdd(f.work_counter + W::kPieces, uint32_t(__popc(kept)));
+      if (lane == 1 && safes) place = atomicAdd(f.work_counter + W::kSafe, uint32_t(__popc(safes)));
+      if (lane == 2 && clips) place = atomicAdd(f.work_counter + W::kClip, uint32_t(__popc(clips)));
+      const uint32_t base = __shfl_sync(0xFFFFFFFFu, place, 0), bs = __shfl_sync(0xFFFFFFFFu, place, 1),
+                     bc = __shfl_sync(0xFFFFFFFFu, place, 2);
+      if (keep) {
+        const uint32_t idx = base + uint32_t(__popc(kept & lt));
+        if (idx >= f.piece_capacity) {
+          atomicOr(f.error_flags, kErrPieces);
+        }
+        else {
+          DevPiece pc;
+#pragma unroll
+          for (int i = 0; i <= DEG; i++) pc.p[i] = make_double2(out[i].x, out[i].y);
+          pc.cmd = cmd_i;
+          pc.any = any;
+          pc.node = 0u;
+          const uint32_t to = DEG == 3 ? idx : f.piece_capacity - 1u - idx;
+          f.pieces[to] = pc;
+          if (safe) list[bs + uint32_t(__popc(safes & lt))] = to;
+          else list[f.piece_capacity - 1u - (bc + uint32_t(__popc(clips & lt)))] = to;
+        }
       }
     }
+    __syncwarp();
   }
   rows = __reduce_add_sync(0xFFFFFFFFu, rows);
   if (lane == 0 && rows) atomicAdd(f.totals + 1, rows);
 }
 
-__global__ void __launch_bounds__(128) curve_split_kernel(FrameView f) {
+__global__ void __launch_bounds__(32 * kSplitWarps, kSplitBlocksPerSM) curve_split_kernel(FrameView f) {
+  __shared__ SplitShared<3> shared[kSplitWarps];
   const uint32_t half = gridDim.x / 2u;
-  if (blockIdx.x >= half) split_curves<2>(f, blockIdx.x - half, half);
-  else split_curves<3>(f, blockIdx.x, half);
+  const int w = threadIdx.x >> 5;
+  if (blockIdx.x >= half) split_curves<2>(f, reinterpret_cast<SplitShared<2>&>(shared[w]), blockIdx.x - half, half);
+  else split_curves<3>(f, shared[w], blockIdx.x, half);
 }
 
 // The clipped pieces: the clipping state machine, one step of a lane's piece per iteration of a
@@ -2444,8 +2598,8 @@ int launch_edges(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st) {
   classify_kernel<<<cdiv(f.num_cmds, kClassifyWarps * per_warp), 32 * kClassifyWarps, 0, st>>>(f, per_warp);
   edge_items_kernel<<<cdiv(f.item_capacity ? f.item_capacity : 1, eb), eb, 0, st>>>(f);
   // every curve kernel has twice the blocks of one kind of curve (the first half cubic, the second quadratic)
-  const uint32_t split_grid = min(cdiv(f.item_capacity ? f.item_capacity : 1, 128), uint32_t(sms) * kSplitBlocksPerSM);
-  curve_split_kernel<<<2 * split_grid, 128, 0, st>>>(f);
+  const uint32_t split_grid = min(cdiv(f.item_capacity ? f.item_capacity : 1, kSplitWarps * 4), uint32_t(sms) * kSplitBlocksPerSM);
+  curve_split_kernel<<<2 * split_grid, 32 * kSplitWarps, 0, st>>>(f);
   // as many warps as there may be pieces, up to the grids' limits
   const uint32_t pgrid = cdiv(f.piece_capacity ? f.piece_capacity : 1, kCurveThreads / 32);
   edge_pieces_kernel<<<2 * min(pgrid, uint32_t(sms * max_per_sm)), kCurveThreads, 0, st>>>(
