@@ -565,7 +565,7 @@ __device__ __forceinline__ void finish_curve(FrameView& f, eb::Builder& b, uint3
 // the batched workload (piece kernel 10.8 -> 14.2 ms): the shared-memory carve-out shrinks the L1
 // that the stacks' and the segment sinks' local memory hits in.
 constexpr int kCurveThreads = 128;
-constexpr uint32_t kSplitBlocksPerSM = 6;      // of each kind of curve
+constexpr uint32_t kSplitBlocksPerSM = 8;      // of each kind of curve
 // Idle lanes a warp waits for before it takes new pieces: each refill's set-up costs the warp its
 // FP64 instructions whatever the number of lanes refilled. On the batched workload 24 and 28
 // measured 246-248 ms per step, 16 and 20 250 ms, 32 251 ms, 8 257 ms and 4 259 ms.
