@@ -1671,43 +1671,77 @@ __global__ void __launch_bounds__(32 * kLayoutWarps) backdrop_prefix_kernel(Fram
 
 // Then the slots with segments that no later command covers (cull_kernel) get their mask index, the
 // mask's record and its first work item, in place of the segment count; the others get none. A warp
-// takes 128 slots and a block its masks and work items from one 64-bit counter with one atomic, so masks
-// and items come in the same order and need no scan over the frame. Bound: the counts' bytes and the
-// command look-up. Both passes in place of one warp per command for the prefix, two frame-wide scans and
-// a flag and a compaction pass over the slots: 2.4 -> 0.51 ms for the 46 M slots of 20,000
+// takes 128 slots, packs those with segments together (in large shapes one in 50 has any) and looks up
+// the places of 32 of them at a time; a block takes its masks and work items from one 64-bit counter with
+// one atomic, so masks and items come in the same order and need no scan over the frame. Bound: the
+// latency of the look-ups. Both passes in place of one warp per command for the prefix, two frame-wide
+// scans and a flag and a compaction pass over the slots: 2.4 -> 0.46 ms for the 46 M slots of 20,000
 // pattern quads on 4096x4096, 0.36 -> 0.03 ms for large shapes on 1023x767, and 8 to 12 launches fewer.
+// Unpacked, with the look-ups of every 32 slots that have one with segments: 0.225 ms of the former, now
+// 0.175; 256 and 512 slots a warp slowed small frames (unpacked: 32 canvases 26 -> 39 and 64 us for both passes).
 __global__ void __launch_bounds__(32 * kLayoutWarps) slot_compact_kernel(FrameView f) {
   if (frame_skipped(f)) return;
   constexpr int kSteps = int(kLayoutSlots) / 32;
   __shared__ uint32_t masks_of[kLayoutWarps], items_of[kLayoutWarps];
+  __shared__ uint2 live_all[kLayoutWarps][kLayoutSlots];      // the warp's slots with segments and their counts
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
   const uint32_t n = frame_slots(f), num_cmds = f.counts[kCntCmds];
   const uint64_t x0 = (uint64_t(blockIdx.x) * kLayoutWarps + uint32_t(w)) * kLayoutSlots;
   if (x0 - uint64_t(w) * kLayoutSlots >= n) return;   // whole blocks leave together
-  uint32_t count[kSteps], mine[kSteps], my_masks = 0, my_items = 0;
+  uint2* live = live_all[w];
+  uint32_t num_live = 0;
+  {
+    uint32_t v[kSteps];
 #pragma unroll
-  for (int k = 0; k < kSteps; k++) {
-    const uint64_t s = x0 + uint64_t(32 * k + lane);
-    count[k] = s < n ? f.slot_mask[s] : 0u;
-    my_items |= count[k];
+    for (int k = 0; k < kSteps; k++) {
+      const uint64_t s = x0 + uint64_t(32 * k + lane);
+      v[k] = s < n ? f.slot_mask[s] : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < kSteps; k++) {
+      const uint32_t some = __ballot_sync(0xFFFFFFFFu, v[k] != 0u);
+      if (v[k]) live[num_live + uint32_t(__popc(some & lt))] = make_uint2(uint32_t(x0) + 32u * uint32_t(k) + uint32_t(lane), v[k]);
+      num_live += uint32_t(__popc(some));
+    }
   }
-  if (!__syncthreads_or(int(my_items != 0u))) return;         // no slot of the block has segments
-  uint32_t c = __any_sync(0xFFFFFFFFu, my_items != 0u) ? slot_command(f, uint32_t(x0), num_cmds, lane) : 0u;
-  my_items = 0;
+  if (!__syncthreads_or(int(num_live != 0u))) return;         // no slot of the block has segments
+  // the slots' commands are mostly all among the 32 after the first slot's: one load for all of them
+  const uint32_t c = num_live ? slot_command(f, uint32_t(x0), num_cmds, lane) : 0u;
+  const uint32_t next = num_live && c + 1u + uint32_t(lane) < num_cmds ? f.cmdrow_base[c + 1u + uint32_t(lane)] : 0xFFFFFFFFu;
+  const bool near = uint64_t(__shfl_sync(0xFFFFFFFFu, next, 31)) >= x0 + kLayoutSlots;
+  uint32_t slot[kSteps], count[kSteps], mine[kSteps], place[kSteps], my_masks = 0, my_items = 0;
 #pragma unroll
   for (int k = 0; k < kSteps; k++) {
-    mine[k] = 0;
-    if (!__any_sync(0xFFFFFFFFu, count[k] != 0u)) continue;
-    const uint32_t it = uint32_t(x0) + 32u * uint32_t(k);
-    mine[k] = slot_commands(f, c, it, n, num_cmds, lane);
-    if (count[k]) {
-      const uint32_t ctx = f.cmd_tile_x[mine[k]], tx0 = ctx & 0xFFFFu, ntx = (ctx >> 16) - tx0 + 1u;
-      const uint32_t local = it + uint32_t(lane) - f.cmdrow_base[mine[k]], row = local / ntx;
-      const uint32_t sr = ((f.cmd_yr[mine[k]] & 0xFFFFu) >> kStripShift) + row;
-      const DevCanvas& cv = f.canvases[f.cmds[mine[k]].canvas];
-      const uint32_t tile = cv.tile_base + (sr >> (kTileShift - kStripShift)) * uint32_t(cv.tiles_x) + tx0 + local - row * ntx;
-      if (mine[k] < f.strip_cmd[tile * kStripsPerTile + (sr & (kStripsPerTile - 1u))]) {
-        f.slot_mask[it + uint32_t(lane)] = 0u;
+    slot[k] = count[k] = mine[k] = place[k] = 0u;
+    if (uint32_t(32 * k) >= num_live) continue;
+    const bool on = uint32_t(32 * k + lane) < num_live;
+    if (on) { slot[k] = live[32 * k + lane].x; count[k] = live[32 * k + lane].y; }
+    uint32_t m = c;
+    if (near) {
+      uint32_t pos = 0;
+#pragma unroll
+      for (int step = 16; step; step >>= 1)
+        if (__shfl_sync(0xFFFFFFFFu, next, int(pos) + step - 1) <= slot[k]) pos += uint32_t(step);
+      m += pos;
+    }
+    else {
+      for (uint32_t hi = num_cmds; hi - m > 1u;) {            // first slots: m's at or before the slot, hi's after it
+        const uint32_t mid = m + (hi - m) / 2u;
+        if (f.cmdrow_base[mid] <= slot[k]) m = mid;
+        else hi = mid;
+      }
+    }
+    if (on) {
+      const uint32_t ctx = f.cmd_tile_x[m], tx0 = ctx & 0xFFFFu, ntx = (ctx >> 16) - tx0 + 1u;
+      const uint32_t local = slot[k] - f.cmdrow_base[m], row = local / ntx;
+      const uint32_t tx = tx0 + local - row * ntx, sr = ((f.cmd_yr[m] & 0xFFFFu) >> kStripShift) + row;
+      const DevCanvas& cv = f.canvases[f.cmds[m].canvas];
+      const uint32_t tile = cv.tile_base + (sr >> (kTileShift - kStripShift)) * uint32_t(cv.tiles_x) + tx;
+      mine[k] = m;
+      place[k] = tx | (sr << 16);
+      if (m < f.strip_cmd[tile * kStripsPerTile + (sr & (kStripsPerTile - 1u))]) {
+        f.slot_mask[slot[k]] = 0u;
         count[k] = 0u;
       }
     }
@@ -1744,21 +1778,17 @@ __global__ void __launch_bounds__(32 * kLayoutWarps) slot_compact_kernel(FrameVi
       if (lane >= o) incl += t;
     }
     if (count[k]) {
-      const uint32_t s = uint32_t(x0) + 32u * uint32_t(k) + uint32_t(lane), m = mine[k];
-      const uint32_t idx = mask_at + uint32_t(__popc(some & ((1u << lane) - 1u)));
-      f.slot_mask[s] = idx + 1u;
+      const uint32_t idx = mask_at + uint32_t(__popc(some & lt));
+      f.slot_mask[slot[k]] = idx + 1u;
       if (idx < f.mask_capacity) {
-        const uint32_t ctx = f.cmd_tile_x[m], tx0 = ctx & 0xFFFFu, ntx = (ctx >> 16) - tx0 + 1u;
-        const uint32_t local = s - f.cmdrow_base[m], row = local / ntx;
-        const uint32_t x = (tx0 + local - row * ntx) << kTileShift;
-        const uint32_t y = (((f.cmd_yr[m] & 0xFFFFu) >> kStripShift) + row) << kStripShift;
-        const DevCmd& cmd = f.cmds[m];
+        const uint32_t x = (place[k] & 0xFFFFu) << kTileShift, y = (place[k] >> 16) << kStripShift;
+        const DevCmd& cmd = f.cmds[mine[k]];
         const DevCanvas& cv = f.canvases[cmd.canvas];
         f.mask_cursor[idx] = item_at + incl - count[k];
         // what the coverage pass needs of the slot
         f.mask_info[idx] = make_uint4((x + min(uint32_t(cv.w) - x, uint32_t(kTileW)) - 1u) |
                                           ((y + min(uint32_t(cv.h) - y, uint32_t(kStripRows)) - 1u) << 16),
-                                      m, (cmd.flags << 16) | cmd.alpha, s);
+                                      mine[k], (cmd.flags << 16) | cmd.alpha, slot[k]);
       }
     }
     mask_at += uint32_t(__popc(some));
