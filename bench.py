@@ -297,7 +297,7 @@ def roofline(st_culled, st_ref, fine_ms: float, comp_ms: float, traffic_name: st
     peak, kind = hbm_peak()
     achieved = alg / (fine_ms / 1e3) / 1e9
     traffic, src = ncu_traffic(traffic_name)
-    return {"bound": "hbm", "kernel": "fine stage (coverage: coverage_kernel; composite: cull_kernel + fine_kernel)",
+    return {"bound": "hbm", "kernel": "fine stage (coverage: backdrop_prefix_kernel + cull_kernel + slot_compact_kernel + seg_bin_kernel + coverage_kernel; composite: fine_kernel)",
             "achieved": round(achieved, 2), "peak": peak, "peak_kind": f"of {kind}", "unit": "GB/s",
             "frac": round(achieved / peak, 4), "traffic": traffic, "traffic_source": src,
             "algorithmic_bytes_per_launch": alg, "fine_ms": round(fine_ms, 4), "composite_kernel_ms": round(comp_ms, 4),

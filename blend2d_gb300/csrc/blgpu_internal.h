@@ -5,13 +5,13 @@
 // formulas), input geometry in double precision, transforms, gradient LUT requests and pattern
 // images. The device pipeline turns it into pixels:
 //
-//   K0 lut_build    - gradient LUTs (one thread per entry, reference builder semantics)
-//   K1 edge_build   - FP64 edge building per analytic command (count pass + emit pass) producing
-//                     24.8 fixed-point segments, exactly the reference's EdgeBuilder output
-//   K2 binning      - per command tile ranges, per (command, tile row) segment lists, per tile row
+//   K0 lut          - gradient LUTs (one warp per table, reference builder semantics)
+//   K1 edge build   - FP64 edge building per line, curve and monotonic piece, producing 24.8
+//                     fixed-point segments, exactly the reference's EdgeBuilder output
+//   K2 binning      - per command tile ranges, segments per (command, strip row, tile column) slot,
 //                     command lists in painter's order
-//   K3 fine         - persistent tile kernel: tile pixels stay in registers while every command
-//                     touching the tile is rasterized into shared-memory cells, swept and composited
+//   K3 fine         - the slots' masks, rasterized in shared-memory cells, and the persistent
+//                     composite: a strip's pixels stay in registers through all its commands
 //
 // Everything here is POD so a frame can be uploaded with one copy.
 #pragma once
