@@ -1173,6 +1173,7 @@ __global__ void __launch_bounds__(kCurveThreads) edge_tree_kernel(FrameView f) {
   else flatten_trees<3>(f, xchg[w], half);
 }
 
+// Lines, and commands built whole: classify_kernel's item list.
 __global__ void __launch_bounds__(256) edge_items_kernel(FrameView f) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t rows = 0;
@@ -1199,16 +1200,9 @@ __global__ void __launch_bounds__(256) edge_items_kernel(FrameView f) {
       src.n = int(cmd.geom_count);
       rc = eb::build(b, src);                  // includes done()
     }
-    else if (it.kind == kItemLine) {
+    else {
       src.i = src.n = 0;                       // no further lines: line_to builds exactly this one
       rc = eb::line_to(b, src, a, a_flags, src.tf(int(it.b)));
-    }
-    else {
-      // the source ends right after this curve, so curve_to consumes exactly one
-      src.i = int(it.b);
-      src.n = int(it.b) + (it.kind == kItemQuad ? 2 : 3);
-      if (it.kind == kItemCubic) eb::curve_to<3>(b, src, a, a_flags, false);
-      else eb::curve_to<2>(b, src, a, a_flags, it.kind == kItemConic);
     }
     if (rc) {
       atomicOr(&f.cmds_rw[it.cmd].status, kCmdInvalid);
