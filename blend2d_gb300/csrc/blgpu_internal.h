@@ -248,8 +248,7 @@ struct DevStrokeFig {
 
 // Stroked curves (stroke.cu): their offset quads in chunks from a pool, and where a curve's quads go in
 // the outline: side A forward from vertex `a`, side B backward from vertex `b`.
-constexpr uint32_t kStrokeChunk = 4;                  // quads per chunk
-constexpr uint32_t kStrokeQuadBytes = 64, kStrokeRecBytes = 136;   // sk::OffsetQuad, sk::CurveRec
+constexpr uint32_t kStrokeRecBytes = 136;             // sk::CurveRec
 enum StrokeCounter : uint32_t { kStrokeCurves = 0, kStrokeChunks = 1, kStrokeCounters = 2 };
 enum CurveDestFlag : uint32_t {
   kDestSideB = 1u,         // the outline has a side B
@@ -371,7 +370,7 @@ struct FrameView {
   void* stroke_pool;          // chunks of sk::OffsetQuad
   uint32_t* stroke_chunk_next;
   DevCurveDest* stroke_dests;
-  uint32_t stroke_curve_cap, stroke_chunk_cap;
+  uint32_t stroke_curve_cap, stroke_chunk_cap;   // no curves: none is stored
   uint32_t num_stroke_figs;
   uint32_t stroke_vert_base;
   uint32_t num_segs;

@@ -784,7 +784,8 @@ struct BLGpuContext {
     Fill f;
     if (n == 0 || !resolve_fill(f, 1)) return BLGPU_SUCCESS;
     stroke_ranges.clear();
-    BLGpuResult r = stroke_figures(cmds, n, stroke_ranges);
+    uint32_t curves = 0;
+    BLGpuResult r = stroke_figures(cmds, n, stroke_ranges, &curves);
     if (r) return r;
     if (stroke_ranges.empty()) return BLGPU_SUCCESS;
     uint32_t xform;
@@ -811,6 +812,7 @@ struct BLGpuContext {
     c.xform = xform;
     const uint32_t cmd_index = uint32_t(frame->cmds.size() - 1);
     const uint32_t base = uint32_t(frame->stroke_cmds.size());
+    frame->stroke_curves += curves;
     frame->stroke_cmds.append(cmds, n);
     frame->stroke_xy.append(xy, 2 * n);
     DevStrokeParams sp{s.stroke.width, s.stroke.miter_limit, s.stroke.join, s.stroke.start_cap, s.stroke.end_cap, 0u};

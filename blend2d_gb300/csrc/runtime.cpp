@@ -78,7 +78,7 @@ void Frame::clear() {
   cmds.clear(); styles.clear(); xforms.clear(); canvases.clear(); targets.clear();
   verts.clear(); path_cmds.clear(); lut_jobs.clear(); stops.clear(); images.clear();
   stroke_figs.clear(); stroke_params.clear(); stroke_xy.clear(); stroke_cmds.clear();
-  image_words = 0; lut_words = 0; tiles = 0; rows = 0;
+  image_words = 0; lut_words = 0; tiles = 0; rows = 0; stroke_curves = 0;
   vert_parts.clear(); ext_verts = 0;
   generation = next_generation();
 }
@@ -138,7 +138,7 @@ void Frame::merge(Frame* const* parts, size_t count, unsigned threads) {
   struct Base {
     size_t cmd, style, xform, canvas, vert, stop, lut_job, image, fig, param, stroke_vert;
     uint64_t image_words;
-    uint32_t lut_words, tiles, rows;
+    uint32_t lut_words, tiles, rows, stroke_curves;
   };
   std::vector<Base> base(count + 1);
   Base acc{};
@@ -151,6 +151,7 @@ void Frame::merge(Frame* const* parts, size_t count, unsigned threads) {
     acc.lut_job += f.lut_jobs.size(); acc.image += f.images.size(); acc.fig += f.stroke_figs.size();
     acc.param += f.stroke_params.size(); acc.stroke_vert += f.stroke_cmds.size();
     acc.image_words += f.image_words; acc.lut_words += f.lut_words; acc.tiles += f.tiles; acc.rows += f.rows;
+    acc.stroke_curves += f.stroke_curves;
   }
   // vertices recorded in page-locked memory stay where they are (uploaded part by part)
   bool refer_verts = true;
@@ -175,6 +176,7 @@ void Frame::merge(Frame* const* parts, size_t count, unsigned threads) {
   targets.resize(acc.canvas);
   images.resize(acc.image);
   image_words = acc.image_words; lut_words = acc.lut_words; tiles = acc.tiles; rows = acc.rows;
+  stroke_curves = acc.stroke_curves;
 
   auto copy_part = [&](size_t p) {
     const Frame& f = *parts[p];
@@ -383,10 +385,8 @@ BLGpuResult Runtime::prepare_strokes(const Frame& fr, FrameView& v, uint32_t& ou
     for (uint32_t k = 0; k < kBuckets; k++) start[k + 1] += start[k];
     for (uint32_t i = 0; i < nf; i++) stroke_order[start[keys[i]]++] = i;
   }
-  // a curve takes two vertices or more; chunks: what a vertex took at most in the frames so far
-  const uint32_t nv = uint32_t(fr.stroke_cmds.size());
-  v.stroke_curve_cap = nv / 2u;
-  v.stroke_chunk_cap = uint32_t(std::min<double>(double(nv) * stroke_chunks_per_vertex, 4e9));
+  v.stroke_curve_cap = fr.stroke_curves;
+  v.stroke_chunk_cap = stroke_pool.chunks(fr.stroke_curves);
   auto plan = [&](Layout& L) {
     v.stroke_figs = L.take<DevStrokeFig>(nf);
     v.stroke_order = L.take<uint32_t>(nf);
@@ -398,7 +398,7 @@ BLGpuResult Runtime::prepare_strokes(const Frame& fr, FrameView& v, uint32_t& ou
     v.stroke_offsets = L.take<uint32_t>(nf + 1 + kStrokeCounters);
     v.stroke_counters = v.stroke_offsets + nf + 1;               // read back with the outline's size
     v.stroke_scan_tmp = L.take<uint32_t>(scan_temp_words(nf + 1));
-    v.stroke_curve_at = L.take<uint32_t>(nv);
+    v.stroke_curve_at = L.take<uint32_t>(v.stroke_curve_cap ? fr.stroke_cmds.size() : 0);
     v.stroke_curves = L.take<uint2>(v.stroke_curve_cap);
     v.stroke_recs = L.take<char>(size_t(v.stroke_curve_cap) * kStrokeRecBytes);
     v.stroke_dests = L.take<DevCurveDest>(v.stroke_curve_cap);
@@ -411,7 +411,17 @@ BLGpuResult Runtime::prepare_strokes(const Frame& fr, FrameView& v, uint32_t& ou
   if (measure.off > stroke_buf.size) {
     graph_valid = false;
     BLGPU_CHECK(cudaStreamSynchronize(stream));
-    BLGPU_CHECK(stroke_buf.reserve(measure.off));
+    cudaError_t e = stroke_buf.reserve(measure.off);
+    if (e == cudaErrorMemoryAllocation && v.stroke_curve_cap) {
+      // no room for the curves' arrays: the figures' threads offset the curves
+      cudaGetLastError();
+      v.stroke_curve_cap = v.stroke_chunk_cap = 0;
+      measure = Layout{};
+      plan(measure);
+      stroke_bytes = measure.off;
+      e = stroke_buf.reserve(measure.off);
+    }
+    BLGPU_CHECK(e);
   }
   Layout L;
   L.base = static_cast<char*>(stroke_buf.ptr);
@@ -432,9 +442,8 @@ BLGpuResult Runtime::prepare_strokes(const Frame& fr, FrameView& v, uint32_t& ou
   BLGPU_CHECK(cudaMemcpyAsync(host_totals + 16, v.stroke_offsets + nf, kBack, cudaMemcpyDeviceToHost, stream));
   d2h_bytes += kBack;
   BLGPU_CHECK(cudaStreamSynchronize(stream));
-  // a pool that ran out costs time, not the outline: the next frame's is larger
-  const uint32_t chunks = host_totals[16 + 1 + kStrokeChunks];
-  if (chunks > v.stroke_chunk_cap) stroke_chunks_per_vertex = 1.25 * double(chunks) / double(nv);
+  // a pool that ran out costs time, not the outline
+  stroke_pool.after(fr.stroke_curves, v.stroke_chunk_cap, host_totals[16 + 1 + kStrokeChunks]);
   if (host_totals[16] > 0x3FFFFFFFu) return BLGPU_ERROR_DATA_TOO_LARGE;
   outline_verts = host_totals[16];
   strokes_counted = true;
@@ -1402,6 +1411,7 @@ BLGpuResult Runtime::release_memory() {
   dyn_buf.release();
   seg_buf.release();
   stroke_buf.release();
+  stroke_pool = StrokePool{};
   seg_capacity = 0;
   return BLGPU_SUCCESS;
 }

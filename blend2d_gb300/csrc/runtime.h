@@ -13,6 +13,7 @@
 #include "blgpu.h"
 #include "blgpu_internal.h"
 #include "launch.h"
+#include "stroke_pool.h"
 
 namespace blgpu {
 
@@ -120,6 +121,7 @@ struct Frame {
   HostArray<DevStrokeParams> stroke_params;
   HostArray<double> stroke_xy;
   HostArray<uint8_t> stroke_cmds;
+  uint32_t stroke_curves = 0;                // quadratic and cubic commands of the figures
   std::vector<FrameImage> images;
   uint64_t image_words = 0;
   uint32_t lut_words = 0;
@@ -187,7 +189,7 @@ struct Runtime {
   DeviceBuffer seg_buf;     // segments + their metadata, appended by the edge builders
   DeviceBuffer stroke_buf;  // stroke inputs, per-figure outline counts and offsets
   bool strokes_counted = false;   // the upload's sizing pass left this frame's counts in place
-  double stroke_chunks_per_vertex = 2.0;   // size of the offset quads' pool (prepare_strokes)
+  StrokePool stroke_pool;         // size of the offset quads' pool (prepare_strokes)
   std::vector<uint32_t> stroke_order;   // thread -> figure order of the frame being uploaded
   uint32_t seg_capacity = 0;
   void* host_staging = nullptr;

@@ -5,8 +5,9 @@
 
 namespace blgpu {
 
-BLGpuResult stroke_figures(const uint8_t* cmd, size_t n, std::vector<uint32_t>& ranges) {
+BLGpuResult stroke_figures(const uint8_t* cmd, size_t n, std::vector<uint32_t>& ranges, uint32_t* curves) {
   const size_t mark = ranges.size();
+  uint32_t num_curves = 0;
   size_t i = 0;
   while (i < n) {
     if (cmd[i] != sk::kMove) {
@@ -24,6 +25,7 @@ BLGpuResult stroke_figures(const uint8_t* cmd, size_t n, std::vector<uint32_t>& 
       if (c == sk::kQuad || c == sk::kCubic) {
         i += c == sk::kQuad ? 2 : 3;
         if (i > n) { ranges.resize(mark); return BLGPU_ERROR_INVALID_GEOMETRY; }
+        num_curves++;
         continue;
       }
       if (c == sk::kClose) i++;
@@ -34,6 +36,7 @@ BLGpuResult stroke_figures(const uint8_t* cmd, size_t n, std::vector<uint32_t>& 
       ranges.push_back(uint32_t(i));
     }
   }
+  if (curves) *curves += num_curves;
   return BLGPU_SUCCESS;
 }
 

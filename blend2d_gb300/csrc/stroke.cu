@@ -19,6 +19,7 @@
 #include "blgpu_internal.h"
 #include "launch.h"
 #include "stroke_core.h"
+#include "stroke_pool.h"
 
 namespace blgpu {
 
@@ -35,7 +36,7 @@ __device__ __forceinline__ sk::Params stroke_params(const FrameView& f, uint32_t
 
 // The curves of a figure as the stroker's kernels find them, and where emit puts them.
 struct StoredCurves {
-  const uint32_t* at;                // vertex -> its curve's index
+  const uint32_t* at;                // vertex -> its curve's index; null: no curve is stored
   const sk::CurveRec* recs;
   const sk::OffsetQuad* pool;
   DevCurveDest* dests;               // emit only
@@ -44,6 +45,7 @@ struct StoredCurves {
   uint32_t flags;                    // DevCurveDest's, without kDestLast
 
   __device__ const sk::CurveRec* find(uint32_t i, sk::V p0) const {
+    if (!at) return nullptr;
     const sk::CurveRec* r = recs + at[i];
     return r->count && sk::same_bits(r->from, p0) ? r : nullptr;
   }
@@ -113,7 +115,7 @@ __global__ void __launch_bounds__(kStrokeThreads) stroke_curves_kernel(FrameView
         rec.last = o;
         n++;
       });
-      // the pool is used up: the figure's thread offsets this curve (the next frame gets more chunks)
+      // the pool is used up: the figure's thread offsets this curve (StrokePool gives the next frame more)
       if (n && chunk >= f.stroke_chunk_cap) { n = 0; break; }
     }
   }
@@ -125,7 +127,7 @@ __global__ void __launch_bounds__(kStrokeThreads) stroke_curves_kernel(FrameView
 
 __device__ __forceinline__ StoredCurves stored_curves(const FrameView& f) {
   StoredCurves c{};
-  c.at = f.stroke_curve_at;
+  c.at = f.stroke_curve_cap ? f.stroke_curve_at : nullptr;
   c.recs = static_cast<const sk::CurveRec*>(f.stroke_recs);
   c.pool = static_cast<const sk::OffsetQuad*>(f.stroke_pool);
   return c;

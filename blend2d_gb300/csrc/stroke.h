@@ -26,7 +26,8 @@ struct StrokeParams {
 // ranges appended to `ranges` (figures with a move only are left out: they stroke to nothing).
 // Returns BLGPU_ERROR_INVALID_GEOMETRY where the reference's stroke fails (a command other than
 // a move or close between figures, a curve running past the path's end): it then draws nothing.
-BLGpuResult stroke_figures(const uint8_t* cmds, size_t n, std::vector<uint32_t>& ranges);
+// `curves`, where given, grows by the figures' quadratic and cubic commands.
+BLGpuResult stroke_figures(const uint8_t* cmds, size_t n, std::vector<uint32_t>& ranges, uint32_t* curves = nullptr);
 
 // The outline a stroke fills non-zero, on the host with the same stroker: per closed figure its
 // two offset figures, per open figure one loop (see stroke_core.h). Used by
