@@ -1917,7 +1917,7 @@ constexpr int kSlotPixels = kStripRows * kTileW;
 constexpr int kCoverWarps = 4;
 
 template<int kSlots>
-__global__ void __launch_bounds__(32 * kCoverWarps) coverage_kernel(FrameView f) {
+__global__ void __launch_bounds__(32 * kCoverWarps) coverage_kernel(FrameView f, bool occlusion) {
   __shared__ __align__(16) uint32_t cells_all[kCoverWarps][kSlots][kSlotPixels];
   __shared__ __align__(16) uint32_t bd_all[kCoverWarps][kSlots][kStripRows];
   __shared__ uint32_t org_all[kCoverWarps][kSlots];   // the slot's last column and row on the canvas
@@ -1980,7 +1980,7 @@ __global__ void __launch_bounds__(32 * kCoverWarps) coverage_kernel(FrameView f)
       cov += cv4.z; m |= px::calc_mask(cov, rule, alpha) << 16;
       cov += cv4.w; m |= px::calc_mask(cov, rule, alpha) << 24;
       reinterpret_cast<uint32_t*>(f.masks + size_t(m0 + uint32_t(j)) * kSlotPixels)[lane] = m;
-      if ((flags & 1u) && alpha == 255u) {
+      if (occlusion && (flags & 1u) && alpha == 255u) {
         // an opaque SrcCopy command that covers every pixel of the slot on the canvas: none before it
         // shows there (what the occlusion pass could not see without the masks)
         const uint32_t o = org[j];
@@ -2680,10 +2680,11 @@ int launch_coverage(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st
   // lanes. The pass at 16, 32 and 64 slots a block: 5.44, 4.37 and 4.66 ms on 512 canvases of the batch,
   // 0.41, 0.36 and 0.41 on 20,000 curve paths.
   const int slots = cfg.cover_slots ? cfg.cover_slots : 32;
+  const bool occlusion = !cfg.no_occlusion_cull;
   const int grid = int(min(uint32_t(sms * per_sm), cdiv(f.mask_capacity, uint32_t(slots))));
-  if (slots == 16) coverage_kernel<16 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f);
-  else if (slots == 64) coverage_kernel<64 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f);
-  else coverage_kernel<32 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f);
+  if (slots == 16) coverage_kernel<16 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f, occlusion);
+  else if (slots == 64) coverage_kernel<64 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f, occlusion);
+  else coverage_kernel<32 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f, occlusion);
   return k + 1;
 }
 
