@@ -296,8 +296,7 @@ struct FrameView {
   DevItem* items;              // lines and curves of every analytic command (any order)
   DevItem* curve_items;        // cubic curves from the front, quadratic / conic curves from the back
   DevPiece* pieces;            // their monotonic pieces, cubic from the front, quadratic from the back
-  uint32_t* piece_list;        // [2 * piece_capacity] cubic, then quadratic piece indices: those the safe loop
-                               //   flattens from the front of their half, clipped ones from its back
+  uint32_t* piece_list;        // [piece_capacity] indices of the cubic, then of the other pieces (kernels.cu, PieceList)
   uint32_t piece_capacity;
   int4* cmd_bbox;              // [num_cmds] 24.8 bbox of the emitted segments: xmin, ymin, xmax, ymax
   DevSeg* segs;                // emitted segments (any order)
@@ -329,9 +328,11 @@ struct FrameView {
                                //   with meta = kind | flags << 2 | alpha << 4; for a solid style the
                                //   style word has bit 31 set and the colour replaces the row state
   uint32_t* row_copies;        // [num_rows] SrcCopy commands in each tile row's list
-  uint32_t* strip_start;       // [num_tiles * strips per tile] first list entry the composite needs (occlusion)
+  uint32_t* strip_start;       // [num_tiles * strips per tile] first list entry the composite needs (occlusion);
+                               //   null: the first one, and strip_cmd alone says what shows
   uint32_t* strip_cmd;         // the same as a command: no command of the canvas before it shows in the strip
   uint32_t* spilled;           // [num_tiles * strips per tile] strips whose list the composite's tail launch finishes
+                               //   (frames of several canvases)
   uint32_t* tile_order;        // tile processing order for the persistent fine kernel
   uint32_t* tile_canvas;       // canvas index per global tile
   uint32_t* work_counter;      // [0] fine work queue, [1] items, [2] cubics, [21] quads, [23] / [25] cubic / quadratic

@@ -562,6 +562,21 @@ constexpr uint32_t kPieceLeafLanes = 16;
 // 0.016 (4, 5, 6 and 8 blocks an SM measured alike).
 constexpr int kSplitWarps = 4;
 
+// A kind's part of the piece list: the pieces the safe loop flattens from its front, the clipped ones from
+// its back. The cubic curves' part takes the most pieces they can have, 8 a curve of three vertices; of
+// three entries per vertex that leaves two per vertex and more for the quadratic and conic ones, which
+// have at most 3 pieces in two vertices.
+struct PieceList {
+  uint32_t* at;
+  uint32_t n;
+};
+template<int DEG>
+__device__ __forceinline__ PieceList piece_list(const FrameView& f) {
+  const unsigned long long most = (eb::kCubicCands + 1ull) * min(f.work_counter[CurveWords<3>::kCurves], f.item_capacity);
+  const uint32_t cubic = most < f.piece_capacity ? uint32_t(most) : f.piece_capacity;
+  return DEG == 3 ? PieceList{f.piece_list, cubic} : PieceList{f.piece_list + cubic, f.piece_capacity - cubic};
+}
+
 template<int DEG>
 struct SplitShared {
   static constexpr int kCands = DEG == 3 ? eb::kCubicCands : 2;
@@ -618,7 +633,7 @@ __device__ void split_curves(FrameView& f, SplitShared<DEG>& sh, uint32_t block,
   const uint32_t n_items = DEG == 3 ? n_cubic : min(f.work_counter[CurveWords<2>::kCurves], f.item_capacity - n_cubic);
   const uint32_t warps = blocks * kSplitWarps;
   const uint32_t share = min(32u, (n_items + warps - 1u) / warps);      // curves a warp takes at a time
-  uint32_t* const list = f.piece_list + (DEG == 3 ? 0u : f.piece_capacity);
+  const PieceList list = piece_list<DEG>(f);
   uint32_t rows = 0;
   for (uint32_t first = (block * kSplitWarps + (threadIdx.x >> 5)) * share; first < n_items; first += warps * share) {
     const int count = int(min(share, n_items - first));
@@ -803,7 +818,8 @@ __device__ void split_curves(FrameView& f, SplitShared<DEG>& sh, uint32_t block,
                      bc = __shfl_sync(0xFFFFFFFFu, place, 2);
       if (keep) {
         const uint32_t idx = base + uint32_t(__popc(kept & lt));
-        if (idx >= f.piece_capacity) {
+        const uint32_t li = safe ? bs + uint32_t(__popc(safes & lt)) : bc + uint32_t(__popc(clips & lt));
+        if (idx >= f.piece_capacity || li >= list.n) {
           atomicOr(f.error_flags, kErrPieces);
         }
         else {
@@ -815,8 +831,7 @@ __device__ void split_curves(FrameView& f, SplitShared<DEG>& sh, uint32_t block,
           pc.node = 0u;
           const uint32_t to = DEG == 3 ? idx : f.piece_capacity - 1u - idx;
           f.pieces[to] = pc;
-          if (safe) list[bs + uint32_t(__popc(safes & lt))] = to;
-          else list[f.piece_capacity - 1u - (bc + uint32_t(__popc(clips & lt)))] = to;
+          list.at[safe ? li : list.n - 1u - li] = to;
         }
       }
     }
@@ -866,9 +881,9 @@ __device__ void flatten_clipped(FrameView& f, uint32_t blocks) {
   const uint32_t n_cubic = min(f.work_counter[CurveWords<3>::kPieces], f.piece_capacity);
   const uint32_t n_quad = min(f.work_counter[CurveWords<2>::kPieces], f.piece_capacity - n_cubic);
   const uint32_t n_mine = DEG == 3 ? n_cubic : n_quad;
-  const uint32_t n_items = min(f.work_counter[W::kClip], n_mine);
+  const PieceList list = piece_list<DEG>(f);
+  const uint32_t n_items = min(f.work_counter[W::kClip], min(n_mine, list.n));
   const uint32_t room = handed_room(f, n_cubic, n_quad), share = piece_share(n_items, blocks);
-  const uint32_t* const list = f.piece_list + (DEG == 3 ? 0u : f.piece_capacity);
   uint32_t* queue = f.work_counter + W::kClipQueue;
   using Lane = eb::LaneCurve<DEG, eb::CachedStack<DEG>>;
   eb::Builder b;
@@ -903,7 +918,7 @@ __device__ void flatten_clipped(FrameView& f, uint32_t blocks) {
           exhausted = true;
         }
         else {
-          const uint32_t pi = list[f.piece_capacity - 1u - t];
+          const uint32_t pi = list.at[list.n - 1u - t];
           // a list entry is written only for a piece that fit in the piece array; with a frame
           // that overflowed it (reported by curve_split), an entry may be stale: the lane then
           // stays idle and takes another piece
@@ -1011,10 +1026,10 @@ __device__ void flatten_trees(FrameView& f, TreeXchg<DEG>* xchg, uint32_t blocks
   const uint32_t lt = (1u << lane) - 1u;
   const uint32_t n_cubic = min(f.work_counter[CurveWords<3>::kPieces], f.piece_capacity);
   const uint32_t n_quad = min(f.work_counter[CurveWords<2>::kPieces], f.piece_capacity - n_cubic);
-  const uint32_t n_safe = min(f.work_counter[W::kSafe], DEG == 3 ? n_cubic : n_quad);
+  const PieceList list = piece_list<DEG>(f);
+  const uint32_t n_safe = min(f.work_counter[W::kSafe], min(DEG == 3 ? n_cubic : n_quad, list.n));
   const uint32_t n_items = n_safe + min(f.work_counter[W::kHanded], handed_room(f, n_cubic, n_quad));
   const uint32_t share = piece_share(n_items, blocks);
-  const uint32_t* const list = f.piece_list + (DEG == 3 ? 0u : f.piece_capacity);
   uint32_t* queue = f.work_counter + W::kTreeQueue;
   const double tol = 0.20 * 256.0;
   const double tol_sq = tol * tol;                    // init_builder's
@@ -1060,7 +1075,7 @@ __device__ void flatten_trees(FrameView& f, TreeXchg<DEG>* xchg, uint32_t blocks
         }
         else {
           const uint32_t e = t - n_safe;         // a handed-over subtree when t >= n_safe
-          const uint32_t pi = t < n_safe ? list[t] : DEG == 3 ? n_cubic + e : f.piece_capacity - 1u - n_quad - e;
+          const uint32_t pi = t < n_safe ? list.at[t] : DEG == 3 ? n_cubic + e : f.piece_capacity - 1u - n_quad - e;
           // an entry of a piece that did not fit in the piece array (the frame fails) is skipped
           if (t >= n_safe || (DEG == 3 ? pi < n_cubic : pi < f.piece_capacity && pi >= f.piece_capacity - n_quad)) {
             const DevPiece pc = f.pieces[pi];
@@ -2162,7 +2177,7 @@ __global__ void __launch_bounds__(kFineThreads) cull_kernel(FrameView f) {
       }
       if (lane < strips) {
         const uint32_t unit = tile * kStripsPerTile + lr * uint32_t(strips) + uint32_t(lane);
-        f.strip_start[unit] = start;
+        if (f.strip_start) f.strip_start[unit] = start;
         f.strip_cmd[unit] = start_cmd;
       }
     }
@@ -2317,7 +2332,7 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
     const uint32_t strip_y = uint32_t(row0) | (uint32_t(row1) << 16);
     const uint32_t strip_x = uint32_t(x_base) | (uint32_t(min(x_base + kTileW, cv.w) - 1) << 16);
 
-    const uint32_t start = f.strip_start[tile * kStripsPerTile + uint32_t(strip)];      // cull_kernel
+    const uint32_t start = f.strip_start ? f.strip_start[tile * kStripsPerTile + uint32_t(strip)] : 0u;   // cull_kernel
     const uint32_t cover = f.strip_cmd[tile * kStripsPerTile + uint32_t(strip)];        // ... and coverage_kernel
     uint32_t pend_mw = 0, pend[PX] = {};   // the command to composite next
     bool pend_copy = false;
@@ -2663,7 +2678,7 @@ int launch_coverage(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st
     k++;
   }
   if (cfg.no_occlusion_cull) {
-    cudaMemsetAsync(f.strip_start, 0, sizeof(uint32_t) * size_t(f.num_tiles) * kStripsPerTile, st);
+    if (f.strip_start) cudaMemsetAsync(f.strip_start, 0, sizeof(uint32_t) * size_t(f.num_tiles) * kStripsPerTile, st);
     cudaMemsetAsync(f.strip_cmd, 0, sizeof(uint32_t) * size_t(f.num_tiles) * kStripsPerTile, st);
   }
   else if (f.num_tiles) {

@@ -536,7 +536,7 @@ BLGpuResult Runtime::upload_frame(const Frame& fr, const FrameSizes* caps) {
     v.items = L.take<DevItem>(item_capacity);
     v.curve_items = L.take<DevItem>(item_capacity);
     v.pieces = L.take<DevPiece>(piece_capacity);
-    v.piece_list = L.take<uint32_t>(2 * size_t(piece_capacity));
+    v.piece_list = L.take<uint32_t>(piece_capacity);
     v.cmd_bbox = L.take<int4>(nc);
     v.cmd_tile_x = L.take<uint32_t>(nc);
     v.cmd_tile_y = L.take<uint32_t>(nc);
@@ -1125,7 +1125,7 @@ BLGpuResult Runtime::run_noalloc(const Frame& fr) {
     v.items = L.take<DevItem>(item_capacity);
     v.curve_items = L.take<DevItem>(item_capacity);
     v.pieces = L.take<DevPiece>(piece_capacity);
-    v.piece_list = L.take<uint32_t>(2 * size_t(piece_capacity));
+    v.piece_list = L.take<uint32_t>(piece_capacity);
     v.cmd_bbox = L.take<int4>(nc);
     v.cmd_tile_x = L.take<uint32_t>(nc);
     v.cmd_tile_y = L.take<uint32_t>(nc);
@@ -1136,9 +1136,8 @@ BLGpuResult Runtime::run_noalloc(const Frame& fr) {
     const size_t list_rows = (size_t(fr.rows) << kMaxListLog2) + 1;
     v.row_offsets = L.take<uint32_t>(list_rows);
     v.row_copies = L.take<uint32_t>(list_rows);
-    v.strip_start = L.take<uint32_t>((size_t(fr.tiles) + 1) * (kTileH / kStripRows));
+    // one array per strip, not three: a canvas of 20,000 x 20,000 px has 390,000 tiles of eight strips
     v.strip_cmd = L.take<uint32_t>((size_t(fr.tiles) + 1) * (kTileH / kStripRows));
-    v.spilled = L.take<uint32_t>((size_t(fr.tiles) + 1) * (kTileH / kStripRows));
     a_row_canvas = L.take<uint32_t>(list_rows);
     v.tile_order = L.take<uint32_t>(fr.tiles + 1);
     v.tile_canvas = L.take<uint32_t>(fr.tiles + 1);
