@@ -348,7 +348,8 @@ struct FrameView {
   uint32_t* error_flags;
   unsigned long long* pixel_ops;   // [2] composited pixels (mask != 0), of which pattern-fetched
   uint32_t num_cmds;
-  uint32_t num_canvases;
+  uint32_t num_canvases;       // (graph frames: the capacity)
+  uint32_t several_canvases;   // 1: the frame has more than one
   uint32_t num_tiles;
   uint32_t num_rows;
   uint32_t num_lut_jobs;

@@ -2716,7 +2716,7 @@ int launch_fine(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st) {
   if (!f.num_tiles) return 0;
   const uint32_t strips = f.num_tiles * kStripsPerTile;
   const uint32_t needed = cdiv(strips, kFineWarps);
-  if (f.num_canvases > 1) {
+  if (f.several_canvases) {
     fine_kernel<kSpill><<<min(uint32_t(fine_grid_size<kSpill>(cfg.fine_blocks_per_sm)), needed), kFineThreads, 0, st>>>(f);
     fine_kernel<kTail><<<min(uint32_t(fine_grid_size<kTail>(cfg.fine_blocks_per_sm)), needed * kStripRows), kFineThreads, 0, st>>>(f);
     return 2;

@@ -325,8 +325,7 @@ BLGpuResult Runtime::init(const BLGpuRuntimeCreateInfo* info) {
 void Runtime::destroy() {
   cudaSetDevice(device);
   if (stream) cudaStreamSynchronize(stream);
-  if (graph) cudaGraphExecDestroy(graph);
-  graph = nullptr;
+  drop_graphs();
   for (auto& e : ev) if (e) cudaEventDestroy(e);
   if (side) { cudaStreamSynchronize(side); cudaStreamDestroy(side); }
   if (fork_ev) cudaEventDestroy(fork_ev);
@@ -678,6 +677,7 @@ BLGpuResult Runtime::upload_frame(const Frame& fr, const FrameSizes* caps) {
   v.piece_capacity = piece_capacity;
   v.num_cmds = nc;
   v.num_canvases = z.canvases;
+  v.several_canvases = ncv > 1 ? 1u : 0u;
   v.num_tiles = z.tiles;
   v.num_rows = z.rows;
   v.num_lut_jobs = z.lut_jobs;
@@ -744,6 +744,38 @@ int Runtime::enqueue_render_half(cudaStream_t st, bool timed, bool gated) {
   k += launch_fine(f, cfg, st);
   if (timed) cudaEventRecord(ev[2], st);
   return k;
+}
+
+void Runtime::drop_graphs() {
+  for (FrameGraph& g : graphs) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g = FrameGraph{};
+  }
+  graph_valid = false;
+}
+
+// The captured pipeline of the current view's kind of frame, captured now if there is none on its layout.
+// Frames of one canvas and of several launch different composites and take turns in some programs: each
+// kind keeps its graph.
+BLGpuResult Runtime::frame_graph(cudaGraphExec_t& out) {
+  if (!graph_valid) drop_graphs();
+  FrameGraph& kept = graphs[view.several_canvases];
+  if (!kept.exec) {
+    cudaGraph_t g = nullptr;
+    BLGPU_CHECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+    int launches = enqueue_count_half(stream);
+    launches += enqueue_render_half(stream, false, view_by_caps);
+    cudaError_t e = cudaStreamEndCapture(stream, &g);
+    if (e != cudaSuccess) return cuda_result(e);
+    e = cudaGraphInstantiate(&kept.exec, g, 0);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) { kept.exec = nullptr; return cuda_result(e); }
+    kept.launches = uint64_t(launches);
+  }
+  graph_valid = true;
+  stats.kernel_launches = kept.launches;
+  out = kept.exec;
+  return BLGPU_SUCCESS;
 }
 
 // Buffers sized by the counting half's totals. Slots with segments are at most min(slots, raster
@@ -944,21 +976,9 @@ BLGpuResult Runtime::run_graph(const Frame& fr) {
   totals = caps.dyn;
   view_by_caps = true;
   planned_list_shift = list_shift_of(cfg);
-  if (!graph_valid) {
-    if (graph) cudaGraphExecDestroy(graph);
-    graph = nullptr;
-    cudaGraph_t g = nullptr;
-    BLGPU_CHECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    int launches = enqueue_count_half(stream);
-    launches += enqueue_render_half(stream, false, true);
-    cudaError_t e = cudaStreamEndCapture(stream, &g);
-    if (e != cudaSuccess) return cuda_result(e);
-    e = cudaGraphInstantiate(&graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) { graph = nullptr; return cuda_result(e); }
-    graph_valid = true;
-    stats.kernel_launches = uint64_t(launches);
-  }
+  cudaGraphExec_t graph = nullptr;
+  r = frame_graph(graph);
+  if (r) return r;
   {
     std::unique_lock<std::mutex> order;
     if (cfg.device_order) {
@@ -1289,21 +1309,9 @@ BLGpuResult Runtime::replay(bool use_graph) {
     pending_timing = 2;
     return BLGPU_SUCCESS;
   }
-  if (!graph_valid) {
-    if (graph) cudaGraphExecDestroy(graph);
-    graph = nullptr;
-    cudaGraph_t g = nullptr;
-    BLGPU_CHECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    int launches = enqueue_count_half(stream);
-    launches += enqueue_render_half(stream, false, view_by_caps);
-    cudaError_t e = cudaStreamEndCapture(stream, &g);
-    if (e != cudaSuccess) return cuda_result(e);
-    e = cudaGraphInstantiate(&graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) { graph = nullptr; return cuda_result(e); }
-    graph_valid = true;
-    stats.kernel_launches = uint64_t(launches);
-  }
+  cudaGraphExec_t graph = nullptr;
+  BLGpuResult r = frame_graph(graph);
+  if (r) return r;
   BLGPU_CHECK(cudaEventRecord(ev[0], stream));
   BLGPU_CHECK(cudaGraphLaunch(graph, stream));
   BLGPU_CHECK(cudaEventRecord(ev[3], stream));
@@ -1401,9 +1409,7 @@ BLGpuResult Runtime::release_memory() {
   BLGPU_CHECK(cudaSetDevice(device));
   BLGPU_CHECK(cudaStreamSynchronize(stream));
   BLGPU_CHECK(cudaStreamSynchronize(side));
-  if (graph) cudaGraphExecDestroy(graph);
-  graph = nullptr;
-  graph_valid = false;
+  drop_graphs();
   has_frame = false;
   pending_timing = 0;
   in_buf.release();

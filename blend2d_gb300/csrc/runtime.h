@@ -205,8 +205,13 @@ struct Runtime {
   cudaStream_t side = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   cudaEvent_t order_ev = nullptr;      // end of this runtime's last ordered pipeline (LaunchConfig::device_order)
-  cudaGraphExec_t graph = nullptr;
-  bool graph_valid = false;
+  // captured pipelines: of frames of one canvas, of several
+  struct FrameGraph {
+    cudaGraphExec_t exec = nullptr;
+    uint64_t launches = 0;
+  };
+  FrameGraph graphs[2];
+  bool graph_valid = false;            // they belong to the present layout and launch shapes
 
   // last executed frame (kept for replay)
   FrameView view{};
@@ -275,6 +280,8 @@ struct Runtime {
   BLGpuResult stage_canvases(const Frame& fr);
   BLGpuResult reserve_segments(uint32_t count);
   void read_pixel_ops();
+  BLGpuResult frame_graph(cudaGraphExec_t& out);
+  void drop_graphs();
 };
 
 BLGpuResult cuda_result(cudaError_t e);
