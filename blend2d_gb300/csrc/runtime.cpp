@@ -974,6 +974,7 @@ BLGpuResult Runtime::run_graph(const Frame& fr) {
   L.base = static_cast<char*>(dyn_buf.ptr);
   plan_dynamic(L, view, caps.dyn);
   totals = caps.dyn;
+  if (!view_by_caps) graph_valid = false;      // a replay may have captured the kept frame on its own layout
   view_by_caps = true;
   planned_list_shift = list_shift_of(cfg);
   cudaGraphExec_t graph = nullptr;
