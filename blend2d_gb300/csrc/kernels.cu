@@ -2688,15 +2688,9 @@ int launch_coverage(const FrameView& f, const LaunchConfig& cfg, cudaStream_t st
   if (!f.num_cmdrows) return k;
   slot_compact_kernel<<<layout_grid, 32 * kLayoutWarps, 0, st>>>(f);
   k += 1 + launch_seg_bin<true>(f, st);
-  // far more blocks than fit at once, so that long groups even out (12, 16, 24, 32 and 64 an SM: 4.79, 4.34,
-  // 4.19, 4.16 and 4.01 ms on the batch's canvases), but none without a group
-  const int per_sm = cfg.cover_blocks_per_sm > 0 ? cfg.cover_blocks_per_sm : 64;
-  // 8 slots a warp: 16 (64 a block) leave less shared memory for other warps, 4 fewer work items than
-  // lanes. The pass at 16, 32 and 64 slots a block: 5.44, 4.37 and 4.66 ms on 512 canvases of the batch,
-  // 0.41, 0.36 and 0.41 on 20,000 curve paths.
-  const int slots = cfg.cover_slots ? cfg.cover_slots : 32;
+  const int slots = cover_slots_of(cfg);       // no block without a group
   const bool occlusion = !cfg.no_occlusion_cull;
-  const int grid = int(min(uint32_t(sms * per_sm), cdiv(f.mask_capacity, uint32_t(slots))));
+  const int grid = int(min(uint32_t(sms * cover_blocks_of(cfg)), cdiv(f.mask_capacity, uint32_t(slots))));
   if (slots == 16) coverage_kernel<16 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f, occlusion);
   else if (slots == 64) coverage_kernel<64 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f, occlusion);
   else coverage_kernel<32 / kCoverWarps><<<grid, 32 * kCoverWarps, 0, st>>>(f, occlusion);

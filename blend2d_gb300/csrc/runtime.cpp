@@ -1372,23 +1372,11 @@ BLGpuResult Runtime::autotune(int trials, LaunchConfig* best_out, double* best_m
   LaunchConfig best = cfg;
   double best_ms = 0.0;
   if (!r) r = measure(best, best_ms);
-  const int cover_slots[] = {0, 16, 32, 64};
-  const int blocks[] = {0, 1, 2, 3};
-  const int edge_blocks[] = {64, 128, 256};
-  const int list_rows[] = {32, 16, 8, 4};
-  // fields: list-row height (binning geometry of the composite), coverage slots per block (the
-  // band of slots a block rasterizes), coverage / composite / curve grids, edges per block
-  const int order[] = {5, 0, 1, 2, 3, 4};
-  for (int fi = 0; fi < 6 && !r; fi++) {
-    const int field = order[fi];
-    const int* vals = field == 0 ? cover_slots : field == 3 ? edge_blocks : field == 5 ? list_rows : blocks;
-    const int nvals = field == 3 ? 3 : 4;
-    for (int k = 0; k < nvals && !r; k++) {
+  for (const LaunchField& f : kLaunchFields) {
+    for (int k = 0; k < f.count && !r; k++) {
       LaunchConfig c = best;
-      int* slot = field == 0 ? &c.cover_slots : field == 1 ? &c.cover_blocks_per_sm : field == 2 ? &c.fine_blocks_per_sm
-                : field == 3 ? &c.edge_block : field == 4 ? &c.cubic_blocks_per_sm : &c.list_rows;
-      if (*slot == vals[k]) continue;
-      *slot = vals[k];
+      c.*f.field = f.values[k];
+      if (same_launches(c, best)) continue;
       double ms = 0.0;
       r = measure(c, ms);
       if (!r && ms < best_ms) { best = c; best_ms = ms; }

@@ -127,15 +127,15 @@ typedef struct BLGpuStats {
   double last_run_ms;      /* host time of the last frame's run: upload, pipeline, read-back */
 } BLGpuStats;
 
-/* Launch shapes of the device pipeline (0 in a *_blocks_per_sm field = as many as fit). Tile and
+/* Launch shapes of the device pipeline (0 in a *_blocks_per_sm field = its default). Tile and
  * band geometry are fixed by the pipeline (32-pixel tile columns matching a warp's lanes, the
  * reference's band heights), so the tunable parameters are how work is grouped and gridded. */
 typedef struct BLGpuLaunchConfig {
   int32_t cover_slots;          /* slots (command x 4-row strip x 32-px tile column) per coverage block: 16, 32 or 64; 0 = 32 */
-  int32_t cover_blocks_per_sm;  /* coverage pass grid */
-  int32_t fine_blocks_per_sm;   /* composite pass grid */
+  int32_t cover_blocks_per_sm;  /* coverage pass grid; 0 = 64, more than fit at once */
+  int32_t fine_blocks_per_sm;   /* composite pass grid; 0 = as many as fit */
   int32_t edge_block;           /* threads per block of the per-item edge builder: 64, 128 or 256 */
-  int32_t cubic_blocks_per_sm;  /* lane-scheduled curve-piece flattener grid */
+  int32_t cubic_blocks_per_sm;  /* clipped curve pieces' flattener grid while the pieces are few; 0 = as many as fit */
   int32_t no_occlusion_cull;    /* 1: composite every command of every strip (pixel-op counts of the
                                    reference's work; same pixels) */
   int32_t max_segments;         /* 0: the segment array grows as frames need; N > 0: it never holds more
