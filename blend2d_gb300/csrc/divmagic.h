@@ -21,12 +21,11 @@ struct DivMagic {
 
 // Magic number and shift for a divisor d >= 1 (Granlund and Montgomery, "Division by Invariant Integers
 // using Multiplication", 1994, section 5): with l = ceil(log2 d), m = floor(2^(31 + l) / d) + 1 - 2^32 and
-// shift l - 1, the quotient is n plus the high product, shifted, plus 1 for a negative n. One division
-// (a search for the smallest shift took 30 steps for the 2^31 - 1 that stands for "no wrap").
+// shift l - 1, the quotient is n plus the high product, shifted, plus 1 for a negative n. One division and
+// no search: one for the smallest shift, or for l, takes 30 steps for the 2^31 - 1 that stands for "no wrap".
 inline DivMagic div_magic(int32_t d) {
   if (d == 1) return DivMagic{0, -1};
-  int32_t l = 1;
-  while (l < 31 && (int32_t(1) << l) < d) l++;
+  const int32_t l = 32 - __builtin_clz(uint32_t(d - 1));
   return DivMagic{int32_t(uint32_t((uint64_t(1) << (31 + l)) / uint32_t(d) + 1u)), l - 1};
 }
 
