@@ -333,7 +333,6 @@ struct FrameView {
   uint32_t* strip_cmd;         // the same as a command: no command of the canvas before it shows in the strip
   uint32_t* spilled;           // [num_tiles * strips per tile] strips whose list the composite's tail launch finishes
                                //   (frames of several canvases)
-  uint32_t* tile_order;        // tile processing order for the persistent fine kernel
   uint32_t* tile_canvas;       // canvas index per global tile
   uint32_t* work_counter;      // [0] fine work queue, [1] items, [2] cubics, [21] quads, [23] / [25] cubic / quadratic
                                //   pieces, [28..31] and [34..37] cubic / quadratic pieces the safe loop flattens, clipped

@@ -1241,6 +1241,10 @@ struct LaneCurve {
   uint32_t any, sign, out;
   double y_start, y_end;
 
+  // prepare and begin_curve (and step without kDefer) build a whole curve on one lane, in the reference's
+  // order: what the host checks hold the kernels' shared steps against. The kernels take curves apart in
+  // curve_split_kernel and begin at begin_piece.
+
   // curve_to for a source holding exactly this one curve, up to the flattening: p0 (with its clip
   // flags) and spline[1..DEG] set by the caller. A curve entirely on one side of the clip box is
   // done here; otherwise its monotonic pieces are left in spline[0..nout] (`any`: the curve's clip

@@ -14,8 +14,8 @@ namespace blgpu {
 
 // ---------------------------------------------------------------------------------------------
 // K0 - gradient LUTs (interpolation.cpp:19-156, interpolation_sse2.cpp:18-171,
-// interpolation_avx2.cpp:18-177), one thread per entry: the entry's value is whatever the
-// reference's sequential span writer leaves there (later spans overwrite earlier ones).
+// interpolation_avx2.cpp:18-177), one warp per table: the spans are written in the order of the
+// reference's sequential span writer (later spans overwrite earlier ones).
 // ---------------------------------------------------------------------------------------------
 
 __device__ __forceinline__ uint32_t rgba32_of(uint64_t v) {
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(32 * kLutWarps) lut_kernel(const DevLutJob* jo
     if (lane < ns) {
       LutSpan sp;
       sp.start = u0 >> 8;
-      if (scalar) {                                     // lut_spans_scalar, one stop
+      if (scalar) {                                     // interpolation.cpp, one stop
         const uint32_t i = (u1 >> 8) - (u0 >> 8);
         if (i == 0) c0 = c1;
         sp.count = i + 1u;
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(32 * kLutWarps) lut_kernel(const DevLutJob* jo
           sp.inc[3] = int32_t(((c1 >> 1) & kMask) - ((c0 >> 1) & kMask)) / div;
         }
       }
-      else {                                            // lut_spans_simd, one stop
+      else {                                            // interpolation_sse2.cpp and _avx2.cpp, one stop
         sp.count = (u1 >> 8) - (u0 >> 8);
         sp.c0 = c0;
         sp.c1 = c1;
@@ -1407,7 +1407,7 @@ __global__ void frame_gate_kernel(FrameView f) {
 
 __device__ __forceinline__ bool frame_skipped(const FrameView& f) { return f.work_counter[kSkipWord] != 0u; }
 
-// Tile/row bookkeeping: canvas of every global tile and list row, identity processing order.
+// Tile/row bookkeeping: canvas of every global tile and list row.
 __device__ __forceinline__ void tile_setup(const FrameView& f, uint32_t i, uint32_t* row_canvas) {
   const uint32_t num_canvases = f.counts[kCntCanvases];
   // binary search the canvas owning tile i / row i
@@ -1415,7 +1415,6 @@ __device__ __forceinline__ void tile_setup(const FrameView& f, uint32_t i, uint3
     uint32_t lo = 0, hi = num_canvases - 1;
     while (lo < hi) { uint32_t mid = (lo + hi + 1) >> 1; if (f.canvases[mid].tile_base <= i) lo = mid; else hi = mid - 1; }
     f.tile_canvas[i] = lo;
-    f.tile_order[i] = i;
   }
   const uint32_t log2 = kTileShift - f.list_shift;
   if (i < (f.counts[kCntRows] << log2)) {
@@ -2285,7 +2284,7 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
     if (unit >= num_units) break;
     const int prow = kMode == kTail ? int(unit % kStripRows) : lane >> 3;     // row within the strip
     if (kMode == kTail) unit = f.spilled[unit / kStripRows];
-    uint32_t tile = f.tile_order[unit / kStripsPerTile];
+    const uint32_t tile = unit / kStripsPerTile;
     int strip = int(unit % kStripsPerTile);
     const DevCanvas cv = f.canvases[f.tile_canvas[tile]];
     uint32_t local = tile - cv.tile_base;
@@ -2440,7 +2439,7 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
           pat_ops += n;
           // one copy of the fetch code: the 4 pixels rotate through the last place
           const DevStyle& st = f.styles[style];
-          const px::RowState rs = px::row_state(st, y, 0);
+          const px::RowState rs = px::row_state(st, y);
           uint32_t m = mw;
 #pragma unroll 1
           for (int k = 0; k < PX; k++, m >>= 8) {
@@ -2486,7 +2485,7 @@ __global__ void __launch_bounds__(kFineThreads, kFineBlocksPerSM) fine_kernel(Fr
   }
 }
 
-// Gradient row states: one thread per (command, row) of every radial/conic command's bbox.
+// Radial row values: one thread per (command, row) of every radial/conic command's bbox.
 __global__ void row_state_kernel(FrameView f) {
   if (frame_skipped(f)) return;
   const uint32_t total = min(f.totals[4], f.num_row_states);
@@ -2495,15 +2494,9 @@ __global__ void row_state_kernel(FrameView f) {
   uint32_t lo = 0, hi = f.counts[kCntCmds] - 1;       // last command whose first row state is <= t
   while (lo < hi) { uint32_t mid = (lo + hi + 1) >> 1; if (f.rs_base[mid] <= t) lo = mid; else hi = mid - 1; }
   const uint32_t c = lo;
-  const DevCmd& cmd = f.cmds[c];
-  const DevCanvas& cv = f.canvases[cmd.canvas];
-  const int y = int(f.cmd_yr[c] & 0xFFFFu) + int(t - f.rs_base[c]);
-  // the row the reference initialized its fetcher at (start of the band for analytic fills)
-  int fetch_y0 = cmd.kind == kFillAnalytic ? max(cmd.box[1], (y / cv.band_height) * cv.band_height) : cmd.fetch_y0;
-  const DevStyle& st = f.styles[cmd.style];
+  const DevStyle& st = f.styles[f.cmds[c].style];
   if (st.fetch == kFetchConic) return;            // conic_rows_kernel
-  px::RowState rs = px::row_state(st, y, fetch_y0);
-  f.row_states[t] = make_float4(rs.f0, rs.f1, rs.f2, 0.0f);
+  f.row_states[t] = px::radial_row(st, int(f.cmd_yr[c] & 0xFFFFu) + int(t - f.rs_base[c]));
 }
 
 // Conic row values, one thread per run of rows sharing a fetcher start: the reference steps the

@@ -5,7 +5,7 @@
 // wrap mod 2^64, float x positions are exact integers, pattern indices are normalized into a
 // unique representative - so each pixel is evaluated directly from (x, y) here. The one stateful
 // exception is the conic gradient's row origin, which the reference accumulates in FP64 from the
-// row at which its fill call initialized the fetcher; RowState reproduces that accumulation.
+// row at which its fill call initialized the fetcher; conic_rows_kernel reproduces that accumulation.
 //
 // Pixel arithmetic follows the reference's 64-bit unpacked form (pixelgeneric_p.h:110-220):
 // lanes [A:48 G:32 R:16 B:0], div255 = ((x + 128) + ((x + 128) >> 8)) >> 8 per 16-bit lane.
@@ -69,9 +69,8 @@ __device__ __forceinline__ uint32_t grad_index(uint32_t idx, bool pad, uint32_t 
 
 // Per (command, row) state computed once per thread row.
 struct RowState {
-  uint64_t a64, b64;     // linear: py | affine: tx, ty of the row
-  float f0, f1, f2;      // radial: b, d, dd | conic: tx, |ay|, by
-  int32_t r0, r1;        // pattern: source rows (r1 = next row for fx/fy)
+  uint64_t a64, b64;     // affine: tx, ty of the row
+  int32_t r0, r1;        // source rows (r1 = next row for fx/fy)
 };
 
 // Vertical pattern mapping (FetchPatternVertAAExtendCtxAny, fetchgeneric_p.h:78-155).
@@ -121,43 +120,27 @@ __device__ __forceinline__ void af_index(const DevStyle& s, uint64_t px, uint64_
   iy = uint32_t(y);
 }
 
-// Row state. `fetch_y0` is the row where the reference initialized its fetcher for this row
-// (only the conic gradient depends on it).
 // Radial and conic fetchers carry FP64 row state; it is tabulated per (command, row) once per
 // frame instead of being recomputed by every lane that composites the row.
 __device__ __forceinline__ bool has_row_table(uint32_t fetch) {
   return fetch == kFetchRadialPad || fetch == kFetchRadialRoR || fetch == kFetchConic;
 }
 
-__device__ RowState row_state(const DevStyle& st, int y, int fetch_y0) {
+// A radial fetcher's row values (a conic's come from a chain over the rows, conic_rows_kernel).
+__device__ __forceinline__ float4 radial_row(const DevStyle& st, int y) {
+  double ry = double(y);
+  double ptx = st.rad_yx * ry + st.rad_tx;
+  double pty = st.rad_yy * ry + st.rad_ty;
+  double b = ry * st.rad_by + st.rad_b0;
+  double sq_dist = ptx * ptx + pty * pty;
+  return make_float4(float(b * st.rad_inv2a), float((st.rad_amul4 * (sq_dist - st.rad_sq_fr) + b * b) * st.rad_sq_inv2a),
+                     float((ry * st.rad_ddy + st.rad_dd0) * st.rad_sq_inv2a), 0.0f);
+}
+
+// Row state of a pattern fetcher.
+__device__ RowState row_state(const DevStyle& st, int y) {
   RowState r{};
   switch (st.fetch) {
-    case kFetchLinearPad: case kFetchLinearRoR:
-      r.a64 = st.lin_pt0 + uint64_t(uint32_t(y)) * st.lin_dy;
-      break;
-    case kFetchRadialPad: case kFetchRadialRoR: {
-      double ry = double(y);
-      double ptx = st.rad_yx * ry + st.rad_tx;
-      double pty = st.rad_yy * ry + st.rad_ty;
-      double b = ry * st.rad_by + st.rad_b0;
-      double sq_dist = ptx * ptx + pty * pty;
-      r.f0 = float(b * st.rad_inv2a);
-      r.f1 = float((st.rad_amul4 * (sq_dist - st.rad_sq_fr) + b * b) * st.rad_sq_inv2a);
-      r.f2 = float((ry * st.rad_ddy + st.rad_dd0) * st.rad_sq_inv2a);
-      break;
-    }
-    case kFetchConic: {
-      double tx = st.con_tx + st.con_yx * double(fetch_y0);
-      double ty = st.con_ty + st.con_yy * double(fetch_y0);
-      for (int k = fetch_y0; k < y; k++) { tx += st.con_yx; ty += st.con_yy; }
-      float ay = float(ty);
-      uint32_t sb = __float_as_uint(ay);
-      uint32_t byb = uint32_t(int32_t(sb) >> 31) & __float_as_uint(st.con_n1);
-      r.f0 = float(tx);
-      r.f1 = fabsf(ay);
-      r.f2 = __uint_as_float(byb);
-      break;
-    }
     case kFetchPatAlignedPad: case kFetchPatAlignedRepeat: case kFetchPatAlignedRoR:
       r.r0 = pat_row(st, y);
       break;

@@ -551,11 +551,8 @@ BLGpuResult Runtime::upload_frame(const Frame& fr, const FrameSizes* caps) {
     v.strip_cmd = L.take<uint32_t>((size_t(z.tiles) + 1) * (kTileH / kStripRows));
     v.spilled = L.take<uint32_t>((size_t(z.tiles) + 1) * (kTileH / kStripRows));
     row_canvas = L.take<uint32_t>(list_rows);
-    v.tile_order = L.take<uint32_t>(z.tiles + 1);
     v.tile_canvas = L.take<uint32_t>(z.tiles + 1);
-    // [0] work queue, [1] line items, [2] cubic curves, [3] their queue, [4..12) totals,
-    // [12..16) error flags, [16..20) pixel ops (2 x u64), [21] quadratic / conic curves, [22] their
-    // queue
+    // [4..12) totals, [12..16) error flags, [16..20) pixel ops (2 x u64); the others as FrameView lists them
     v.work_counter = L.take<uint32_t>(kCounterWords + list_rows);        // cleared together with row_counts
     v.row_counts = v.work_counter + kCounterWords;
     v.totals = v.work_counter + 4;
@@ -1160,7 +1157,6 @@ BLGpuResult Runtime::run_noalloc(const Frame& fr) {
     // one array per strip, not three: a canvas of 20,000 x 20,000 px has 390,000 tiles of eight strips
     v.strip_cmd = L.take<uint32_t>((size_t(fr.tiles) + 1) * (kTileH / kStripRows));
     a_row_canvas = L.take<uint32_t>(list_rows);
-    v.tile_order = L.take<uint32_t>(fr.tiles + 1);
     v.tile_canvas = L.take<uint32_t>(fr.tiles + 1);
     v.work_counter = L.take<uint32_t>(kCounterWords + list_rows);        // cleared together with row_counts
     v.row_counts = v.work_counter + kCounterWords;
