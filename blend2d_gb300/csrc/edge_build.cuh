@@ -847,8 +847,10 @@ __device__ __forceinline__ int fixed7(double x) {
 // are whole 1/128 units (of 1/256 px), off by less than one, and so are their differences v = last -
 // first and a, b = control - first. Bounded control points stay in the node's box through every
 // split, so |a| and |b| are at most |v| + 1 per axis and a cross product is off by at most 2 (|vx| +
-// |vy|) + 4, and in FP32 by the roundings of two products and their difference, 2^-21 len, more. All
-// of it is 0.05 of the tolerance's 51.2 units: about one node in a thousand is too close to tell.
+// |vy|) + 4, and in FP32 by the roundings of two products and their difference, 2^-21 len, more. As
+// a distance that is at most 0.022 units and 0.00012 more per pixel of the node's length, of the tolerance's
+// 51.2: 0.05 for a node of 230 px, 0.5 for one of 4,096. Of the nodes of 512 canvases of the batch (curves
+// in boxes of 8 to 256 px a side) 0.08 % are too close to tell.
 template<int DEG>
 __device__ __forceinline__ int flat_guess(const Pt* p) {
   const int x0 = fixed7(p[0].x), y0 = fixed7(p[0].y);
