@@ -853,8 +853,8 @@ __global__ void __launch_bounds__(32 * kSplitWarps, kSplitBlocksPerSM) curve_spl
 // warp-wide loop. Only the nodes on the way to a clip are walked here: a subtree inside the clip box
 // is handed to the tree flattener, as a piece in the gap between the cubic pieces (from the front of
 // the piece array) and the others (from its back), while there is room (half of the gap each). A
-// clipped piece then costs its lane some seven steps on average, not one per leaf. Bound: latency, with
-// 5 of 32 lanes active. Against flattening every leaf here, one kernel per kind of curve, all
+// clipped piece then costs its lane some seven steps on average, not one per leaf. Bound: latency - of instruction
+// fetches, every warp being somewhere else in the state machine, then FP64 - with 7 to 9 of 32 lanes active. Against flattening every leaf here, one kernel per kind of curve, all
 // quadratic pieces included: large shapes on 1023x767 0.65 -> 0.06 ms (the tree flattener 0.07 ->
 // 0.04), 10,000 stroked paths (quadratic outlines) 0.94 -> 0.06 (tree 0.03 -> 0.30), a 64x64 icon
 // 0.10 -> 0.04, 20,000 curve paths on 1920x1080 0.17 -> 0.13, 512 canvases of the batch 3.04 -> 2.12
