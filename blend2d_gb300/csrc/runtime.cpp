@@ -1155,6 +1155,7 @@ BLGpuResult Runtime::run_noalloc(const Frame& fr) {
     v.row_offsets = L.take<uint32_t>(list_rows);
     v.row_copies = L.take<uint32_t>(list_rows);
     // one array per strip, not three: a canvas of 20,000 x 20,000 px has 390,000 tiles of eight strips
+    // (strip_start is taken below from what is left)
     v.strip_cmd = L.take<uint32_t>((size_t(fr.tiles) + 1) * (kTileH / kStripRows));
     a_row_canvas = L.take<uint32_t>(list_rows);
     v.tile_canvas = L.take<uint32_t>(fr.tiles + 1);
@@ -1249,6 +1250,8 @@ BLGpuResult Runtime::run_noalloc(const Frame& fr) {
     D.off = dyn_begin;
     plan_dynamic(D, view, t);
     if (D.off > kNoAllocArenaBytes) { r = BLGPU_ERROR_DATA_TOO_LARGE; break; }
+    const size_t strips = (size_t(fr.tiles) + 1) * (kTileH / kStripRows);
+    if (D.off + 256 + sizeof(uint32_t) * strips <= kNoAllocArenaBytes) view.strip_start = D.take<uint32_t>(strips);
     launches += enqueue_render_half(stream, false, false);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(host_totals + 20, view.error_flags, 4, cudaMemcpyDeviceToHost, stream);
